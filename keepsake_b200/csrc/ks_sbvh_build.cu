@@ -813,7 +813,10 @@ __global__ void k_emit(const BuildRec *recs, uint32_t n, const uint32_t *pool, R
 // Traversal layout: one 64-byte record per interior node (DFS order), children boxes inline.
 // Leaf children carry their primitive count (the count the reference's traversal derives from
 // primOffset differences, cuda/sbvh.cu:546-552).
-__global__ void k_trav(const BuildRec *recs, uint32_t n, const uint32_t *interior_scan, TravNode *trav)
+// Also marks each leaf child's last primitive (kLastPrim in the w component of its second vertex,
+// written after k_prim_tris), where the resumable traversal ends the leaf.
+__global__ void k_trav(const BuildRec *recs, uint32_t n, const uint32_t *interior_scan, TravNode *trav,
+                       float4 *prim_tris)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -830,6 +833,10 @@ __global__ void k_trav(const BuildRec *recs, uint32_t n, const uint32_t *interio
     t.c = make_float4(R.bmin[2], R.bmax[0], R.bmax[1], R.bmax[2]);
     t.d = make_uint4(ref_of(L), ref_of(R), L.prims | (p.axis << 30), R.prims);
     trav[interior_scan[p.dfs]] = t;
+    if (L.leaf && L.prims)
+        prim_tris[3 * (size_t)(L.prim_off + L.prims - 1) + 1].w = __uint_as_float(kLastPrim);
+    if (R.leaf && R.prims)
+        prim_tris[3 * (size_t)(R.prim_off + R.prims - 1) + 1].w = __uint_as_float(kLastPrim);
 }
 
 __global__ void k_prim_tris(const uint32_t *prims, uint32_t n_prims, const float *verts, const uint32_t *idx,
@@ -845,6 +852,8 @@ __global__ void k_prim_tris(const uint32_t *prims, uint32_t n_prims, const float
         v[k] = make_float4(verts[3 * vi], verts[3 * vi + 1], verts[3 * vi + 2], 0.0f);
     }
     v[0].w = __uint_as_float(t);
+    if (i + 1 == n_prims) // ends the last leaf (the whole tree may be one)
+        v[1].w = __uint_as_float(kLastPrim);
     out[3 * i + 0] = v[0];
     out[3 * i + 1] = v[1];
     out[3 * i + 2] = v[2];
@@ -1042,10 +1051,11 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     KS_CUDA_TRY(ctx, cudaMemcpyAsync(&n_trav, interior_scan.ptr + n_nodes, 4, cudaMemcpyDeviceToHost, st));
     KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     KS_CUDA_TRY(ctx, out.trav.alloc(n_trav > 0 ? n_trav : 1));
-    k_trav<<<grid_for(n_nodes, 256), 256, 0, st>>>(recs.ptr, n_nodes, interior_scan.ptr, out.trav.ptr);
     KS_CUDA_TRY(ctx, out.prim_tris.alloc((size_t)pool_used * 3));
     k_prim_tris<<<grid_for(pool_used, 256), 256, 0, st>>>(out.prims.ptr, pool_used, verts, indices,
                                                           out.prim_tris.ptr);
+    k_trav<<<grid_for(n_nodes, 256), 256, 0, st>>>(recs.ptr, n_nodes, interior_scan.ptr, out.trav.ptr,
+                                                   out.prim_tris.ptr);
     KS_CUDA_TRY(ctx, cudaGetLastError());
     if (done)
         KS_CUDA_TRY(ctx, cudaEventRecord(done, st));

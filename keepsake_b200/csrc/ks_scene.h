@@ -29,6 +29,8 @@ struct TravNode
     uint4 d;
 };
 constexpr uint32_t kLeafBit = 0x80000000u;
+// Bits of v1.w in a primitive's record (3 float4: v0 + triangle id, v1 + this mark, v2) that ends a leaf.
+constexpr uint32_t kLastPrim = 0x3f800000u;
 
 // 4-wide view of the same SBVH, read by the renderer's traversal kernels: wide node i holds the
 // children of interior node i, each interior child replaced by its own two children (2 to 4 slots).

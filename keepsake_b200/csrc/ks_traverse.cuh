@@ -302,20 +302,32 @@ struct TravState
 {
     RayQuery ray;
     TriHelper th;
-    BoxHelper bh;
-    uint32_t ref, cnt;
+    f3 inv;          // 1 / direction
+    int px, py, pz;  // byte offsets of the entry planes in a WideNode: lo or hi by the direction's sign
+    bool guard;      // some 1 / direction is infinite: the slab test needs its 0 * inf guard
+    uint32_t ref;
     int sp;
     Hit hit;
 };
 
+KS_D BoxHelper box_helper_of(f3 inv)
+{
+    BoxHelper b;
+    b.inv = inv;
+    b.neg[0] = signbit(inv.x); // the sign of 1 / d is the sign of d, also for zeros
+    b.neg[1] = signbit(inv.y);
+    b.neg[2] = signbit(inv.z);
+    return b;
+}
+
 // Traversal stack of the persistent kernels (blocks of kTravBlock threads): each thread's first
 // KS_SMEM_STACK entries live in shared memory, laid out [entry][thread] so that a warp whose lanes
-// sit at different depths still touches distinct banks; deeper entries spill to local memory.
-// 8 entries (16 KB per CTA, 128 KB per SM at 8 CTAs) measured best on the bench frame: +3.7 %
-// over a local-memory stack; 12 or 16 take L1 capacity from the node cache and lose.
+// sit at different depths still touches distinct banks; deeper entries spill to local memory.  An
+// entry is the node ref and the entry time (8 bytes; a leaf's end is marked in its last primitive,
+// so no count travels with the ref).
 constexpr int kTravBlock = 128;
 #ifndef KS_SMEM_STACK
-#define KS_SMEM_STACK 8
+#define KS_SMEM_STACK 16
 #endif
 // Capacity: the binary traversal pushes at most one entry per level and stops at kStackDepth; the
 // 4-wide one pushes up to three per wide level and stops at kWideStackDepth.
@@ -323,21 +335,22 @@ constexpr int kWideStackDepth = 96;
 constexpr int kSmemStack = KS_SMEM_STACK < kStackDepth ? KS_SMEM_STACK : kStackDepth;
 struct TravStack
 {
-    uint4 *sm; // this thread's column of the block's shared array: entry i at sm[i * kTravBlock]
-    uint4 loc[kWideStackDepth - kSmemStack];
-    KS_D void set(int i, uint4 e)
+    uint2 *sm; // this thread's column of the block's shared array: entry i at sm[i * kTravBlock]
+    uint2 loc[kWideStackDepth - kSmemStack];
+    KS_D void set(int i, uint32_t ref, float t)
     {
+        const uint2 e = make_uint2(ref, __float_as_uint(t));
         if (i < kSmemStack)
             sm[i * kTravBlock] = e;
         else
             loc[i - kSmemStack] = e;
     }
-    KS_D uint4 get(int i) const { return i < kSmemStack ? sm[i * kTravBlock] : loc[i - kSmemStack]; }
+    KS_D uint2 get(int i) const { return i < kSmemStack ? sm[i * kTravBlock] : loc[i - kSmemStack]; }
 };
 // The shared part of a block's stacks; every persistent traversal kernel declares one and points
 // each thread's TravStack at its column.
 #define KS_TRAV_STACK(name)                                                                                       \
-    __shared__ uint4 name##_smem[kSmemStack > 0 ? kSmemStack * kTravBlock : 1];                                  \
+    __shared__ uint2 name##_smem[kSmemStack > 0 ? kSmemStack * kTravBlock : 1];                                  \
     TravStack name;                                                                                                \
     name.sm = name##_smem + threadIdx.x
 
@@ -348,12 +361,16 @@ KS_D bool trav_begin(TravState &s, const RayQuery &ray, uint32_t root_ref, uint3
     s.hit.tri = ~0u;
     s.ray = ray;
     s.th = make_tri_helper(ray.d);
-    s.bh = make_box_helper(ray.d);
+    const BoxHelper bh = make_box_helper(ray.d);
+    s.inv = bh.inv;
+    s.px = bh.neg[0] ? 48 : 0;
+    s.py = bh.neg[1] ? 64 : 16;
+    s.pz = bh.neg[2] ? 80 : 32;
+    s.guard = isinf(bh.inv.x) || isinf(bh.inv.y) || isinf(bh.inv.z);
     s.sp = 0;
     s.ref = root_ref;
-    s.cnt = root_count;
     float t0, t1;
-    return slab(s.ray, s.bh, root_bmin, root_bmax, t0, t1) && t0 < s.ray.tmax && t1 > s.ray.tmin;
+    return root_count != 0 && slab(s.ray, bh, root_bmin, root_bmax, t0, t1) && t0 < s.ray.tmax && t1 > s.ray.tmin;
 }
 
 // Interior node test of trav_step: descends to the near child (pushing the far one when both are
@@ -365,18 +382,17 @@ KS_D int trav_interior(const TravNode *__restrict__ nodes, TravState &s, TravSta
     const TravNode *n = nodes + s.ref;
     if (count)
         count->nodes++;
+    const BoxHelper bh = box_helper_of(s.inv);
     float4 A = __ldg(&n->a), B = __ldg(&n->b), C = __ldg(&n->c);
     uint4 D = __ldg(&n->d);
     float lmin[3] = {A.x, A.y, A.z}, lmax[3] = {A.w, B.x, B.y};
     float rmin[3] = {B.z, B.w, C.x}, rmax[3] = {C.y, C.z, C.w};
     float lt0, lt1, rt0, rt1;
-    bool lok = slab(s.ray, s.bh, lmin, lmax, lt0, lt1) && lt1 > s.ray.tmin && lt0 < s.ray.tmax;
-    bool rok = slab(s.ray, s.bh, rmin, rmax, rt0, rt1) && rt1 > s.ray.tmin && rt0 < s.ray.tmax;
+    bool lok = slab(s.ray, bh, lmin, lmax, lt0, lt1) && lt1 > s.ray.tmin && lt0 < s.ray.tmax;
+    bool rok = slab(s.ray, bh, rmin, rmax, rt0, rt1) && rt1 > s.ray.tmin && rt0 < s.ray.tmax;
     uint32_t axis = D.z >> 30;
-    uint32_t lcnt = D.z & 0x3fffffffu, rcnt = D.w;
-    bool right_first = s.bh.neg[axis] != 0;
+    bool right_first = bh.neg[axis] != 0;
     uint32_t near_ref = right_first ? D.y : D.x, far_ref = right_first ? D.x : D.y;
-    uint32_t near_cnt = right_first ? rcnt : lcnt, far_cnt = right_first ? lcnt : rcnt;
     bool near_ok = right_first ? rok : lok, far_ok = right_first ? lok : rok;
     float far_t = right_first ? lt0 : rt0;
     if (near_ok && far_ok) {
@@ -384,13 +400,38 @@ KS_D int trav_interior(const TravNode *__restrict__ nodes, TravState &s, TravSta
             overflow = 1;
             return -1;
         }
-        stack.set(s.sp++, make_uint4(far_ref, far_cnt, __float_as_uint(far_t), 0u));
+        stack.set(s.sp++, far_ref, far_t);
     }
     if (!near_ok && !far_ok)
         return 0;
     s.ref = near_ok ? near_ref : far_ref;
-    s.cnt = near_ok ? near_cnt : far_cnt;
     return 1;
+}
+
+// Entry times of a wide node's slots with the guard of slab() for rays along an axis (0 * inf), and
+// a bit per slot that passes; out of line, so that the common rays' code stays small.
+struct WideHits
+{
+    float t[4];
+    uint32_t ok;
+};
+static __device__ __noinline__ WideHits wide_slabs_guarded(const WideNode *n, f3 o, f3 inv, float tmin, float tmax)
+{
+    const RayQuery ray{o, o, tmin, tmax};
+    const BoxHelper bh = box_helper_of(inv);
+    WideHits h;
+    h.ok = 0;
+    const float *lo = reinterpret_cast<const float *>(n->lo), *hi = reinterpret_cast<const float *>(n->hi);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float bmin[3] = {__ldg(lo + k), __ldg(lo + 4 + k), __ldg(lo + 8 + k)};
+        const float bmax[3] = {__ldg(hi + k), __ldg(hi + 4 + k), __ldg(hi + 8 + k)};
+        float a, b;
+        const bool ok = slab(ray, bh, bmin, bmax, a, b) && b > tmin && a < tmax;
+        h.t[k] = a;
+        h.ok |= (uint32_t)ok << k;
+    }
+    return h;
 }
 
 // Interior step of the 4-wide view (WideNode): the slots' boxes are tested with the same slab test,
@@ -400,36 +441,48 @@ KS_D int trav_interior(const TravNode *__restrict__ nodes, TravState &s, TravSta
 // trav_interior.  The set of leaves a closest-hit ray can reach is that of the binary tree (a
 // slot's slab interval lies inside its parent's: same operations, monotone rounding), so the
 // closest hit is the binary traversal's up to the order of exact ties.
+// The step is bound by the instructions it issues, so the arithmetic of slab() is laid out for few:
+// entry and exit planes are picked by address instead of by selects, the running maximum and
+// minimum of slab() are one max and one min over the axes (equal for boxes with lo <= hi), and the
+// 0 * inf guard, which changes nothing while every 1 / d is finite, is a path of its own.  With ranks
+// instead of a sorting network over four values per slot and 8-byte stack entries the mesh frame
+// (1.3 M triangles, 1024 x 1024 x 64) went from 101.9 to 93.5 ms, the instanced one (1080p x 4) from
+// 41.3 to 38.0 ms, every image bit for bit the same.
 template <bool kAnyHit>
 KS_D int trav_wide(const WideNode *__restrict__ wide, TravState &s, TravStack &stack, int &overflow,
                    TravCount *count)
 {
-    const WideNode *n = wide + s.ref;
+    const char *n = reinterpret_cast<const char *>(wide + s.ref);
     if (count)
         count->nodes += 2; // 128 bytes: two 64-byte node units
-    const float4 lx = __ldg(&n->lo[0]), ly = __ldg(&n->lo[1]), lz = __ldg(&n->lo[2]);
-    const float4 hx = __ldg(&n->hi[0]), hy = __ldg(&n->hi[1]), hz = __ldg(&n->hi[2]);
-    const uint4 ref = __ldg(&n->ref), cnt = __ldg(&n->cnt);
-    const float blo[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w}, {lz.x, lz.y, lz.z, lz.w}};
-    const float bhi[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w}, {hz.x, hz.y, hz.z, hz.w}};
-    // counts are below 2^30 (the bound TravNode's packed counts have); masked to those bits, the
-    // kernel measured 0.6 % faster on the bench frame (the compiler keeps it free of spills)
-    constexpr uint32_t kCount = 0x3fffffffu;
-    const uint32_t refs[4] = {ref.x, ref.y, ref.z, ref.w};
-    const uint32_t cnts[4] = {cnt.x & kCount, cnt.y & kCount, cnt.z & kCount, cnt.w & kCount};
+    const uint4 ref4 = __ldg(reinterpret_cast<const uint4 *>(n + 96));
+    const uint32_t refs[4] = {ref4.x, ref4.y, ref4.z, ref4.w};
     float t0[4];
     bool ok[4];
+    if (!s.guard) {
+        auto plane = [&](int off) { return __ldg(reinterpret_cast<const float4 *>(n + off)); };
+        const float4 ax = plane(s.px), ay = plane(s.py), az = plane(s.pz);
+        const float4 bx = plane(48 - s.px), by = plane(80 - s.py), bz = plane(112 - s.pz);
+        const float ex[4] = {ax.x, ax.y, ax.z, ax.w}, ey[4] = {ay.x, ay.y, ay.z, ay.w}, ez[4] = {az.x, az.y, az.z, az.w};
+        const float lx[4] = {bx.x, bx.y, bx.z, bx.w}, ly[4] = {by.x, by.y, by.z, by.w}, lz[4] = {bz.x, bz.y, bz.z, bz.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float bmin[3] = {blo[0][k], blo[1][k], blo[2][k]}, bmax[3] = {bhi[0][k], bhi[1][k], bhi[2][k]};
-        float a, b;
-        ok[k] = slab(s.ray, s.bh, bmin, bmax, a, b) && b > s.ray.tmin && a < s.ray.tmax;
-        t0[k] = a;
+        for (int k = 0; k < 4; ++k) {
+            const float t_in = fmaxf(fmaxf((ex[k] - s.ray.o.x) * s.inv.x, (ey[k] - s.ray.o.y) * s.inv.y),
+                                     (ez[k] - s.ray.o.z) * s.inv.z);
+            const float t_out = fminf(fminf((lx[k] - s.ray.o.x) * s.inv.x, (ly[k] - s.ray.o.y) * s.inv.y),
+                                      (lz[k] - s.ray.o.z) * s.inv.z);
+            ok[k] = t_in <= t_out && t_out > s.ray.tmin && t_in < s.ray.tmax;
+            t0[k] = t_in;
+        }
+    } else {
+        const WideHits h = wide_slabs_guarded(wide + s.ref, s.ray.o, s.inv, s.ray.tmin, s.ray.tmax);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ok[k] = (h.ok >> k) & 1u;
+            t0[k] = h.t[k];
+        }
     }
-    int n_hit = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        n_hit += ok[k] ? 1 : 0;
+    const int n_hit = (int)ok[0] + (int)ok[1] + (int)ok[2] + (int)ok[3];
     if (n_hit == 0)
         return 0;
     if (s.sp + n_hit - 1 > kWideStackDepth) {
@@ -438,53 +491,36 @@ KS_D int trav_wide(const WideNode *__restrict__ wide, TravState &s, TravStack &s
     }
     if constexpr (kAnyHit) {
         // any-hit: the first slot hit next, the others pushed in slot order.  Nearest first (the
-        // network below) took 2.5 % off the bench frame's shadow rays but made a pass of the
+        // ranks below) took 2.5 % off the bench frame's shadow rays but made a pass of the
         // occluded glossy scene 17 % slower: shadow rays blocked by a distant occluder then search
         // the nearby geometry's subtrees first.
         const int f = ok[0] ? 0 : (ok[1] ? 1 : (ok[2] ? 2 : 3));
         s.ref = f == 0 ? refs[0] : (f == 1 ? refs[1] : (f == 2 ? refs[2] : refs[3]));
-        s.cnt = f == 0 ? cnts[0] : (f == 1 ? cnts[1] : (f == 2 ? cnts[2] : cnts[3]));
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+            if (ok[k] && k != f)
+                stack.set(s.sp++, refs[k], t0[k]);
+    } else {
+        // visiting order (entry time, then slot) as ranks from the six pairwise comparisons; a slot
+        // goes straight to its place on the stack (the same instructions in every lane)
+        float kt[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (ok[k] && k != f)
-                stack.set(s.sp++, make_uint4(refs[k], cnts[k], __float_as_uint(t0[k]), 0u));
-    } else {
-        // the slots in visiting order (entry time, then slot index; the slots not hit last) by a
-        // 4-input sorting network: the same instructions in every lane, where branches on the
-        // number of slots hit split the warp (measured 6 % off the closest-hit kernel)
-        float kt[4];
-        uint32_t kr[4], kc[4], ks[4];
+            kt[k] = ok[k] ? t0[k] : kInf;
+        const int c01 = kt[1] < kt[0], c02 = kt[2] < kt[0], c03 = kt[3] < kt[0];
+        const int c12 = kt[2] < kt[1], c13 = kt[3] < kt[1], c23 = kt[3] < kt[2];
+        const int rank[4] = {c01 + c02 + c03, 1 - c01 + c12 + c13, 2 - c02 - c12 + c23, 3 - c03 - c13 - c23};
+        const int top = s.sp + n_hit - 1;
+        uint32_t next = refs[0];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            kt[k] = ok[k] ? t0[k] : kInf;
-            ks[k] = ok[k] ? (uint32_t)k : 4u + k;
-            kr[k] = refs[k];
-            kc[k] = cnts[k];
+            if (rank[k] == 0)
+                next = refs[k];
+            else if (ok[k])
+                stack.set(top - rank[k], refs[k], t0[k]);
         }
-        auto cex = [&](int i, int j) {
-            const bool sw = kt[j] < kt[i] || (kt[j] == kt[i] && ks[j] < ks[i]);
-            const float t = sw ? kt[j] : kt[i];
-            kt[j] = sw ? kt[i] : kt[j];
-            kt[i] = t;
-            const uint32_t a = sw ? ks[j] : ks[i], b = sw ? kr[j] : kr[i], c = sw ? kc[j] : kc[i];
-            ks[j] = sw ? ks[i] : ks[j];
-            kr[j] = sw ? kr[i] : kr[j];
-            kc[j] = sw ? kc[i] : kc[j];
-            ks[i] = a;
-            kr[i] = b;
-            kc[i] = c;
-        };
-        cex(0, 1);
-        cex(2, 3);
-        cex(0, 2);
-        cex(1, 3);
-        cex(1, 2);
-#pragma unroll
-        for (int r = 3; r >= 1; --r)
-            if (r < n_hit)
-                stack.set(s.sp++, make_uint4(kr[r], kc[r], __float_as_uint(kt[r]), 0u));
-        s.ref = kr[0];
-        s.cnt = kc[0];
+        s.ref = next;
+        s.sp = top;
     }
     return 1;
 }
@@ -507,49 +543,50 @@ KS_D int trav_node(const WideNode *__restrict__ nodes, TravState &s, TravStack &
 KS_D bool trav_pop(TravState &s, const TravStack &stack)
 {
     while (s.sp > 0) {
-        const uint4 e = stack.get(--s.sp);
-        if (__uint_as_float(e.z) < s.ray.tmax) {
+        const uint2 e = stack.get(--s.sp);
+        if (__uint_as_float(e.y) < s.ray.tmax) {
             s.ref = e.x;
-            s.cnt = e.y;
             return true;
         }
     }
     return false;
 }
 
-// Leaf triangles of trav_step; true when an any-hit query found an occluder.
+// Leaf triangles of trav_step (up to the one marked as the leaf's last); true when an any-hit query
+// found an occluder.
 template <bool kAnyHit, class Alpha = NoAlpha>
 KS_D bool trav_leaf(const float4 *__restrict__ tris, TravState &s, int culling, TravCount *count,
                     const Alpha &alpha = Alpha{})
 {
     const uint32_t first = s.ref & ~kLeafBit;
-    for (uint32_t k = 0; k < s.cnt; ++k) {
+    bool last;
+    uint32_t slot = first;
+    do {
         if (count)
             count->tris++;
-        const float4 *p = tris + 3 * (size_t)(first + k);
+        const float4 *p = tris + 3 * (size_t)slot;
         float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+        last = __float_as_uint(b.w) != 0u;
         f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
-        if (cull_tri(s.ray, v0, v1, v2, culling))
-            continue;
         float t, b0, b1, b2;
-        if (isect_tri(s.ray, s.th, v0, v1, v2, t, b0, b1, b2)) {
+        if (!cull_tri(s.ray, v0, v1, v2, culling) && isect_tri(s.ray, s.th, v0, v1, v2, t, b0, b1, b2)) {
             if (kAnyHit) {
-                if (!alpha(__float_as_uint(a.w), b1, b2, s.ray))
-                    continue;
-                s.hit.tri = __float_as_uint(a.w);
-                return true;
-            }
-            if (t < s.ray.tmax && alpha(__float_as_uint(a.w), b1, b2, s.ray)) {
+                if (alpha(__float_as_uint(a.w), b1, b2, s.ray)) {
+                    s.hit.tri = __float_as_uint(a.w);
+                    return true;
+                }
+            } else if (t < s.ray.tmax && alpha(__float_as_uint(a.w), b1, b2, s.ray)) {
                 s.ray.tmax = t;
                 s.hit.tri = __float_as_uint(a.w);
-                s.hit.slot = first + k;
+                s.hit.slot = slot;
                 s.hit.t = t;
                 s.hit.b0 = b0;
                 s.hit.b1 = b1;
                 s.hit.b2 = b2;
             }
         }
-    }
+        ++slot;
+    } while (!last);
     return false;
 }
 
