@@ -37,27 +37,16 @@ namespace
 {
 using namespace wave;
 
-// Minimum resident CTAs per SM asked of the compiler (a register cap) for the persistent
-// traversal kernels: at 8 CTAs of 128 (64 registers) they run a little faster than at 7.
-#ifndef KS_TRAV_MIN_BLOCKS
-#define KS_TRAV_MIN_BLOCKS 8
+// Minimum resident CTAs per SM asked of the compiler (a register cap) for the persistent traversal
+// kernels.  The closest-hit kernel spills at 8 (mesh frame, 1.3 M triangles, 1024 x 1024 x 64: 43.8 ms of
+// closest hits at 8, 38.5 at 7, 40.7 at 6), the any-hit kernel does not (17.1 ms of shadow rays at 8, 18.3
+// at 7).
+#ifndef KS_EXT_MIN_BLOCKS
+#define KS_EXT_MIN_BLOCKS 7
 #endif
-// Persistent traversal with dynamic ray fetch (1) or one thread per ray (0) for flat scenes.
-#ifndef KS_PERSISTENT_TRAV
-#define KS_PERSISTENT_TRAV 1
+#ifndef KS_SHADOW_MIN_BLOCKS
+#define KS_SHADOW_MIN_BLOCKS 8
 #endif
-constexpr bool kPersistentTraversal = KS_PERSISTENT_TRAV != 0;
-// Tree layouts of the persistent kernels: the SBVH nodes (0) or their 4-wide view (1).  Measured on
-// the bench frame: the 4-wide view takes 15 % off the any-hit kernel and 2 % off the closest-hit
-// one (whose nearest-first ordering of up to four slots eats most of the saving).
-#ifndef KS_WIDE_EXTEND
-#define KS_WIDE_EXTEND 1
-#endif
-#ifndef KS_WIDE_SHADOW
-#define KS_WIDE_SHADOW 1
-#endif
-using ExtendNode = std::conditional_t<KS_WIDE_EXTEND != 0, WideNode, TravNode>;
-using ShadowNode = std::conditional_t<KS_WIDE_SHADOW != 0, WideNode, TravNode>;
 // Path slots of a single-frame wavefront (log2).  More rays per launch shorten the share of each
 // persistent traversal launch that its last rays run alone, and halve the iterations (and host
 // round trips) per doubling: on the bench frame 4 M slots 1458 Mrays/s, 16 M 1643, 32 M 1690,
@@ -217,56 +206,25 @@ KS_D void flush_counts(const TravCount &c, unsigned long long *dst)
     }
 }
 
-// Closest hit for every queued ray; the path index goes to the hit queue or the miss queue.
-// kInst: two-level traversal of an instanced scene; the instance of each hit goes to hit_inst.
-// kBatch: paths of many jobs (flat scenes), the count read from the batch state.
-template <bool kInst, bool kBatch = false>
-__global__ void __launch_bounds__(128) k_extend(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
-                                                float4 *hits, uint32_t *hit_inst, uint32_t *hit_queue,
-                                                uint32_t *miss_queue, uint32_t *queue_counts, int *overflow,
-                                                unsigned long long *work, BatchView bv)
+// The extension ray of path slot i.
+KS_D RayQuery path_ray(const PathBuf &pb, uint32_t i)
 {
-    TravCount tc;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    if constexpr (kBatch)
-        count = bv.state->count;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
-        uint32_t i = base + threadIdx.x;
-        bool valid = i < count, is_hit = false;
-        if (valid) {
-            const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
-            const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
-            float4 a = pb.o_pdf[i], b = pb.d_info[i];
-            RayQuery q;
-            q.o = mk(a.x, a.y, a.z);
-            q.d = mk(b.x, b.y, b.z);
-            q.tmin = 0.0f;
-            q.tmax = kInf;
-            Hit h;
-            int of = 0;
-            if constexpr (kInst) {
-                uint32_t inst = 0;
-                traverse_instances<false>(sv.nodes, sv.prim_tris, sv.inst, q, 2, h, inst, of, &tc);
-                hit_inst[i] = inst;
-            } else {
-                traverse<false>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, q, 2, h, of,
-                                &tc);
-            }
-            if (of)
-                atomicOr(overflow, 1);
-            is_hit = h.tri != ~0u;
-            hits[i] = is_hit ? make_float4(h.t, h.b1, h.b2, fbits(h.slot)) : make_float4(0, 0, 0, fbits(~0u));
-        }
-        uint32_t jh = warp_append(queue_counts, valid && is_hit);
-        uint32_t jm = warp_append(queue_counts + 1, valid && !is_hit);
-        if (valid) {
-            if (is_hit)
-                hit_queue[jh] = i;
-            else
-                miss_queue[jm] = i;
-        }
-    }
-    flush_counts(tc, work);
+    const float4 a = pb.o_pdf[i], b = pb.d_info[i];
+    RayQuery q;
+    q.o = mk(a.x, a.y, a.z);
+    q.d = mk(b.x, b.y, b.z);
+    q.tmin = 0.0f;
+    q.tmax = kInf;
+    return q;
+}
+
+// A ray's result: distance, barycentrics, primitive slot (kNoHit: none, kRetrace: k_build_queues has
+// to trace it again).
+constexpr uint32_t kNoHit = ~0u, kRetrace = ~1u;
+KS_D float4 hit_record(const Hit &h, bool retrace = false)
+{
+    return h.tri == ~0u ? make_float4(0, 0, 0, fbits(kNoHit))
+                        : make_float4(h.t, h.b1, h.b2, fbits(retrace ? kRetrace : h.slot));
 }
 
 // ---- persistent traversal with dynamic ray fetch (flat scenes) --------------------------------
@@ -279,8 +237,9 @@ __global__ void __launch_bounds__(128) k_extend(const __grid_constant__ SceneVie
 // paths into the hit and miss queues in index order, so that shading reads the path state in
 // order.  kBatch: paths of many jobs, the count read from the batch state.
 // kAlpha: the scene has opacity maps; candidate hits go through their stochastic test (SceneAlpha).
-template <bool kBatch = false, bool kAlpha = false>
-__global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
+// kDeep: the tree (of some job) is too deep for the 4-wide view.
+template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
+__global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
                                                    float4 *hits, uint32_t *fetch, int *overflow,
                                                    unsigned long long *work, BatchView bv)
 {
@@ -288,9 +247,14 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_extend_pt(const __g
         count = bv.state->count;
     TravCount tc;
     KS_TRAV_STACK(stack);
-    TravState s;
-    const ExtendNode *nodes = tree_of<ExtendNode>(sv_in);
+    using View = TreeOf<kDeep>;
+    typename View::State s;
+    typename View::Tree tree = View::tree(sv_in);
     const float4 *tris = sv_in.prim_tris;
+    using Alpha = std::conditional_t<kAlpha, SceneAlpha, NoAlpha>;
+    Alpha filter;
+    if constexpr (kAlpha)
+        filter.sv = &sv_in;
     uint32_t ray = ~0u;
     bool drained = false;
     int of = 0;
@@ -299,15 +263,9 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_extend_pt(const __g
         if (id != ~0u) {
             const uint32_t job = kBatch ? (bits(pb.beta_pix[id].w) >> kJobShift) : 0u;
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
-            nodes = tree_of<ExtendNode>(sv);
+            tree = View::tree(sv);
             tris = sv.prim_tris;
-            float4 a = pb.o_pdf[id], b = pb.d_info[id];
-            RayQuery q;
-            q.o = mk(a.x, a.y, a.z);
-            q.d = mk(b.x, b.y, b.z);
-            q.tmin = 0.0f;
-            q.tmax = kInf;
-            if (trav_begin(s, q, sv.root_ref, sv.root_count, sv.bmin, sv.bmax))
+            if (trav_begin(s, path_ray(pb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
             else
                 hits[id] = make_float4(0, 0, 0, fbits(~0u));
@@ -318,14 +276,8 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_extend_pt(const __g
             continue;
         }
         while (true) {
-            bool done;
-            if constexpr (kAlpha)
-                done = trav_warp_step<false>(nodes, tris, s, stack, 2, of, &tc, ray != ~0u, SceneAlpha{&sv_in});
-            else
-                done = trav_warp_step<false>(nodes, tris, s, stack, 2, of, &tc, ray != ~0u);
-            if (done) {
-                hits[ray] = s.hit.tri != ~0u ? make_float4(s.hit.t, s.hit.b1, s.hit.b2, fbits(s.hit.slot))
-                                             : make_float4(0, 0, 0, fbits(~0u));
+            if (trav_warp_step<false>(tree, tris, s, stack, 2, of, &tc, ray != ~0u, filter)) {
+                hits[ray] = hit_record(s.hit, ambiguous(s));
                 ray = ~0u;
             }
             const int n_idle = __popc(__ballot_sync(0xffffffffu, ray == ~0u));
@@ -339,19 +291,37 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_extend_pt(const __g
 }
 
 // Hit and miss queues from the per-ray results of k_extend_pt, one CTA-aggregated append per
-// kind (queue order follows the path index within each CTA's tile).
+// kind (queue order follows the path index within each CTA's tile).  The few rays whose closest hit
+// depends on the visiting order are traced again here first.
 template <bool kBatch = false>
-__global__ void __launch_bounds__(256) k_build_queues(const float4 *hits, uint32_t count, uint32_t *hit_queue,
-                                                      uint32_t *miss_queue, uint32_t *queue_counts, BatchView bv)
+__global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__ SceneView sv_in, PathBuf pb, float4 *hits,
+                                                      uint32_t count, uint32_t *hit_queue,
+                                                      uint32_t *miss_queue, uint32_t *queue_counts, int *overflow,
+                                                      int alpha, BatchView bv)
 {
     if constexpr (kBatch)
         count = bv.state->count;
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t *slot = reinterpret_cast<const uint32_t *>(hits) + 3;
+    const uint32_t *slots = reinterpret_cast<const uint32_t *>(hits) + 3;
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
         const uint32_t i = base + threadIdx.x;
         const bool valid = i < count;
-        const bool is_hit = valid && slot[4 * (size_t)i] != ~0u;
+        uint32_t slot = valid ? slots[4 * (size_t)i] : kNoHit;
+        if (slot == kRetrace) {
+            const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
+            const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+            const RayQuery q = path_ray(pb, i);
+            Retraced r;
+            if (alpha)
+                r = retrace(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, q, 2, SceneAlpha{&sv});
+            else
+                r = retrace(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, q, 2);
+            hits[i] = hit_record(r.hit);
+            if (r.overflow)
+                atomicOr(overflow, 1);
+            slot = r.hit.tri == ~0u ? kNoHit : r.hit.slot;
+        }
+        const bool is_hit = slot != kNoHit;
         uint32_t jh, jm;
         block_append2(queue_counts, is_hit, queue_counts + 1, valid && !is_hit, jh, jm);
         if (valid) {
@@ -361,58 +331,6 @@ __global__ void __launch_bounds__(256) k_build_queues(const float4 *hits, uint32
                 miss_queue[jm] = i;
         }
     }
-}
-
-template <bool kInst, bool kBatch = false>
-__global__ void __launch_bounds__(128) k_shadow(const __grid_constant__ SceneView sv_in, ShadowBuf sb,
-                                                const uint32_t *shadow_count, PathBuf nxt, double *accum_in,
-                                                double *weights_in, int *overflow, unsigned long long *work,
-                                                GuideView gv, BatchView bv)
-{
-    const uint32_t n = *shadow_count;
-    TravCount tc;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 c = sb.contrib[i];
-        const uint32_t job = kBatch ? bits(c.w) : 0u;
-        const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
-        double *accum = kBatch ? bv.accum[job] : accum_in;
-        double *weights = kBatch ? bv.weights[job] : weights_in;
-        float4 a = sb.o_tmax[i], b = sb.d_target[i];
-        RayQuery q;
-        q.o = mk(a.x, a.y, a.z);
-        q.d = mk(b.x, b.y, b.z);
-        q.tmin = 0.0f;
-        q.tmax = a.w;
-        Hit h;
-        int of = 0;
-        bool occ;
-        if constexpr (kInst) {
-            uint32_t inst = 0;
-            occ = traverse_instances<true>(sv.nodes, sv.prim_tris, sv.inst, q, 2, h, inst, of, &tc);
-        } else {
-            occ = traverse<true>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, q, 2, h, of,
-                                 &tc);
-        }
-        if (of)
-            atomicOr(overflow, 1);
-        uint32_t target = bits(b.w);
-        if (gv.rec_cap && !occ && bits(c.w) != kNoRecord)
-            record_add(gv, bits(c.w), mk(c.x, c.y, c.z));
-        if (target & kTermBit) {
-            float4 l = sb.L_term[i];
-            f3 L = mk(l.x, l.y, l.z);
-            if (!occ)
-                L += mk(c.x, c.y, c.z);
-            accumulate(accum, weights, kBatch ? (target & kPixMask) : (target & ~kTermBit), L);
-        } else if (!occ) {
-            float4 l = nxt.L_smp[target];
-            l.x += c.x;
-            l.y += c.y;
-            l.z += c.z;
-            nxt.L_smp[target] = l;
-        }
-    }
-    flush_counts(tc, work);
 }
 
 // Completion of shadow ray i: records, then the contribution goes to the continuing path or, for a
@@ -445,8 +363,8 @@ KS_D void shadow_done(const ShadowBuf &sb, uint32_t i, bool occ, PathBuf nxt, do
 
 // Any-hit traversal of the NEE shadow rays with dynamic ray fetch (flat scenes); each ray is
 // finished by shadow_done as soon as its traversal ends.
-template <bool kBatch = false, bool kAlpha = false>
-__global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __grid_constant__ SceneView sv_in, ShadowBuf sb,
+template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
+__global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const __grid_constant__ SceneView sv_in, ShadowBuf sb,
                                                    const uint32_t *shadow_count, uint32_t *fetch, PathBuf nxt,
                                                    double *accum_in, double *weights_in, int *overflow,
                                                    unsigned long long *work, GuideView gv, BatchView bv)
@@ -454,9 +372,14 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __g
     const uint32_t count = *shadow_count;
     TravCount tc;
     KS_TRAV_STACK(stack);
-    TravState s;
-    const ShadowNode *nodes = tree_of<ShadowNode>(sv_in);
+    using View = TreeOf<kDeep>;
+    typename View::State s;
+    typename View::Tree tree = View::tree(sv_in);
     const float4 *tris = sv_in.prim_tris;
+    using Alpha = std::conditional_t<kAlpha, SceneAlpha, NoAlpha>;
+    Alpha filter;
+    if constexpr (kAlpha)
+        filter.sv = &sv_in;
     uint32_t ray = ~0u;
     bool drained = false;
     int of = 0;
@@ -465,7 +388,7 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __g
         if (id != ~0u) {
             const uint32_t job = kBatch ? bits(sb.contrib[id].w) : 0u;
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
-            nodes = tree_of<ShadowNode>(sv);
+            tree = View::tree(sv);
             tris = sv.prim_tris;
             float4 a = sb.o_tmax[id], b = sb.d_target[id];
             RayQuery q;
@@ -473,7 +396,7 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __g
             q.d = mk(b.x, b.y, b.z);
             q.tmin = 0.0f;
             q.tmax = a.w;
-            if (trav_begin(s, q, sv.root_ref, sv.root_count, sv.bmin, sv.bmax))
+            if (trav_begin(s, q, View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
             else
                 shadow_done<kBatch>(sb, id, false, nxt, accum_in, weights_in, gv, bv);
@@ -484,12 +407,7 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __g
             continue;
         }
         while (true) {
-            bool done;
-            if constexpr (kAlpha)
-                done = trav_warp_step<true>(nodes, tris, s, stack, 2, of, &tc, ray != ~0u, SceneAlpha{&sv_in});
-            else
-                done = trav_warp_step<true>(nodes, tris, s, stack, 2, of, &tc, ray != ~0u);
-            if (done) {
+            if (trav_warp_step<true>(tree, tris, s, stack, 2, of, &tc, ray != ~0u, filter)) {
                 shadow_done<kBatch>(sb, ray, s.hit.tri != ~0u, nxt, accum_in, weights_in, gv, bv);
                 ray = ~0u;
             }
@@ -507,11 +425,6 @@ __global__ void __launch_bounds__(128, KS_TRAV_MIN_BLOCKS) k_shadow_pt(const __g
 #ifndef KS_INST_MIN_BLOCKS
 #define KS_INST_MIN_BLOCKS 1
 #endif
-// BLAS layout of the instanced kernels: the SBVH nodes (0) or their 4-wide view (1).
-#ifndef KS_WIDE_INST
-#define KS_WIDE_INST 1
-#endif
-using InstNode = std::conditional_t<KS_WIDE_INST != 0, WideNode, TravNode>;
 // The same warp-level ray fetch as k_extend_pt / k_shadow_pt over inst_step (ks_traverse.cuh):
 // each ray makes the tests of traverse_instances, in resumable steps.
 __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_extend_inst_pt(const __grid_constant__ SceneView sv, PathBuf pb,
@@ -528,13 +441,7 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_extend_inst_pt(cons
     while (true) {
         const uint32_t id = warp_fetch(fetch, count, ray == ~0u, drained);
         if (id != ~0u) {
-            float4 a = pb.o_pdf[id], b = pb.d_info[id];
-            RayQuery q;
-            q.o = mk(a.x, a.y, a.z);
-            q.d = mk(b.x, b.y, b.z);
-            q.tmin = 0.0f;
-            q.tmax = kInf;
-            if (inst_begin(s, sv.inst, q)) {
+            if (inst_begin(s, sv.inst, path_ray(pb, id))) {
                 ray = id;
             } else {
                 hits[id] = make_float4(0, 0, 0, fbits(~0u));
@@ -547,10 +454,9 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_extend_inst_pt(cons
             continue;
         }
         while (true) {
-            if (inst_warp_step<false>(tree_of<InstNode>(sv), sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc,
+            if (inst_warp_step<false>(sv.inst_wide, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc,
                                       ray != ~0u)) {
-                hits[ray] = s.hit.tri != ~0u ? make_float4(s.hit.t, s.hit.b1, s.hit.b2, fbits(s.hit.slot))
-                                             : make_float4(0, 0, 0, fbits(~0u));
+                hits[ray] = hit_record(s.hit);
                 hit_inst[ray] = s.hit_inst;
                 ray = ~0u;
             }
@@ -598,7 +504,7 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_shadow_inst_pt(cons
         }
         while (true) {
             if (ray != ~0u &&
-                inst_step<true>(tree_of<InstNode>(sv), sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc)) {
+                inst_step<true>(sv.inst_wide, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc)) {
                 shadow_done<false>(sb, ray, s.hit.tri != ~0u, nxt, accum, weights, gv, BatchView{});
                 ray = ~0u;
             }
@@ -1026,12 +932,15 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     const unsigned max_grid = (unsigned)ctx->sm_count * 16;
     // opacity maps: the traversal kernels with the candidate-hit filter (flat scenes)
     const bool alpha = scene->any_opacity;
-    const unsigned ext_grid = alpha ? resident_grid(k_extend_pt<false, true>, 128, ctx->sm_count)
-                                    : resident_grid(k_extend_pt<false>, 128, ctx->sm_count);
-    const unsigned shadow_grid = alpha ? resident_grid(k_shadow_pt<false, true>, 128, ctx->sm_count)
-                                       : resident_grid(k_shadow_pt<false>, 128, ctx->sm_count);
-    const unsigned inst_ext_grid = resident_grid(k_extend_inst_pt, 128, ctx->sm_count);
-    const unsigned inst_shadow_grid = resident_grid(k_shadow_inst_pt, 128, ctx->sm_count);
+    // and the variants of trees too deep for the 4-wide view
+    const auto ext_kernel = scene->deep ? (alpha ? k_extend_pt<false, true, true> : k_extend_pt<false, false, true>)
+                                        : (alpha ? k_extend_pt<false, true> : k_extend_pt<false>);
+    const auto shadow_kernel = scene->deep ? (alpha ? k_shadow_pt<false, true, true> : k_shadow_pt<false, false, true>)
+                                           : (alpha ? k_shadow_pt<false, true> : k_shadow_pt<false>);
+    const unsigned ext_grid = scene->n_instances ? resident_grid(k_extend_inst_pt, 128, ctx->sm_count)
+                                                 : resident_grid(ext_kernel, 128, ctx->sm_count);
+    const unsigned shadow_grid = scene->n_instances ? resident_grid(k_shadow_inst_pt, 128, ctx->sm_count)
+                                                    : resident_grid(shadow_kernel, 128, ctx->sm_count);
     int cur = 0;
     cudaError_t err = cudaSuccess;
     std::vector<double> cb_acc, cb_w;
@@ -1069,34 +978,16 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             cudaMemsetAsync(w.counters.ptr, 0, sizeof(uint32_t) * kCounters, st);
             unsigned grid = std::min<unsigned>((count + 127) / 128, max_grid);
             cudaEventRecord(ev[1], st);
-            if (scene->n_instances) {
-                if (kPersistentTraversal) {
-                    k_extend_inst_pt<<<std::min(grid, inst_ext_grid), 128, 0, st>>>(
-                        sv, pb[cur], count, w.hits.ptr, w.hit_inst.ptr, w.counters.ptr + 4, w.overflow.ptr, work.ptr);
-                    k_build_queues<false><<<std::min((count + 255) / 256, max_grid), 256, 0, st>>>(
-                        w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2, BatchView{});
-                    stats.kernel_launches++;
-                } else {
-                    k_extend<true><<<grid, 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, w.hit_inst.ptr,
-                                                         w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2,
-                                                         w.overflow.ptr, work.ptr, BatchView{});
-                }
-            } else if (!kPersistentTraversal)
-                k_extend<false><<<grid, 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, nullptr, w.queue[0].ptr,
-                                                      w.queue[1].ptr, w.counters.ptr + 2, w.overflow.ptr, work.ptr,
-                                                      BatchView{});
-            else {
-                if (alpha)
-                    k_extend_pt<false, true><<<std::min(grid, ext_grid), 128, 0, st>>>(
-                        sv, pb[cur], count, w.hits.ptr, w.counters.ptr + 4, w.overflow.ptr, work.ptr, BatchView{});
-                else
-                    k_extend_pt<false><<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr,
-                                                                                 w.counters.ptr + 4, w.overflow.ptr,
-                                                                                 work.ptr, BatchView{});
-                k_build_queues<false><<<std::min((count + 255) / 256, max_grid), 256, 0, st>>>(
-                    w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2, BatchView{});
-                stats.kernel_launches++;
-            }
+            if (scene->n_instances)
+                k_extend_inst_pt<<<std::min(grid, ext_grid), 128, 0, st>>>(
+                    sv, pb[cur], count, w.hits.ptr, w.hit_inst.ptr, w.counters.ptr + 4, w.overflow.ptr, work.ptr);
+            else
+                ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, w.counters.ptr + 4,
+                                                                     w.overflow.ptr, work.ptr, BatchView{});
+            k_build_queues<false><<<std::min((count + 255) / 256, max_grid), 256, 0, st>>>(
+                sv, pb[cur], w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2,
+                w.overflow.ptr, alpha, BatchView{});
+            stats.kernel_launches++;
             cudaEventRecord(ev[2], st);
             const bool guiding = guide && gv.active;
             if (guiding) {
@@ -1139,25 +1030,14 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                              w.counters.ptr, sb, w.counters.ptr + 1, d_accum, d_weights, gv, BatchView{});
             }
             cudaEventRecord(ev[3], st);
-            if (scene->n_instances) {
-                if (kPersistentTraversal)
-                    k_shadow_inst_pt<<<std::min(grid, inst_shadow_grid), 128, 0, st>>>(
-                        sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights,
-                        w.overflow.ptr, work.ptr + 2, gv);
-                else
-                    k_shadow<true><<<grid, 128, 0, st>>>(sv, sb, w.counters.ptr + 1, pb[1 - cur], d_accum, d_weights,
-                                                         w.overflow.ptr, work.ptr + 2, gv, BatchView{});
-            } else if (!kPersistentTraversal)
-                k_shadow<false><<<grid, 128, 0, st>>>(sv, sb, w.counters.ptr + 1, pb[1 - cur], d_accum, d_weights,
-                                                      w.overflow.ptr, work.ptr + 2, gv, BatchView{});
-            else if (alpha)
-                k_shadow_pt<false, true><<<std::min(grid, shadow_grid), 128, 0, st>>>(
+            if (scene->n_instances)
+                k_shadow_inst_pt<<<std::min(grid, shadow_grid), 128, 0, st>>>(
+                    sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
+                    work.ptr + 2, gv);
+            else
+                shadow_kernel<<<std::min(grid, shadow_grid), 128, 0, st>>>(
                     sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
                     work.ptr + 2, gv, BatchView{});
-            else
-                k_shadow_pt<false><<<std::min(grid, shadow_grid), 128, 0, st>>>(sv, sb, w.counters.ptr + 1, w.counters.ptr + 5,
-                                                                pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
-                                                                work.ptr + 2, gv, BatchView{});
             cudaEventRecord(ev[4], st);
             stats.kernel_launches += 5;
             cudaMemcpyAsync(h_counts, w.counters.ptr, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost, st);
@@ -1286,6 +1166,7 @@ struct BatchWork
     DevBuf<float> filters; // the jobs' pixel-filter sample tables, concatenated
     unsigned ext_grid = 0, shadow_grid = 0; // one wave of resident CTAs of the traversal kernels
     int variant = kShadePlain;              // the shading kernel variant of the most demanding job
+    bool deep = false;                      // some job's tree is too deep for the 4-wide view
 };
 
 // Validates the jobs and fills the per-job tables; returns the total path count in *total.
@@ -1302,6 +1183,7 @@ static ks_status batch_tables(ks_context *ctx, const ks_batch_job *jobs, uint32_
     std::vector<size_t> filter_off(n, 0);
     *max_bounces = 0;
     w.variant = kShadePlain;
+    w.deep = false;
     for (uint32_t j = 0; j < n; ++j) {
         const ks_batch_job &jb = jobs[j];
         const ks_small_pt_params &in = jb.params;
@@ -1335,6 +1217,7 @@ static ks_status batch_tables(ks_context *ctx, const ks_batch_job *jobs, uint32_
                                                      "with ks_small_pt_render)");
         views[j] = make_view(jb.scene);
         w.variant = std::max(w.variant, views[j].shade_variant);
+        w.deep = w.deep || jb.scene->deep;
         acc[j] = jb.accum_rgb_device;
         wts[j] = jb.weights_device;
         begin[j + 1] = begin[j] + (unsigned long long)params[j].cw * params[j].ch * (unsigned long long)in.spp;
@@ -1373,16 +1256,19 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     const GuideView gv{};
     k_batch_prep<<<1, 32, 0, st>>>(bv.state, cnt, capacity);
     k_raygen_batch<<<(unsigned)ctx->sm_count * 8, 256, 0, st>>>(bv, pb[cur]);
-    k_extend_pt<true><<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, cnt + 4, w.overflow.ptr,
+    const auto ext_kernel = w.deep ? k_extend_pt<true, false, true> : k_extend_pt<true>;
+    const auto shadow_kernel = w.deep ? k_shadow_pt<true, false, true> : k_shadow_pt<true>;
+    ext_kernel<<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, cnt + 4, w.overflow.ptr,
                                                 w.work.ptr, bv);
-    k_build_queues<true><<<grid, 256, 0, st>>>(w.hits.ptr, 0u, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, bv);
+    k_build_queues<true><<<grid, 256, 0, st>>>(SceneView{}, pb[cur], w.hits.ptr, 0u, w.queue[0].ptr,
+                                               w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, bv);
     launch_sample(true, grid, st, SceneView{}, RenderParams{}, pb[cur], w.hits.ptr, nullptr, w.queue[0].ptr, cnt + 2,
                   w.samples.ptr, bv);
     for (int miss = 0; miss < 2; ++miss)
         launch_shade(miss != 0, false, true, w.variant, grid, st, SceneView{}, RenderParams{}, pb[cur], pb[1 - cur], w.hits.ptr,
                      nullptr, w.samples.ptr, w.queue[miss].ptr, cnt + 2 + miss, cnt, sb, cnt + 1, nullptr, nullptr,
                      gv, bv);
-    k_shadow_pt<true><<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
+    shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
                                                    w.overflow.ptr, w.work.ptr + 2, gv, bv);
     k_batch_advance<<<1, 32, 0, st>>>(bv.state, cnt, handle, use_graph);
 }
@@ -1401,8 +1287,10 @@ static ks_status batch_render(ks_context *ctx, const ks_batch_job *jobs, uint32_
         (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(o.capacity ? o.capacity : 1u << 22,
                                                                                total));
     const unsigned grid = (unsigned)ctx->sm_count * (o.grid_per_sm ? std::min(o.grid_per_sm, 64u) : 16u);
-    w.ext_grid = resident_grid(k_extend_pt<true>, 128, ctx->sm_count);
-    w.shadow_grid = resident_grid(k_shadow_pt<true>, 128, ctx->sm_count);
+    w.ext_grid = w.deep ? resident_grid(k_extend_pt<true, false, true>, 128, ctx->sm_count)
+                        : resident_grid(k_extend_pt<true>, 128, ctx->sm_count);
+    w.shadow_grid = w.deep ? resident_grid(k_shadow_pt<true, false, true>, 128, ctx->sm_count)
+                           : resident_grid(k_shadow_pt<true>, 128, ctx->sm_count);
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < 4; ++f)
             KS_CUDA_TRY(ctx, w.state[b][f].alloc(capacity));

@@ -19,6 +19,7 @@
 // can differ from the reference (it depends on std::partition's swap order).
 #include "ks_scan.cuh"
 #include "ks_scene.h"
+#include "ks_traverse4.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -814,9 +815,9 @@ __global__ void k_emit(const BuildRec *recs, uint32_t n, const uint32_t *pool, R
 // Leaf children carry their primitive count (the count the reference's traversal derives from
 // primOffset differences, cuda/sbvh.cu:546-552).
 // Also marks each leaf child's last primitive (kLastPrim in the w component of its second vertex,
-// written after k_prim_tris), where the resumable traversal ends the leaf.
+// written after k_prim_tris), where the resumable traversal ends the leaf, and writes the leaf's box.
 __global__ void k_trav(const BuildRec *recs, uint32_t n, const uint32_t *interior_scan, TravNode *trav,
-                       float4 *prim_tris)
+                       float4 *prim_tris, float4 *leaf_box)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -833,14 +834,18 @@ __global__ void k_trav(const BuildRec *recs, uint32_t n, const uint32_t *interio
     t.c = make_float4(R.bmin[2], R.bmax[0], R.bmax[1], R.bmax[2]);
     t.d = make_uint4(ref_of(L), ref_of(R), L.prims | (p.axis << 30), R.prims);
     trav[interior_scan[p.dfs]] = t;
-    if (L.leaf && L.prims)
-        prim_tris[3 * (size_t)(L.prim_off + L.prims - 1) + 1].w = __uint_as_float(kLastPrim);
-    if (R.leaf && R.prims)
-        prim_tris[3 * (size_t)(R.prim_off + R.prims - 1) + 1].w = __uint_as_float(kLastPrim);
+    for (const BuildRec *c : {&L, &R}) {
+        if (!c->leaf || !c->prims)
+            continue;
+        prim_tris[3 * (size_t)(c->prim_off + c->prims - 1) + 1].w = __uint_as_float(kLastPrim);
+        leaf_box[2 * (size_t)c->prim_off] = make_float4(c->bmin[0], c->bmin[1], c->bmin[2], 0.0f);
+        leaf_box[2 * (size_t)c->prim_off + 1] = make_float4(c->bmax[0], c->bmax[1], c->bmax[2], 0.0f);
+    }
 }
 
+// recs[0] is the root: the box of the leaf when the whole tree is one.
 __global__ void k_prim_tris(const uint32_t *prims, uint32_t n_prims, const float *verts, const uint32_t *idx,
-                            float4 *out)
+                            const BuildRec *recs, float4 *out, float4 *leaf_box)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_prims)
@@ -854,6 +859,10 @@ __global__ void k_prim_tris(const uint32_t *prims, uint32_t n_prims, const float
     v[0].w = __uint_as_float(t);
     if (i + 1 == n_prims) // ends the last leaf (the whole tree may be one)
         v[1].w = __uint_as_float(kLastPrim);
+    if (i == 0) {
+        leaf_box[0] = make_float4(recs[0].bmin[0], recs[0].bmin[1], recs[0].bmin[2], 0.0f);
+        leaf_box[1] = make_float4(recs[0].bmax[0], recs[0].bmax[1], recs[0].bmax[2], 0.0f);
+    }
     out[3 * i + 0] = v[0];
     out[3 * i + 1] = v[1];
     out[3 * i + 2] = v[2];
@@ -870,8 +879,8 @@ struct RangeOut
     DevBuf<RefNode> ref_nodes;
     DevBuf<uint32_t> prims;
     DevBuf<TravNode> trav;
-    DevBuf<float4> prim_tris;
-    uint32_t n_nodes = 0, n_prims = 0, n_trav = 0;
+    DevBuf<float4> prim_tris, leaf_box;
+    uint32_t n_nodes = 0, n_prims = 0, n_trav = 0, n_levels = 0;
     float bound[6] = {0, 0, 0, 0, 0, 0};
 };
 
@@ -889,6 +898,8 @@ struct BuildScratch
     DevBuf<NodeInfo> info;
     DevBuf<uint32_t> bnd, obj, sp, item_cnt, item_off, cl, cr, cp, sl, sr, spool, split_flag, split_scan, pool, flag;
     DevBuf<uint32_t> interior_flag, interior_scan;
+    DevBuf<uint32_t> wide_binary, wide_child, wide_level;
+    DevBuf<float> wide_bound;
     DevBuf<BuildRec> recs;
     ScanScratch scan;
 };
@@ -1052,10 +1063,11 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     KS_CUDA_TRY(ctx, out.trav.alloc(n_trav > 0 ? n_trav : 1));
     KS_CUDA_TRY(ctx, out.prim_tris.alloc((size_t)pool_used * 3));
-    k_prim_tris<<<grid_for(pool_used, 256), 256, 0, st>>>(out.prims.ptr, pool_used, verts, indices,
-                                                          out.prim_tris.ptr);
+    KS_CUDA_TRY(ctx, out.leaf_box.alloc((size_t)pool_used * 2));
+    k_prim_tris<<<grid_for(pool_used, 256), 256, 0, st>>>(out.prims.ptr, pool_used, verts, indices, recs.ptr,
+                                                          out.prim_tris.ptr, out.leaf_box.ptr);
     k_trav<<<grid_for(n_nodes, 256), 256, 0, st>>>(recs.ptr, n_nodes, interior_scan.ptr, out.trav.ptr,
-                                                   out.prim_tris.ptr);
+                                                   out.prim_tris.ptr, out.leaf_box.ptr);
     KS_CUDA_TRY(ctx, cudaGetLastError());
     if (done)
         KS_CUDA_TRY(ctx, cudaEventRecord(done, st));
@@ -1069,61 +1081,180 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     out.n_nodes = n_nodes;
     out.n_prims = pool_used;
     out.n_trav = n_trav;
+    out.n_levels = (uint32_t)level_begin.size() - 1;
     return KS_OK;
 }
 
-// BLAS concatenation: interior refs move by the node base, leaf refs by the slot base.
-// Wide node i from interior node i: its leaf children as they are, its interior children replaced
-// by their two children (boxes and refs read from the child's node).
-__global__ void k_widen(const TravNode *nodes, uint32_t n, WideNode *wide)
+// ---- the renderer's 4-wide view (Wide4Node) ----------------------------------------------------
+// Built from the binary nodes level by level.  A wide node opens its binary node: two children, then
+// the interior child of the largest area replaced by its own two, until there are 4 or only leaves.
+// k_wide4_alloc finds each node's interior children and gives them nodes of the next level (one atomic
+// per node); k_wide4_fill then writes all nodes at once, opening each the same way again.
+struct Opened4
+{
+    float lo[4][3], hi[4][3];
+    uint32_t ref[4];
+    int n;
+};
+
+__device__ __forceinline__ void open4(const TravNode *__restrict__ nodes, uint32_t ref, Opened4 &c)
+{
+    float area[4]; // of interior children
+    auto put = [&](int at, const TravNode &t, int side) {
+        const float4 A = t.a, B = t.b, C = t.c;
+        const float l0[3] = {A.x, A.y, A.z}, h0[3] = {A.w, B.x, B.y};
+        const float l1[3] = {B.z, B.w, C.x}, h1[3] = {C.y, C.z, C.w};
+        for (int a = 0; a < 3; ++a) {
+            c.lo[at][a] = side ? l1[a] : l0[a];
+            c.hi[at][a] = side ? h1[a] : h0[a];
+        }
+        c.ref[at] = side ? t.d.y : t.d.x;
+        const float x = c.hi[at][0] - c.lo[at][0], y = c.hi[at][1] - c.lo[at][1], z = c.hi[at][2] - c.lo[at][2];
+        area[at] = x * y + y * z + z * x;
+    };
+    {
+        const TravNode t = nodes[ref];
+        put(0, t, 0);
+        put(1, t, 1);
+    }
+    c.n = 2;
+    while (c.n < 4) {
+        int best = -1;
+        for (int k = 0; k < c.n; ++k)
+            if (!(c.ref[k] & kLeafBit) && (best < 0 || area[k] > area[best]))
+                best = k;
+        if (best < 0)
+            break;
+        const TravNode t = nodes[c.ref[best]];
+        for (int k = c.n; k > best + 1; --k) { // the two children take their parent's place
+            for (int a = 0; a < 3; ++a) {
+                c.lo[k][a] = c.lo[k - 1][a];
+                c.hi[k][a] = c.hi[k - 1][a];
+            }
+            c.ref[k] = c.ref[k - 1];
+            area[k] = area[k - 1];
+        }
+        put(best, t, 0);
+        put(best + 1, t, 1);
+        ++c.n;
+    }
+}
+
+// Level `level` of the view: binary[i] is wide node i's binary node (kLeafBit: a tree that is one
+// leaf), level_n[l] the nodes of level l (complete below `level` + 1), child[i] the first child.
+__global__ void k_wide4_alloc(const TravNode *__restrict__ nodes, uint32_t level, uint32_t *level_n, uint32_t *binary,
+                              uint32_t *child)
+{
+    uint32_t begin = 0;
+    for (uint32_t l = 0; l < level; ++l)
+        begin += level_n[l];
+    const uint32_t n = level_n[level], next = begin + n;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t ref = binary[begin + i];
+        if (ref & kLeafBit) {
+            child[begin + i] = 0;
+            continue;
+        }
+        Opened4 c;
+        open4(nodes, ref, c);
+        uint32_t inner = 0;
+        for (int k = 0; k < c.n; ++k)
+            inner += (c.ref[k] & kLeafBit) ? 0u : 1u;
+        uint32_t at = inner ? next + atomicAdd(&level_n[level + 1], inner) : 0u;
+        child[begin + i] = at;
+        for (int k = 0; k < c.n; ++k)
+            if (!(c.ref[k] & kLeafBit))
+                binary[at++] = c.ref[k];
+    }
+}
+
+// root_bound: the root's box, read when the tree is one leaf.
+__global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, const uint32_t *__restrict__ binary,
+                             const uint32_t *__restrict__ child, const float *__restrict__ root_bound, Wide4Node *out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    float lo[3][4], hi[3][4];
-    uint32_t ref[4], cnt[4];
+    const uint32_t ref = binary[i];
+    Opened4 c;
+    if (ref & kLeafBit) {
+        c.n = 1;
+        for (int a = 0; a < 3; ++a) {
+            c.lo[0][a] = root_bound[a];
+            c.hi[0][a] = root_bound[3 + a];
+        }
+        c.ref[0] = ref;
+    } else {
+        open4(nodes, ref, c);
+    }
+    Wide4Node w;
+    float *plane = reinterpret_cast<float *>(w.plane);
+    uint32_t next = child[i];
     for (int k = 0; k < 4; ++k) {
         for (int a = 0; a < 3; ++a) {
-            lo[a][k] = __int_as_float(0x7f800000);  // +inf
-            hi[a][k] = __int_as_float(0xff800000);  // -inf
+            plane[8 * a + k] = k < c.n ? c.lo[k][a] : kInf;
+            plane[8 * a + 4 + k] = k < c.n ? c.hi[k][a] : -kInf;
         }
-        ref[k] = kLeafBit;
-        cnt[k] = 0;
+        w.ref[k] = k >= c.n ? kLeafBit : (c.ref[k] & kLeafBit) ? c.ref[k] : next++;
+        w.pad[k] = 0;
     }
-    int m = 0;
-    auto put = [&](const TravNode &nd, int side) {
-        const float4 A = nd.a, B = nd.b, C = nd.c;
-        const float l0[3] = {A.x, A.y, A.z}, h0[3] = {A.w, B.x, B.y};
-        const float l1[3] = {B.z, B.w, C.x}, h1[3] = {C.y, C.z, C.w};
-        for (int a = 0; a < 3; ++a) {
-            lo[a][m] = side ? l1[a] : l0[a];
-            hi[a][m] = side ? h1[a] : h0[a];
-        }
-        ref[m] = side ? nd.d.y : nd.d.x;
-        cnt[m] = side ? nd.d.w : (nd.d.z & 0x3fffffffu);
-        ++m;
-    };
-    const TravNode nd = nodes[i];
-    for (int side = 0; side < 2; ++side) {
-        const uint32_t r = side ? nd.d.y : nd.d.x;
-        if (r & kLeafBit) {
-            put(nd, side);
-        } else {
-            const TravNode c = nodes[r];
-            put(c, 0);
-            put(c, 1);
-        }
-    }
-    WideNode w;
-    for (int a = 0; a < 3; ++a) {
-        w.lo[a] = make_float4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
-        w.hi[a] = make_float4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
-    }
-    w.ref = make_uint4(ref[0], ref[1], ref[2], ref[3]);
-    w.cnt = make_uint4(cnt[0], cnt[1], cnt[2], cnt[3]);
-    wide[i] = w;
+    out[i] = w;
 }
 
+// The view of the tree over `nodes` whose root is root_ref with box root_bound (6 floats), into out (node 0:
+// the root).  Launches kWide4Chunk levels between two looks at the counts (a level without nodes costs its
+// launch); max_levels: levels of the binary tree.
+static ks_status build_wide4(ks_context *ctx, BuildScratch &bs, const TravNode *nodes, uint32_t n_trav, uint32_t root_ref,
+                             const float *root_bound, uint32_t max_levels, DevBuf<Wide4Node> &out, bool &too_deep)
+{
+    constexpr uint32_t kWide4Chunk = 16;
+    cudaStream_t st = ctx->stream;
+    const uint32_t levels = max_levels + kWide4Chunk + 1, one = 1;
+    KS_CUDA_TRY(ctx, bs.wide_binary.reserve((size_t)n_trav + 1));
+    KS_CUDA_TRY(ctx, bs.wide_child.reserve((size_t)n_trav + 1));
+    KS_CUDA_TRY(ctx, bs.wide_level.reserve(levels));
+    KS_CUDA_TRY(ctx, bs.wide_bound.reserve(6));
+    KS_CUDA_TRY(ctx, cudaMemsetAsync(bs.wide_level.ptr, 0, sizeof(uint32_t) * levels, st));
+    KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_level.ptr, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_binary.ptr, &root_ref, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_bound.ptr, root_bound, sizeof(float) * 6, cudaMemcpyHostToDevice, st));
+    std::vector<uint32_t> count(levels, 0);
+    count[0] = 1;
+    uint32_t done = 0;
+    while (done < levels && count[done]) {
+        const uint32_t end = std::min(done + kWide4Chunk, levels - 1);
+        if (end == done)
+            return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: 4-wide level limit reached");
+        for (; done < end; ++done)
+            k_wide4_alloc<<<(unsigned)ctx->sm_count * 4, 128, 0, st>>>(nodes, done, bs.wide_level.ptr, bs.wide_binary.ptr,
+                                                                       bs.wide_child.ptr);
+        KS_CUDA_TRY(ctx, cudaMemcpyAsync(count.data(), bs.wide_level.ptr, sizeof(uint32_t) * levels,
+                                         cudaMemcpyDeviceToHost, st));
+        KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    }
+    uint32_t n = 0, wide_levels = 0;
+    for (uint32_t c : count) {
+        n += c;
+        wide_levels += c ? 1 : 0;
+    }
+    too_deep = wide_levels > kMaxWideLevels;
+    if (too_deep)
+        return KS_OK;
+    KS_CUDA_TRY(ctx, out.alloc(n));
+    k_wide4_fill<<<grid_for(n, 128), 128, 0, st>>>(nodes, n, bs.wide_binary.ptr, bs.wide_child.ptr, bs.wide_bound.ptr,
+                                                   out.ptr);
+    KS_CUDA_TRY(ctx, cudaGetLastError());
+    return KS_OK;
+}
+
+__global__ void k_widen(const TravNode *nodes, uint32_t n, WideNode *wide)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        wide[i] = widen(reinterpret_cast<const LazyWide *>(nodes), i);
+}
+
+// BLAS concatenation: interior refs move by the node base, leaf refs by the slot base.
 __global__ void k_offset_trav(const TravNode *src, uint32_t n, uint32_t node_base, uint32_t slot_base, TravNode *dst)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1283,10 +1414,10 @@ static ks_status build_instanced(ks_scene *scene, const Params &p)
         slot_base += r.n_prims;
     }
     KS_CUDA_TRY(ctx, cudaGetLastError());
-    // the renderer's 4-wide view of the concatenated BLAS nodes (their refs are already global)
-    KS_CUDA_TRY(ctx, scene->wide_nodes.alloc(total_trav > 0 ? total_trav : 1));
+    // 4-wide steps over the concatenated BLAS nodes (their refs are already global)
+    KS_CUDA_TRY(ctx, scene->inst_wide.alloc(total_trav > 0 ? total_trav : 1));
     if (total_trav > 0)
-        k_widen<<<grid_for(total_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, total_trav, scene->wide_nodes.ptr);
+        k_widen<<<grid_for(total_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, total_trav, scene->inst_wide.ptr);
     // instance boxes: the 8 corners of the prototype box, transformed, padded by a relative epsilon
     TlasBuilder tb;
     for (uint32_t i = 0; i < scene->n_instances; ++i) {
@@ -1379,6 +1510,7 @@ ks_status build_sbvh(ks_scene *scene, const ks_sbvh_options &o, float *build_ms)
             scene->prims.swap(r.prims);
             scene->trav_nodes.swap(r.trav);
             scene->prim_tris.swap(r.prim_tris);
+            scene->leaf_box.swap(r.leaf_box);
             std::memcpy(scene->scene_bound, r.bound, sizeof(r.bound));
             scene->n_nodes = r.n_nodes;
             scene->n_prims = r.n_prims;
@@ -1386,14 +1518,14 @@ ks_status build_sbvh(ks_scene *scene, const ks_sbvh_options &o, float *build_ms)
             scene->root_count = r.n_prims;
             scene->root_ref = r.n_trav > 0 ? 0u : kLeafBit;
             // the renderer's 4-wide view of the tree (timed with the build)
-            if (scene->wide_nodes.alloc(r.n_trav > 0 ? r.n_trav : 1) != cudaSuccess) {
-                s = fail(ctx, KS_ERR_OUT_OF_MEMORY, "ks_scene_build_bvh: wide nodes");
-            } else if (r.n_trav > 0) {
+            scene->deep = r.n_levels > kMaxBinaryLevels;
+            scene->wide_nodes.release();
+            if (!scene->deep) {
                 cudaEventRecord(ev2, st);
-                k_widen<<<grid_for(r.n_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, r.n_trav,
-                                                                  scene->wide_nodes.ptr);
+                s = build_wide4(ctx, build_scratch(ctx), scene->trav_nodes.ptr, r.n_trav, scene->root_ref, r.bound,
+                                r.n_levels, scene->wide_nodes, scene->deep);
                 cudaEventRecord(ev3, st);
-                widened = true;
+                widened = s == KS_OK;
             }
         }
     }

@@ -1,13 +1,14 @@
 // Scene lifetime, SBVH build/export entry points and the ray-query parity kernel.
 #include "ks_lights.cuh"
 #include "ks_scene.h"
-#include "ks_traverse.cuh"
+#include "ks_traverse4.cuh"
 
 #include <atomic>
 #include <cmath>
 
 #include <cstring>
 #include <new>
+#include <type_traits>
 
 using namespace ksb;
 
@@ -18,6 +19,18 @@ SceneView make_view(const ks_scene *s);
 
 namespace
 {
+
+// Ray i of a batch of host rays (8 floats each).
+KS_D RayQuery host_ray(const float *rays, uint32_t i)
+{
+    const float *r = rays + 8 * (size_t)i;
+    RayQuery q;
+    q.o = mk(r[0], r[1], r[2]);
+    q.tmin = r[3];
+    q.d = mk(r[4], r[5], r[6]);
+    q.tmax = r[7];
+    return q;
+}
 
 __global__ void trace_kernel(const TravNode *nodes, const float4 *tris, uint32_t root_ref, uint32_t root_count,
                              float bx0, float by0, float bz0, float bx1, float by1, float bz1, const float *rays,
@@ -62,18 +75,19 @@ __global__ void trace_kernel(const TravNode *nodes, const float4 *tris, uint32_t
 }
 
 // ks_trace_rays for flat scenes: the same queries as trace_kernel, traversed by trav_step with
-// dynamic ray fetch.  Node = TravNode: each ray makes the same tests as traverse() (same triangle, t
-// and barycentrics); Node = WideNode (ks_trace_rays_wide): the renderer's 4-wide traversal.
-template <class Node>
-__global__ void __launch_bounds__(128) trace_kernel_pt(const Node *nodes, const float4 *tris, uint32_t root_ref,
-                                                       uint32_t root_count, float bx0, float by0, float bz0, float bx1,
+// dynamic ray fetch.  Tree = const TravNode *: each ray makes the same tests as traverse() (same triangle, t
+// and barycentrics); Tree = Tree4 or, in deep trees, const LazyWide * (ks_trace_rays_wide): the renderer's
+// traversal, State its state; nodes_wide and root_wide are the tree it walks.
+template <class Tree, class State>
+__global__ void __launch_bounds__(128) trace_kernel_pt(const Tree nodes_wide, uint32_t root_wide, const TravNode *nodes,
+                                                       const float4 *tris, uint32_t root_ref, uint32_t root_count, float bx0, float by0, float bz0, float bx1,
                                                        float by1, float bz1, const float *rays, uint32_t n, int any_hit,
                                                        int culling, uint32_t *tri_out, float *t_out, float *bary_out,
                                                        int *overflow_flag, uint32_t *fetch)
 {
     const float bmin[3] = {bx0, by0, bz0}, bmax[3] = {bx1, by1, bz1};
     KS_TRAV_STACK(stack);
-    TravState s;
+    State s;
     uint32_t ray = ~0u;
     bool drained = false;
     int overflow = 0;
@@ -91,13 +105,7 @@ __global__ void __launch_bounds__(128) trace_kernel_pt(const Node *nodes, const 
     while (true) {
         const uint32_t id = warp_fetch(fetch, n, ray == ~0u, drained);
         if (id != ~0u) {
-            const float *r = rays + 8 * (size_t)id;
-            RayQuery q;
-            q.o = mk(r[0], r[1], r[2]);
-            q.tmin = r[3];
-            q.d = mk(r[4], r[5], r[6]);
-            q.tmax = r[7];
-            if (trav_begin(s, q, root_ref, root_count, bmin, bmax))
+            if (trav_begin(s, host_ray(rays, id), root_wide, root_count, bmin, bmax))
                 ray = id;
             else
                 finish(id, s.hit);
@@ -109,9 +117,16 @@ __global__ void __launch_bounds__(128) trace_kernel_pt(const Node *nodes, const 
         }
         while (true) {
             const bool done =
-                any_hit ? trav_warp_step<true>(nodes, tris, s, stack, culling, overflow, nullptr, ray != ~0u)
-                        : trav_warp_step<false>(nodes, tris, s, stack, culling, overflow, nullptr, ray != ~0u);
+                any_hit ? trav_warp_step<true>(nodes_wide, tris, s, stack, culling, overflow, nullptr, ray != ~0u)
+                        : trav_warp_step<false>(nodes_wide, tris, s, stack, culling, overflow, nullptr, ray != ~0u);
             if (done) {
+                if constexpr (std::is_same_v<State, Trav4>)
+                    if (!any_hit && ambiguous(s)) {
+                        const Retraced x = retrace(nodes, tris, root_ref, root_count, bmin, bmax, host_ray(rays, ray),
+                                                   culling);
+                        s.hit = x.hit;
+                        overflow |= x.overflow;
+                    }
                 finish(ray, s.hit);
                 ray = ~0u;
             }
@@ -125,9 +140,9 @@ __global__ void __launch_bounds__(128) trace_kernel_pt(const Node *nodes, const 
 }
 
 // ks_trace_rays_wide for instanced scenes: the renderer's persistent two-level traversal
-// (inst_step over the 4-wide view of the BLAS nodes).
+// (inst_step over 4-wide steps of the BLAS nodes).
 __global__ void __launch_bounds__(128) trace_inst_kernel_pt(const WideNode *nodes, const float4 *tris,
-                                                            InstanceView iv, const float *rays, uint32_t n,
+                                                            const __grid_constant__ InstanceView iv, const float *rays, uint32_t n,
                                                             int any_hit, int culling, uint32_t *tri_out,
                                                             float *t_out, float *bary_out, int *overflow_flag,
                                                             uint32_t *fetch)
@@ -152,13 +167,7 @@ __global__ void __launch_bounds__(128) trace_inst_kernel_pt(const WideNode *node
     while (true) {
         const uint32_t id = warp_fetch(fetch, n, ray == ~0u, drained);
         if (id != ~0u) {
-            const float *r = rays + 8 * (size_t)id;
-            RayQuery q;
-            q.o = mk(r[0], r[1], r[2]);
-            q.tmin = r[3];
-            q.d = mk(r[4], r[5], r[6]);
-            q.tmax = r[7];
-            if (inst_begin(s, iv, q))
+            if (inst_begin(s, iv, host_ray(rays, id)))
                 ray = id;
             else
                 finish(id, s.hit);
@@ -889,7 +898,7 @@ static ks_status trace_rays_impl(ks_scene *scene, const float *rays, uint32_t n,
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_inst_kernel_pt, 128, 0);
         const unsigned grid = std::min<unsigned>((n + 127) / 128, (unsigned)std::max(per_sm, 1) * ctx->sm_count);
-        trace_inst_kernel_pt<<<grid, 128, 0, st>>>(scene->wide_nodes.ptr, scene->prim_tris.ptr, make_view(scene).inst,
+        trace_inst_kernel_pt<<<grid, 128, 0, st>>>(scene->inst_wide.ptr, scene->prim_tris.ptr, make_view(scene).inst,
                                                    d_rays.ptr, n, any_hit, culling, d_tri.ptr, d_t.ptr, d_bary.ptr,
                                                    d_flag.ptr, d_fetch.ptr);
     } else if (scene->n_instances) {
@@ -901,21 +910,22 @@ static ks_status trace_rays_impl(ks_scene *scene, const float *rays, uint32_t n,
         KS_CUDA_TRY(ctx, d_fetch.alloc(1));
         KS_CUDA_TRY(ctx, cudaMemsetAsync(d_fetch.ptr, 0, sizeof(uint32_t), st));
         int per_sm = 1;
-        if (wide)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel_pt<WideNode>, 128, 0);
+        auto run = [&](auto kernel, auto nodes_wide, uint32_t root_wide) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
+            const unsigned grid = std::min<unsigned>((n + 127) / 128, (unsigned)std::max(per_sm, 1) * ctx->sm_count);
+            kernel<<<grid, 128, 0, st>>>(nodes_wide, root_wide, scene->trav_nodes.ptr, scene->prim_tris.ptr,
+                                         scene->root_ref, scene->root_count, b[0], b[1], b[2], b[3], b[4], b[5],
+                                         d_rays.ptr, n, any_hit, culling, d_tri.ptr, d_t.ptr, d_bary.ptr, d_flag.ptr,
+                                         d_fetch.ptr);
+        };
+        if (!wide)
+            run(trace_kernel_pt<const TravNode *, TravState>, static_cast<const TravNode *>(scene->trav_nodes.ptr),
+                scene->root_ref);
+        else if (scene->deep)
+            run(trace_kernel_pt<const LazyWide *, TravState>,
+                reinterpret_cast<const LazyWide *>(scene->trav_nodes.ptr), scene->root_ref);
         else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel_pt<TravNode>, 128, 0);
-        const unsigned grid = std::min<unsigned>((n + 127) / 128, (unsigned)std::max(per_sm, 1) * ctx->sm_count);
-        if (wide)
-            trace_kernel_pt<<<grid, 128, 0, st>>>(scene->wide_nodes.ptr, scene->prim_tris.ptr, scene->root_ref,
-                                                  scene->root_count, b[0], b[1], b[2], b[3], b[4], b[5], d_rays.ptr,
-                                                  n, any_hit, culling, d_tri.ptr, d_t.ptr, d_bary.ptr, d_flag.ptr,
-                                                  d_fetch.ptr);
-        else
-            trace_kernel_pt<<<grid, 128, 0, st>>>(scene->trav_nodes.ptr, scene->prim_tris.ptr, scene->root_ref,
-                                                  scene->root_count, b[0], b[1], b[2], b[3], b[4], b[5], d_rays.ptr,
-                                                  n, any_hit, culling, d_tri.ptr, d_t.ptr, d_bary.ptr, d_flag.ptr,
-                                                  d_fetch.ptr);
+            run(trace_kernel_pt<Tree4, Trav4>, Tree4{scene->wide_nodes.ptr, scene->leaf_box.ptr}, 0u);
     }
     KS_CUDA_TRY(ctx, cudaGetLastError());
     int overflow = 0;

@@ -32,19 +32,31 @@ constexpr uint32_t kLeafBit = 0x80000000u;
 // Bits of v1.w in a primitive's record (3 float4: v0 + triangle id, v1 + this mark, v2) that ends a leaf.
 constexpr uint32_t kLastPrim = 0x3f800000u;
 
-// 4-wide view of the same SBVH, read by the renderer's traversal kernels: wide node i holds the
-// children of interior node i, each interior child replaced by its own two children (2 to 4 slots).
-// Slot boxes are the SBVH's boxes of those nodes; unused slots hold an empty box (lo +inf, hi -inf),
-// which the slab test always rejects.  Indexed like the TravNode array (entries of nodes at odd
-// depth are written but never read), so child refs need no renumbering.
+// A node of the exact traversal's 4-wide steps (ks_traverse.cuh): the children of an interior node, each
+// interior child replaced by its own two children (2 to 4 slots, in order).  Slot boxes are the SBVH's
+// boxes of those nodes; unused slots hold an empty box (lo +inf, hi -inf), which the slab test always
+// rejects.  Instanced scenes keep them for every interior node (indexed like the TravNode array, so child
+// refs need no renumbering; entries of nodes at odd depth are written but never read).
 struct WideNode
 {
     float4 lo[3]; // per axis: the 4 slots' lower bounds
     float4 hi[3]; // per axis: the 4 slots' upper bounds
     uint4 ref;    // child refs (kLeafBit: leaf, first primitive slot)
-    uint4 cnt;    // primitive counts of leaf children
+    uint4 pad;
 };
 static_assert(sizeof(WideNode) == 128, "one 128-byte line per wide node");
+
+// The 4-wide view of the same SBVH that the renderer's traversal kernels read (ks_traverse4.cuh): a node
+// holds 1 to 4 nodes of the binary tree, found by replacing the largest interior child by its two
+// children until there are 4 (or leaves only), in their order.  Boxes are the SBVH's own; unused slots
+// hold an empty box, never hit.  Every tree has a root node here, also one that is a single leaf.
+struct __align__(128) Wide4Node
+{
+    float4 plane[6];    // x lower, x upper, y lower, ...: the 4 slots
+    uint32_t ref[4];    // child: node index, or kLeafBit | first primitive slot
+    uint32_t pad[4];
+};
+static_assert(sizeof(Wide4Node) == 128, "one 128-byte line per node");
 
 // Per-mesh shading flags (MeshData::twosided; use_smooth_normal with vertex normals given;
 // texcoords given).
@@ -110,7 +122,10 @@ struct ks_scene
     uint32_t n_nodes = 0, n_prims = 0;
     // traversal layout
     ksb::DevBuf<ksb::TravNode> trav_nodes;
-    ksb::DevBuf<ksb::WideNode> wide_nodes; // the 4-wide view of trav_nodes
+    ksb::DevBuf<ksb::Wide4Node> wide_nodes; // flat scenes: the renderer's 4-wide view of trav_nodes
+    ksb::DevBuf<ksb::WideNode> inst_wide;   // instanced scenes: 4-wide steps over trav_nodes
+    ksb::DevBuf<float4> leaf_box; // per leaf, at its first primitive slot: its box (2 float4: lower, upper corner)
+    bool deep = false; // the tree is too deep for the view's stack: the exact traversal over trav_nodes
     ksb::DevBuf<float4> prim_tris; // 3 float4 per primitive slot: v0 (+tri index bits in w), v1, v2
     uint32_t n_trav = 0;
     uint32_t root_ref = 0;   // ref of the root (leaf bit when the whole tree is one leaf)

@@ -308,6 +308,8 @@ struct TravState
     uint32_t ref;
     int sp;
     Hit hit;
+
+    KS_D bool at_leaf() const { return (ref & kLeafBit) != 0; }
 };
 
 KS_D BoxHelper box_helper_of(f3 inv)
@@ -347,6 +349,13 @@ struct TravStack
     }
     KS_D uint2 get(int i) const { return i < kSmemStack ? sm[i * kTravBlock] : loc[i - kSmemStack]; }
 };
+// A stack of one thread's own.
+struct LocalStack
+{
+    uint2 e[kWideStackDepth];
+    KS_D void set(int i, uint32_t ref, float t) { e[i] = make_uint2(ref, __float_as_uint(t)); }
+    KS_D uint2 get(int i) const { return e[i]; }
+};
 // The shared part of a block's stacks; every persistent traversal kernel declares one and points
 // each thread's TravStack at its column.
 #define KS_TRAV_STACK(name)                                                                                       \
@@ -376,7 +385,8 @@ KS_D bool trav_begin(TravState &s, const RayQuery &ray, uint32_t root_ref, uint3
 // Interior node test of trav_step: descends to the near child (pushing the far one when both are
 // hit) and returns 1, returns 0 when neither child is hit, and -1 with the overflow flag set when
 // the stack is full (the caller then ends the ray).
-KS_D int trav_interior(const TravNode *__restrict__ nodes, TravState &s, TravStack &stack, int &overflow,
+template <class Stack>
+KS_D int trav_interior(const TravNode *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
                         TravCount *count)
 {
     const TravNode *n = nodes + s.ref;
@@ -424,8 +434,8 @@ static __device__ __noinline__ WideHits wide_slabs_guarded(const WideNode *n, f3
     const float *lo = reinterpret_cast<const float *>(n->lo), *hi = reinterpret_cast<const float *>(n->hi);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float bmin[3] = {__ldg(lo + k), __ldg(lo + 4 + k), __ldg(lo + 8 + k)};
-        const float bmax[3] = {__ldg(hi + k), __ldg(hi + 4 + k), __ldg(hi + 8 + k)};
+        const float bmin[3] = {lo[k], lo[4 + k], lo[8 + k]};
+        const float bmax[3] = {hi[k], hi[4 + k], hi[8 + k]};
         float a, b;
         const bool ok = slab(ray, bh, bmin, bmax, a, b) && b > tmin && a < tmax;
         h.t[k] = a;
@@ -448,19 +458,25 @@ static __device__ __noinline__ WideHits wide_slabs_guarded(const WideNode *n, f3
 // instead of a sorting network over four values per slot and 8-byte stack entries the mesh frame
 // (1.3 M triangles, 1024 x 1024 x 64) went from 101.9 to 93.5 ms, the instanced one (1080p x 4) from
 // 41.3 to 38.0 ms, every image bit for bit the same.
-template <bool kAnyHit>
-KS_D int trav_wide(const WideNode *__restrict__ wide, TravState &s, TravStack &stack, int &overflow,
-                   TravCount *count)
+// kGlobal: the node lies in global memory (else it was just made, LazyWide).
+template <bool kAnyHit, bool kGlobal, class Stack>
+KS_D int trav_wide(const WideNode *wide, TravState &s, Stack &stack, int &overflow, TravCount *count)
 {
-    const char *n = reinterpret_cast<const char *>(wide + s.ref);
+    const char *n = reinterpret_cast<const char *>(wide);
     if (count)
-        count->nodes += 2; // 128 bytes: two 64-byte node units
-    const uint4 ref4 = __ldg(reinterpret_cast<const uint4 *>(n + 96));
+        count->nodes += kGlobal ? 2 : 3; // 64-byte node units (made: of the node and two children)
+    auto load = [](const auto *p) {
+        if constexpr (kGlobal)
+            return __ldg(p);
+        else
+            return *p;
+    };
+    const uint4 ref4 = load(reinterpret_cast<const uint4 *>(n + 96));
     const uint32_t refs[4] = {ref4.x, ref4.y, ref4.z, ref4.w};
     float t0[4];
     bool ok[4];
     if (!s.guard) {
-        auto plane = [&](int off) { return __ldg(reinterpret_cast<const float4 *>(n + off)); };
+        auto plane = [&](int off) { return load(reinterpret_cast<const float4 *>(n + off)); };
         const float4 ax = plane(s.px), ay = plane(s.py), az = plane(s.pz);
         const float4 bx = plane(48 - s.px), by = plane(80 - s.py), bz = plane(112 - s.pz);
         const float ex[4] = {ax.x, ax.y, ax.z, ax.w}, ey[4] = {ay.x, ay.y, ay.z, ay.w}, ez[4] = {az.x, az.y, az.z, az.w};
@@ -475,7 +491,7 @@ KS_D int trav_wide(const WideNode *__restrict__ wide, TravState &s, TravStack &s
             t0[k] = t_in;
         }
     } else {
-        const WideHits h = wide_slabs_guarded(wide + s.ref, s.ray.o, s.inv, s.ray.tmin, s.ray.tmax);
+        const WideHits h = wide_slabs_guarded(wide, s.ray.o, s.inv, s.ray.tmin, s.ray.tmax);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             ok[k] = (h.ok >> k) & 1u;
@@ -526,21 +542,70 @@ KS_D int trav_wide(const WideNode *__restrict__ wide, TravState &s, TravStack &s
 }
 
 // Interior step for either tree layout.
-template <bool kAnyHit>
-KS_D int trav_node(const TravNode *__restrict__ nodes, TravState &s, TravStack &stack, int &overflow,
+template <bool kAnyHit, class Stack>
+KS_D int trav_node(const TravNode *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
                    TravCount *count)
 {
     return trav_interior(nodes, s, stack, overflow, count);
 }
-template <bool kAnyHit>
-KS_D int trav_node(const WideNode *__restrict__ nodes, TravState &s, TravStack &stack, int &overflow,
+// The 4-wide view of binary nodes, made when a node is visited: wide node i holds the children of
+// interior node i, each interior child replaced by its own two children (2 to 4 slots, in order).
+struct LazyWide
+{
+    TravNode node;
+};
+KS_D WideNode widen(const LazyWide *__restrict__ nodes, uint32_t i)
+{
+    WideNode w;
+    for (int a = 0; a < 3; ++a) {
+        w.lo[a] = make_float4(kInf, kInf, kInf, kInf); // unused slots: an empty box, never hit
+        w.hi[a] = make_float4(-kInf, -kInf, -kInf, -kInf);
+    }
+    w.ref = make_uint4(kLeafBit, kLeafBit, kLeafBit, kLeafBit);
+    float *lo = reinterpret_cast<float *>(w.lo), *hi = reinterpret_cast<float *>(w.hi);
+    uint32_t *ref = reinterpret_cast<uint32_t *>(&w.ref);
+    int m = 0;
+    auto put = [&](const TravNode &nd, int side) {
+        const float4 A = nd.a, B = nd.b, C = nd.c;
+        const float l0[3] = {A.x, A.y, A.z}, h0[3] = {A.w, B.x, B.y};
+        const float l1[3] = {B.z, B.w, C.x}, h1[3] = {C.y, C.z, C.w};
+        for (int a = 0; a < 3; ++a) {
+            lo[4 * a + m] = side ? l1[a] : l0[a];
+            hi[4 * a + m] = side ? h1[a] : h0[a];
+        }
+        ref[m] = side ? nd.d.y : nd.d.x;
+        ++m;
+    };
+    const TravNode nd = nodes[i].node;
+    for (int side = 0; side < 2; ++side) {
+        const uint32_t r = side ? nd.d.y : nd.d.x;
+        if (r & kLeafBit) {
+            put(nd, side);
+        } else {
+            const TravNode c = nodes[r].node;
+            put(c, 0);
+            put(c, 1);
+        }
+    }
+    return w;
+}
+template <bool kAnyHit, class Stack>
+KS_D int trav_node(const LazyWide *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
                    TravCount *count)
 {
-    return trav_wide<kAnyHit>(nodes, s, stack, overflow, count);
+    const WideNode w = widen(nodes, s.ref);
+    return trav_wide<kAnyHit, false>(&w, s, stack, overflow, count);
+}
+template <bool kAnyHit, class Stack>
+KS_D int trav_node(const WideNode *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
+                   TravCount *count)
+{
+    return trav_wide<kAnyHit, true>(nodes + s.ref, s, stack, overflow, count);
 }
 
 // Pops the next node whose entry time is below the current tmax; false when the stack is empty.
-KS_D bool trav_pop(TravState &s, const TravStack &stack)
+template <class Stack>
+KS_D bool trav_pop(TravState &s, const Stack &stack)
 {
     while (s.sp > 0) {
         const uint2 e = stack.get(--s.sp);
@@ -592,9 +657,9 @@ KS_D bool trav_leaf(const float4 *__restrict__ tris, TravState &s, int culling, 
 
 // One step; returns true when the traversal of the ray is over (any-hit: found an occluder).
 // A step visits one node (an interior node or a leaf), then descends or pops.
-template <bool kAnyHit, class Node, class Alpha = NoAlpha>
+template <bool kAnyHit, class Node, class Stack, class Alpha = NoAlpha>
 KS_D bool trav_step(const Node *__restrict__ nodes, const float4 *__restrict__ tris, TravState &s,
-                    TravStack &stack, int culling, int &overflow, TravCount *count, const Alpha &alpha = Alpha{})
+                    Stack &stack, int culling, int &overflow, TravCount *count, const Alpha &alpha = Alpha{})
 {
     if (s.ref & kLeafBit) {
         if (trav_leaf<kAnyHit>(tris, s, culling, count, alpha))
@@ -612,17 +677,22 @@ KS_D bool trav_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
 // them (or all busy lanes) are at a leaf, then test their leaves together; the others descend
 // through interior nodes meanwhile.  Each ray's own sequence of tests is that of trav_step (a
 // waiting ray just pauses), but a warp runs the large triangle test with many lanes at once
-// instead of with the two or three that reach a leaf in the same step (about 10 % less time for
-// extension rays).  Any-hit queries step without waiting: holding back a leaf that may end the
-// ray costs them more than the batching saves.  Returns true when this lane's ray is over.
+// instead of with the two or three that reach a leaf in the same step.  Any-hit queries step without
+// waiting: holding back a leaf that may end the ray costs them more than the batching saves.  Returns
+// true when this lane's ray is over.  Leaf batches of 8, 12, 16 lanes: mesh frame (1.3 M triangles,
+// 1024 x 1024 x 64) 38.9, 37.7, 37.5 ms of closest hits, box room 1.80, 1.71, 1.65; instanced scenes
+// (whose lanes also wait at the upper level) 21.9, 22.8, 24.0.
 #ifndef KS_LEAF_BATCH
-#define KS_LEAF_BATCH 8
+#define KS_LEAF_BATCH 12
+#endif
+#ifndef KS_LEAF_BATCH_INST
+#define KS_LEAF_BATCH_INST 8
 #endif
 #ifndef KS_LEAF_BATCH_ANY
 #define KS_LEAF_BATCH_ANY 0
 #endif
-template <bool kAnyHit, class Node, class Alpha = NoAlpha>
-KS_D bool trav_warp_step(const Node *__restrict__ nodes, const float4 *__restrict__ tris, TravState &s,
+template <bool kAnyHit, class Tree, class State, class Alpha = NoAlpha>
+KS_D bool trav_warp_step(const Tree &nodes, const float4 *__restrict__ tris, State &s,
                          TravStack &stack, int culling, int &overflow, TravCount *count, bool busy,
                          const Alpha &alpha = Alpha{})
 {
@@ -630,30 +700,22 @@ KS_D bool trav_warp_step(const Node *__restrict__ nodes, const float4 *__restric
     if constexpr (kBatch == 0) {
         return busy && trav_step<kAnyHit>(nodes, tris, s, stack, culling, overflow, count, alpha);
     } else {
-        const bool at_leaf = busy && (s.ref & kLeafBit);
+        const bool at_leaf = busy && s.at_leaf();
         const uint32_t leaves = __ballot_sync(0xffffffffu, at_leaf);
         const uint32_t inner = __ballot_sync(0xffffffffu, busy && !at_leaf);
-        if (__popc(leaves) >= kBatch || inner == 0) {
-            if (!at_leaf)
-                return false;
-            if (trav_leaf<kAnyHit>(tris, s, culling, count, alpha))
-                return true;
-            return !trav_pop(s, stack);
-        }
-        if (!busy || at_leaf)
+        const bool leaf_phase = __popc(leaves) >= kBatch || inner == 0;
+        if (leaf_phase ? !at_leaf : (!busy || at_leaf))
             return false;
-        const int r = trav_node<kAnyHit>(nodes, s, stack, overflow, count);
-        if (r != 0)
-            return r < 0;
-        return !trav_pop(s, stack);
+        return trav_step<kAnyHit>(nodes, tris, s, stack, culling, overflow, count, alpha);
     }
 }
 
 // Dynamic ray fetch for trav_step: each warp takes rays from a global counter and hands every lane
 // that finished a new ray once at least KS_TRAV_REFILL lanes are idle, so a warp no longer runs
-// until its longest ray ends with most lanes masked off.
+// until its longest ray ends with most lanes masked off.  (12 or 16 idle lanes: mesh frame 37.7 or 36.8 ms
+// of closest hits.)
 #ifndef KS_TRAV_REFILL
-#define KS_TRAV_REFILL 12
+#define KS_TRAV_REFILL 16
 #endif
 
 // Hands the idle lanes of the warp rays [base, base + popc(idle)) in lane order; every lane calls
@@ -819,6 +881,21 @@ struct InstTravState
     uint32_t hit_inst;  // its instance
 };
 
+// The world-space ray in the object space of instance id (the direction not renormalised).
+KS_D RayQuery object_ray(const InstanceView &iv, uint32_t id, const RayQuery &ray)
+{
+    const float *m = iv.inv + 12 * (size_t)id;
+    float mi[12];
+#pragma unroll
+    for (int e = 0; e < 12; ++e)
+        mi[e] = __ldg(&m[e]);
+    RayQuery q;
+    q.o = xf_point(mi, ray.o);
+    q.d = xf_dir(mi, ray.d);
+    q.tmin = ray.tmin;
+    q.tmax = ray.tmax;
+    return q;
+}
 // False when the ray misses the TLAS root box.
 KS_D bool inst_begin(InstTravState &s, const InstanceView &iv, const RayQuery &ray)
 {
@@ -880,16 +957,7 @@ KS_D bool inst_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
         if (s.item < s.cnt) {
             // the next instance of the leaf: the ray in object space, then its prototype's BLAS
             const uint32_t id = __ldg(&iv.items[(s.ref & ~kLeafBit) + s.item]);
-            const float *m = iv.inv + 12 * (size_t)id;
-            float mi[12];
-#pragma unroll
-            for (int e = 0; e < 12; ++e)
-                mi[e] = __ldg(&m[e]);
-            RayQuery q;
-            q.o = xf_point(mi, s.ray.o);
-            q.d = xf_dir(mi, s.ray.d);
-            q.tmin = s.ray.tmin;
-            q.tmax = s.ray.tmax;
+            const RayQuery q = object_ray(iv, id, s.ray);
             const uint32_t pr = __ldg(&iv.proto[id]);
             const uint4 r = __ldg(&iv.proto_root[pr]);
             float pb[6];
@@ -941,20 +1009,20 @@ KS_D bool inst_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
 
 // Warp-wide step of the two-level traversal (every lane calls it; busy: the lane holds a ray).
 // Closest-hit queries batch their BLAS leaf tests like trav_warp_step: a lane whose BLAS node is
-// a leaf waits until KS_LEAF_BATCH lanes (or all busy lanes) are at one.  Each ray's own sequence
+// a leaf waits until KS_LEAF_BATCH_INST lanes (or all busy lanes) are at one.  Each ray's own sequence
 // of tests is that of inst_step.
 template <bool kAnyHit, class Node>
 KS_D bool inst_warp_step(const Node *__restrict__ nodes, const float4 *__restrict__ tris, const InstanceView &iv,
                          InstTravState &s, uint4 *tstack, TravStack &blas_stack, int culling, int &overflow,
                          TravCount *count, bool busy)
 {
-    if constexpr (kAnyHit || KS_LEAF_BATCH == 0) {
+    if constexpr (kAnyHit || KS_LEAF_BATCH_INST == 0) {
         return busy && inst_step<kAnyHit>(nodes, tris, iv, s, tstack, blas_stack, culling, overflow, count);
     } else {
-        const bool at_leaf = busy && s.in_blas && (s.blas.ref & kLeafBit);
+        const bool at_leaf = busy && s.in_blas && s.blas.at_leaf();
         const uint32_t leaves = __ballot_sync(0xffffffffu, at_leaf);
         const uint32_t others = __ballot_sync(0xffffffffu, busy && !at_leaf);
-        const bool leaf_phase = __popc(leaves) >= KS_LEAF_BATCH || others == 0;
+        const bool leaf_phase = __popc(leaves) >= KS_LEAF_BATCH_INST || others == 0;
         if (leaf_phase ? !at_leaf : (!busy || at_leaf))
             return false;
         return inst_step<false>(nodes, tris, iv, s, tstack, blas_stack, culling, overflow, count);

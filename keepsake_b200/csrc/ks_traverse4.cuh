@@ -1,0 +1,326 @@
+// Traversal of the renderer's 4-wide view of the SBVH (Wide4Node): its ray queries on the device.
+//
+// The result of a query is the one that the 4-wide steps of ks_traverse.cuh give (the closest hit, or
+// whether anything is hit: "the exact traversal" below), reached with cheaper steps, since the kernels
+// are bound by the instructions they issue:
+//   * the box test need only be conservative: one fused multiply-add per plane instead of a
+//     subtraction, a product and a guard, with its rounding widened away (Trav4::set_ray);
+//   * a closest-hit node's slots are sorted as integers, the entry time with the slot in its last two
+//     bits; a pending child is that key and its parent's index, and its ref is read when it is visited.
+// What keeps the result:
+//   * a triangle that is hit counts when slab() accepts its leaf's box, which is when the exact
+//     traversal tests the triangle at all (a leaf's box passes only if every box above it does);
+//   * which of several hits is the closest does not depend on the visiting order unless two of them
+//     are nearly equally far: within rounding of each other, or one nearer than the other's box is
+//     entered.  Trav4 keeps what is needed to see that, and such a ray (about one in a million) is
+//     traced again in the exact traversal's order (retrace).
+// Trees too deep for the stack keep the exact traversal, whose stack overflow is an error status, and so do
+// instanced scenes: beside the state of their upper level this one's does not fit the registers (closest hit
+// over 400 instances at 1080p x 4: 22.0 ms by the exact traversal, 23.8 by this one at its best).
+#pragma once
+#include "ks_traverse.cuh"
+
+namespace ksb
+{
+
+// Deepest SBVH (levels) with this view: the exact traversal pushes at most 3 entries per two levels, so
+// up to here it never outgrows kWideStackDepth.  This one pushes at most 3 per level of the view.
+constexpr uint32_t kMaxBinaryLevels = 2 * (kWideStackDepth / 3), kMaxWideLevels = kWideStackDepth / 3;
+
+KS_D float max3f(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+KS_D float min3f(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Relative slack of the box test, of the pruning distance and of the tie test (Trav4).
+constexpr float kMaxInv = 1e30f; // 1 / d is clamped to it
+constexpr float kBoxSlack = 0x1p-20f, kPruneSlack = 0x1p-12f, kTieSlack = 0x1p-20f;
+
+// What the traversal reads: the nodes, and per leaf (at its first primitive slot) its box, 2 float4.
+struct Tree4
+{
+    const Wide4Node *nodes;
+    const float4 *leaf_box;
+};
+
+struct Trav4
+{
+    RayQuery ray;            // tmax: as the query gave it
+    TriHelper th;
+    f3 inv;                  // 1 / d
+    f3 o_in, inv_out, o_out; // t of an entry plane: b inv - o_in; of an exit plane: b inv_out - o_out
+    uint32_t ref;            // the node or leaf to visit
+    int sp;
+    float limit;             // boxes and triangles beyond it are skipped
+    Hit hit;
+    float entry;             // entry time of the hit's leaf
+    float second;            // distance of the closest other hit seen
+
+    KS_D bool at_leaf() const { return (ref & kLeafBit) != 0; }
+
+    // The plane equations.  Against slab()'s t = (b - o) * inv the fused form is off by at most
+    // 2^-24 |o inv| per rounded constant and a few 2^-24 |t|: the offsets are moved out by
+    // 2^-22 |o inv|, exit planes are scaled by 1 + 2^-20.  A zero component's infinite 1 / d is
+    // clamped, which keeps the products finite: inside its slab the interval stays at least +-1e30
+    // times the distance to the planes, outside it starts beyond every other exit.
+    KS_D void set_ray(f3 d)
+    {
+        auto axis = [&](float o, float dc, float &iv, float &oi, float &io, float &oo) {
+            iv = 1.0f / dc;
+            if (!(fabsf(iv) <= kMaxInv))
+                iv = copysignf(kMaxInv, iv);
+            const float oc = o * iv, pad = fabsf(oc) * 0x1p-22f;
+            oi = oc + pad;
+            io = iv * (1.0f + kBoxSlack);
+            oo = oc * (1.0f + kBoxSlack) - pad;
+            if (ray.tmin < 0.0f) // negative distances: the scale would move exit planes inwards
+                oo += ray.tmin * 0x1p-18f;
+        };
+        axis(ray.o.x, d.x, inv.x, o_in.x, inv_out.x, o_out.x);
+        axis(ray.o.y, d.y, inv.y, o_in.y, inv_out.y, o_out.y);
+        axis(ray.o.z, d.z, inv.z, o_in.z, inv_out.z, o_out.z);
+    }
+};
+
+// The query's own 1 / d: what set_ray clamped was infinite.  (Or the component was a nonzero one below
+// 1e-30, whose slab a ray leaves within a distance of 1e-25 of its plane: infinity decides the same.)
+KS_D BoxHelper exact_helper(const Trav4 &s)
+{
+    auto own = [](float iv) { return fabsf(iv) == kMaxInv ? copysignf(kInf, iv) : iv; };
+    return box_helper_of(mk(own(s.inv.x), own(s.inv.y), own(s.inv.z)));
+}
+
+// Whether another visiting order could have found another closest hit: one within rounding of it, or
+// nearer than its leaf is entered (a leaf is skipped when the ray enters it beyond the hit at hand).
+KS_D bool ambiguous(const Trav4 &s)
+{
+    const float far = fmaxf(s.hit.t, s.entry);
+    return s.hit.tri != ~0u && (!(s.second > far + fabsf(far) * kTieSlack) ||
+                                s.entry > s.hit.t + fabsf(s.hit.t) * (0.5f * kPruneSlack));
+}
+
+// False when the ray misses the root box.
+KS_D bool trav_begin(Trav4 &s, const RayQuery &ray, uint32_t root, uint32_t root_count, const float root_bmin[3],
+                     const float root_bmax[3])
+{
+    s.hit.tri = ~0u;
+    s.ray = ray;
+    s.th = make_tri_helper(ray.d);
+    s.set_ray(ray.d);
+    s.limit = ray.tmax;
+    s.entry = 0.0f;
+    s.second = kInf;
+    s.sp = 0;
+    s.ref = root;
+    float t0, t1;
+    return root_count != 0 && slab(ray, make_box_helper(ray.d), root_bmin, root_bmax, t0, t1) && t0 < ray.tmax &&
+           t1 > ray.tmin;
+}
+
+// The next pending child; false when there is none.  Closest hit: entries are (parent index, key), dropped
+// beyond the limit.  Any hit: the child's ref.
+template <bool kAnyHit>
+KS_D bool trav4_pop(const Wide4Node *__restrict__ nodes, Trav4 &s, const TravStack &stack)
+{
+    while (s.sp > 0) {
+        const uint2 e = stack.get(--s.sp);
+        if constexpr (kAnyHit) {
+            s.ref = e.x;
+            return true;
+        } else if (__uint_as_float(e.y) <= s.limit) {
+            s.ref = __ldg(&nodes[e.x].ref[e.y & 3u]);
+            return true;
+        }
+    }
+    return false;
+}
+
+// Visits node s.ref: descends to a child and returns true, or returns false when none is hit.
+// Any-hit queries take the children in slot order: nearest first took 2.5 % off the bench frame's
+// shadow rays once but made a pass of the occluded glossy scene 17 % slower (rays blocked by a distant
+// occluder then search the nearby geometry's subtrees first).
+template <bool kAnyHit>
+KS_D bool trav4_node(const Wide4Node *__restrict__ nodes, Trav4 &s, TravStack &stack, TravCount *count)
+{
+    if (count)
+        count->nodes += 2; // 128 bytes: two 64-byte node units
+    const uint32_t at = s.ref;
+    const uintptr_t n = reinterpret_cast<uintptr_t>(nodes + at);
+    // the entry plane of an axis is its upper one (16 bytes on) when the direction is negative
+    auto plane = [&](uint32_t axis, uint32_t upper) {
+        return __ldg(reinterpret_cast<const float4 *>((n | (upper & 16u)) + 32u * axis));
+    };
+    const uint32_t ux = __float_as_uint(s.inv.x) >> 27, uy = __float_as_uint(s.inv.y) >> 27,
+                   uz = __float_as_uint(s.inv.z) >> 27;
+    const float4 ax = plane(0, ux), ay = plane(1, uy), az = plane(2, uz);
+    const float4 bx = plane(0, ~ux), by = plane(1, ~uy), bz = plane(2, ~uz);
+    const float ex[4] = {ax.x, ax.y, ax.z, ax.w}, ey[4] = {ay.x, ay.y, ay.z, ay.w}, ez[4] = {az.x, az.y, az.z, az.w};
+    const float lx[4] = {bx.x, bx.y, bx.z, bx.w}, ly[4] = {by.x, by.y, by.z, by.w}, lz[4] = {bz.x, bz.y, bz.z, bz.w};
+    float t_in[4];
+    bool ok[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        t_in[k] = max3f(fmaf(ex[k], s.inv.x, -s.o_in.x), fmaf(ey[k], s.inv.y, -s.o_in.y),
+                        fmaxf(fmaf(ez[k], s.inv.z, -s.o_in.z), s.ray.tmin));
+        const float t_out = min3f(fmaf(lx[k], s.inv_out.x, -s.o_out.x), fmaf(ly[k], s.inv_out.y, -s.o_out.y),
+                                  fminf(fmaf(lz[k], s.inv_out.z, -s.o_out.z), s.limit));
+        ok[k] = t_in[k] <= t_out;
+    }
+    if constexpr (kAnyHit) {
+        const uint4 child = __ldg(reinterpret_cast<const uint4 *>(n + 96));
+        const uint32_t ref[4] = {child.x, child.y, child.z, child.w};
+        // the first slot hit next, the others below it on the stack, the last one deepest
+        const int top = s.sp + (int)ok[0] + (int)ok[1] + (int)ok[2] + (int)ok[3] - 1;
+        if (top < s.sp)
+            return false;
+        s.ref = ok[0] ? ref[0] : (ok[1] ? ref[1] : (ok[2] ? ref[2] : ref[3]));
+        int put = s.sp;
+#pragma unroll
+        for (int k = 3; k >= 1; --k)
+            if (ok[k] && put < top)
+                stack.set(put++, ref[k], 0.0f);
+        s.sp = top;
+    } else {
+        // t_in >= tmin >= 0 in a render: the bits order like the times (a negative tmin only costs order)
+        uint32_t key[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            key[k] = ok[k] ? ((__float_as_uint(t_in[k]) & ~3u) | (uint32_t)k) : ~0u;
+        auto cex = [&](int i, int j) {
+            const uint32_t lo = min(key[i], key[j]), hi = max(key[i], key[j]);
+            key[i] = lo;
+            key[j] = hi;
+        };
+        cex(0, 1);
+        cex(2, 3);
+        cex(0, 2);
+        cex(1, 3);
+        cex(1, 2);
+        if (key[0] == ~0u)
+            return false;
+        const int top = s.sp + (key[1] != ~0u) + (key[2] != ~0u) + (key[3] != ~0u);
+        if (top <= kSmemStack) {
+            uint2 *e = stack.sm + top * kTravBlock;
+#pragma unroll
+            for (int r = 1; r < 4; ++r)
+                if (key[r] != ~0u)
+                    e[-r * kTravBlock] = make_uint2(at, key[r]);
+        } else {
+            for (int r = 3; r >= 1; --r)
+                if (key[r] != ~0u)
+                    stack.set(top - r, at, __uint_as_float(key[r]));
+        }
+        s.sp = top;
+        s.ref = __ldg(&nodes[at].ref[key[0] & 3u]);
+    }
+    return true;
+}
+
+// The box of a leaf in slab()'s own arithmetic: whether the exact traversal tests the leaf, and when
+// the ray enters it.
+KS_D bool leaf_reached(const float4 *__restrict__ leaf_box, const Trav4 &s, uint32_t first, float &entry)
+{
+    const float4 lo = __ldg(leaf_box + 2 * (size_t)first), hi = __ldg(leaf_box + 2 * (size_t)first + 1);
+    const float bmin[3] = {lo.x, lo.y, lo.z}, bmax[3] = {hi.x, hi.y, hi.z};
+    float t1;
+    return slab(s.ray, exact_helper(s), bmin, bmax, entry, t1) && t1 > s.ray.tmin && entry < s.ray.tmax;
+}
+
+// Tests the leaf at hand; true when an any-hit query found an occluder.
+template <bool kAnyHit, class Alpha>
+KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restrict__ tris, Trav4 &s, int culling,
+                     TravCount *count, const Alpha &alpha)
+{
+    const uint32_t first = s.ref & ~kLeafBit;
+    uint32_t slot = first;
+    bool last;
+    do {
+        if (count)
+            count->tris++;
+        const float4 *p = tris + 3 * (size_t)slot;
+        const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+        last = __float_as_uint(b.w) != 0u;
+        const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
+        const uint32_t tri = __float_as_uint(a.w);
+        RayQuery q = s.ray;
+        q.tmax = s.limit;
+        float t, b0, b1, b2;
+        if (!cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, t, b0, b1, b2)) {
+            float entry;
+            if (kAnyHit) {
+                if (leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
+                    s.hit.tri = tri;
+                    return true;
+                }
+            } else if (t < s.limit && leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
+                if (tri == s.hit.tri) {
+                    s.entry = fminf(s.entry, entry); // the same triangle through another of its leaves
+                } else if (s.hit.tri == ~0u || t < s.hit.t) {
+                    if (s.hit.tri != ~0u)
+                        s.second = fminf(s.second, s.hit.t);
+                    s.entry = entry;
+                    s.limit = fminf(s.ray.tmax, t + fabsf(t) * kPruneSlack);
+                    s.hit.tri = tri;
+                    s.hit.slot = slot;
+                    s.hit.t = t;
+                    s.hit.b0 = b0;
+                    s.hit.b1 = b1;
+                    s.hit.b2 = b2;
+                } else {
+                    s.second = fminf(s.second, t);
+                }
+            }
+        }
+        ++slot;
+    } while (!last);
+    return false;
+}
+
+// One step (a node or a leaf); true when the traversal of the ray is over.
+template <bool kAnyHit, class Alpha = NoAlpha>
+KS_D bool trav_step(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 &s, TravStack &stack, int culling, int &,
+                    TravCount *count, const Alpha &alpha = Alpha{})
+{
+    if (s.at_leaf()) {
+        if (trav4_leaf<kAnyHit>(tree.leaf_box, tris, s, culling, count, alpha))
+            return true;
+    } else {
+        if (trav4_node<kAnyHit>(tree.nodes, s, stack, count))
+            return false;
+    }
+    return !trav4_pop<kAnyHit>(tree.nodes, s, stack);
+}
+
+// The closest hit by the exact traversal's own order: the 4-wide steps over boxes read from the
+// binary nodes.  Out of line and called from other kernels than the traversal's: a call there would
+// cost its registers and its stack their places (measured: 1.3 x the time).
+struct Retraced
+{
+    Hit hit;
+    int overflow;
+};
+template <class Alpha = NoAlpha>
+static __device__ __noinline__ Retraced retrace(const TravNode *nodes, const float4 *tris, uint32_t root_ref,
+                                                uint32_t root_count, const float *bmin, const float *bmax, RayQuery q,
+                                                int culling, Alpha alpha = Alpha{})
+{
+    TravState s;
+    LocalStack stack;
+    Retraced r;
+    r.overflow = 0;
+    if (trav_begin(s, q, root_ref, root_count, bmin, bmax))
+        while (!trav_step<false>(reinterpret_cast<const LazyWide *>(nodes), tris, s, stack, culling, r.overflow, nullptr,
+                                 alpha)) {
+        }
+    r.hit = s.hit;
+    return r;
+}
+} // namespace ksb

@@ -4,6 +4,7 @@
 #pragma once
 #include "ks_guide_view.cuh"
 #include "ks_lights.cuh"
+#include "ks_traverse4.cuh"
 
 namespace ksb
 {
@@ -421,19 +422,25 @@ KS_D f3 clamp_contrib(f3 v, int bounce_for_direct, const RenderParams &rp, bool 
     return v;
 }
 
-// The tree a kernel traverses: the SBVH nodes or their 4-wide view.
-template <class Node>
-KS_D const Node *tree_of(const SceneView &sv);
-template <>
-KS_D const TravNode *tree_of<TravNode>(const SceneView &sv)
+// What a flat scene's traversal kernel walks: the renderer's 4-wide view of the tree, or (kDeep) binary
+// nodes by the exact traversal's steps.
+template <bool kDeep>
+struct TreeOf
 {
-    return sv.nodes;
-}
+    using State = Trav4;
+    using Tree = Tree4;
+    KS_D static Tree tree(const SceneView &sv) { return Tree4{sv.wide, sv.leaf_box}; }
+    KS_D static uint32_t root(const SceneView &) { return 0u; }
+};
 template <>
-KS_D const WideNode *tree_of<WideNode>(const SceneView &sv)
+struct TreeOf<true>
 {
-    return sv.wide;
-}
+    using State = TravState;
+    using Tree = const LazyWide *;
+    KS_D static Tree tree(const SceneView &sv) { return reinterpret_cast<const LazyWide *>(sv.nodes); }
+    KS_D static uint32_t root(const SceneView &sv) { return sv.root_ref; }
+};
+KS_D bool ambiguous(const TravState &) { return false; }
 
 // ---- shading launchers (ks_shade.cu) ----------------------------------------------------------
 // k_sample: Sobol values and the NEE light sample of every path in the hit queue.

@@ -1,0 +1,59 @@
+"""The renderer's traversal (ks_trace_rays_wide: the 4-wide view, conservative box tests, leaves checked
+when a triangle is hit) against the reference-order binary traversal (ks_trace_rays) on the same
+device, over trees of one leaf, a few and many nodes, duplicated and flat triangles, and rays with
+zero components, finite and negative ranges, unnormalised directions.
+
+Occlusion does not depend on the visiting order, so it is equal for every ray.  The closest hit is
+equal bit for bit unless two triangles lie within rounding of each other on the ray; then the two
+orders may keep different ones, whose distances agree within 8 ulp (the bound of the hit-id tests)
+or, for hits whose computed distance lies before their leaf's entry, one part in 2^12."""
+import numpy as np
+import pytest
+
+import scenes
+
+
+def rays(v, idx, n, seed):
+    rng = np.random.default_rng(seed)
+    a = scenes.random_rays(v, n, seed)
+    b = scenes.rays_at_triangles(v, idx, n, seed + 1)
+    axis = scenes.random_rays(v, n, seed + 2)
+    axis[:, 4:7] = 0.0
+    axis[np.arange(n), 4 + rng.integers(0, 3, n)] = np.where(rng.random(n) < 0.5, 1.0, -1.0)
+    axis[: n // 2, 0:3] = v[idx[rng.integers(0, len(idx), n // 2), 0]]  # from vertices: on the boxes' planes
+    ranged = scenes.random_rays(v, n, seed + 3)
+    ranged[:, 3] = rng.normal(size=n) * 0.2
+    ranged[:, 7] = rng.random(n) * np.ptp(v) * 0.3
+    scaled = scenes.random_rays(v, n, seed + 4)
+    scaled[:, 4:7] *= rng.choice([1e-3, 37.0], size=(n, 1))
+    scaled[: n // 2, 4] = -0.0
+    return np.concatenate([a, b, axis, ranged, scaled]).astype(np.float32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,n", [("one", 1), ("leaf", 4), ("small", 9), ("soup", 3000), ("flat", 0), ("copies", 400)])
+@pytest.mark.parametrize("culling", [2, 0])
+def test_wide_traversal_matches_binary(ctx, kind, n, culling):
+    import keepsake_b200 as ks
+    if kind == "flat":
+        v, idx = scenes.degenerate_soup(2)
+    else:
+        v, idx = scenes.soup(n, seed=n, spread=1.0 if n < 10 else 6.0)
+    if kind == "copies":
+        v, idx = np.concatenate([v, v]), np.concatenate([idx, idx + len(v)])
+    desc, keep = ks.triangle_soup_desc(v, idx)
+    s = ks.Scene(ctx, desc, keep)
+    s.build_bvh()
+    r = rays(v, np.asarray(idx), 20000, 3)
+    assert np.array_equal(s.trace(r, any_hit=True, culling=culling, wide=True)[0],
+                          s.trace(r, any_hit=True, culling=culling)[0])
+    tri, t, bary = s.trace(r, culling=culling, wide=True)
+    tri0, t0, bary0 = s.trace(r, culling=culling)
+    assert np.array_equal(tri == 0xFFFFFFFF, tri0 == 0xFFFFFFFF)
+    same = tri == tri0
+    assert np.array_equal(t[same], t0[same]) and np.array_equal(bary[same], bary0[same])
+    off = np.abs(t[~same].astype(np.float64) - t0[~same]) / np.abs(t0[~same])
+    assert (off <= 2.0 ** -12).all()
+    if kind not in ("flat", "copies"):  # no coplanar or repeated triangles: ties are rare
+        assert (~same).mean() < 1e-3 and (off <= 8 * 2.0 ** -23).all()
+    s.close()
