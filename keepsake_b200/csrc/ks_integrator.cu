@@ -56,8 +56,8 @@ using namespace wave;
 #endif
 
 // Per-iteration counters: paths continuing, shadow rays, hit queue, miss queue, extension-ray
-// fetch, shadow-ray fetch.
-constexpr uint32_t kCounters = 6;
+// fetch, shadow-ray fetch, subsurface walks, walk fetch.
+constexpr uint32_t kCounters = 8;
 
 // ---- kernels --------------------------------------------------------------------------------
 
@@ -602,6 +602,7 @@ struct RenderWork
     DevBuf<float4> shadow[4];
     DevBuf<uint32_t> counters; // [next, shadow, hit queue, miss queue, extension fetch, shadow fetch]
     DevBuf<uint32_t> queue[2]; // hit / miss path indices
+    DevBuf<uint32_t> walks;    // scenes with subsurface materials: paths that walk this bounce
     DevBuf<int> overflow;
     DevBuf<float> filter; // the pixel filter's sample table (Gaussian / Blackman-Harris)
     uint32_t capacity = 0;
@@ -839,6 +840,8 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     KS_CUDA_TRY(ctx, w.hits.reserve(w.capacity));
     if (scene->n_instances)
         KS_CUDA_TRY(ctx, w.hit_inst.reserve(w.capacity));
+    if (scene->any_subsurface)
+        KS_CUDA_TRY(ctx, w.walks.reserve(w.capacity));
     KS_CUDA_TRY(ctx, w.samples.reserve(4 * (size_t)w.capacity));
     if (rp.filter_n) {
         KS_CUDA_TRY(ctx, w.filter.reserve(ftab.size()));
@@ -1015,9 +1018,9 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             }
             cudaEventRecord(ev[5], st);
             if (scene->any_subsurface) {
-                launch_subsurface(grid, st, sv, rp, pb[cur], w.hits.ptr, w.queue[0].ptr, w.counters.ptr + 2,
-                                  w.overflow.ptr);
-                stats.kernel_launches++;
+                launch_subsurface(grid, (unsigned)ctx->sm_count, st, sv, rp, pb[cur], w.hits.ptr, w.queue[0].ptr,
+                                  w.counters.ptr + 2, w.walks.ptr, w.counters.ptr + 6, w.overflow.ptr);
+                stats.kernel_launches += 2;
             }
             launch_sample(false, grid, st, sv, rp, pb[cur], w.hits.ptr, w.hit_inst.ptr, w.queue[0].ptr,
                           w.counters.ptr + 2, w.samples.ptr, BatchView{});

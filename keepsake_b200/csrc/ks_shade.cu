@@ -14,6 +14,7 @@
 #include "ks_wavefront.cuh"
 #include "ks_subsurface.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace ksb
@@ -601,84 +602,144 @@ struct MeshOnly
     KS_D bool operator()(uint32_t tri, float, float, const RayQuery &) const { return __ldg(&tri_mesh[tri]) == mesh; }
 };
 
-__global__ void __launch_bounds__(128) k_subsurface(const __grid_constant__ SceneView sv, const __grid_constant__ RenderParams rp,
-                                                    PathBuf cur, float4 *hits, const uint32_t *queue,
-                                                    const uint32_t *queue_count, int *overflow)
+// The draw at every such hit; the hits that walk go to the walk queue.
+__global__ void __launch_bounds__(128) k_subsurface_select(const __grid_constant__ SceneView sv,
+                                                           const __grid_constant__ RenderParams rp, PathBuf cur,
+                                                           const float4 *hits, const uint32_t *queue,
+                                                           const uint32_t *queue_count, uint32_t *walks,
+                                                           uint32_t *walk_count)
 {
     const uint32_t count = *queue_count;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-        const uint32_t i = queue[q];
-        const float4 h = hits[i];
-        const float4 *pt = sv.prim_tris + 3 * (size_t)bits(h.w);
-        const float4 v0 = __ldg(pt), v1 = __ldg(pt + 1), v2 = __ldg(pt + 2);
-        const uint32_t tri = bits(v0.w);
-        const uint32_t mesh = __ldg(&sv.tri_mesh[tri]);
-        const MaterialGPU &mat = sv.materials[__ldg(&sv.mesh_material[mesh])];
-        if (!mat.has_ss)
-            continue;
-        float4 d4 = cur.d_info[i];
-        const uint32_t info = bits(d4.w);
-        const uint32_t bounce = info & 0xffffu;
-        if ((int)bounce == rp.bounces)
-            continue; // the path ends at this hit (small_pt.cpp:140-142): nothing is sampled
-        const int dim = (int)(info >> 16);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+        const uint32_t q = base + threadIdx.x;
+        bool walk = false;
+        uint32_t i = 0;
+        if (q < count) {
+            i = queue[q];
+            const uint32_t tri = bits(__ldg(sv.prim_tris + 3 * (size_t)bits(hits[i].w)).w);
+            const MaterialGPU &mat = sv.materials[__ldg(&sv.mesh_material[__ldg(&sv.tri_mesh[tri])])];
+            const uint32_t info = bits(cur.d_info[i].w);
+            const uint32_t bounce = info & 0xffffu;
+            // at the last bounce the path ends at this hit (small_pt.cpp:140-142): nothing is sampled
+            if (mat.has_ss && (int)bounce != rp.bounces) {
+                const int dim = (int)(info >> 16);
+                const float4 bp = cur.beta_pix[i];
+                const uint32_t pix = bits(bp.w), smp = bits(cur.L_smp[i].w);
+                SobolSampler sob = SobolSampler::start(pix % (uint32_t)rp.W, pix / (uint32_t)rp.W, smp, rp.log2_spp,
+                                                       rp.n_digits, (uint32_t)rp.seed, dim);
+                const float u_sel = sob.next();
+                cur.d_info[i].w = fbits(((uint32_t)(dim + 1) << 16) | bounce);
+                walk = !(u_sel < 0.5f);
+                if (!walk) {
+                    f3 beta = mk(bp.x, bp.y, bp.z);
+                    beta *= 2.0f;
+                    cur.beta_pix[i] = make_float4(beta.x, beta.y, beta.z, bp.w);
+                }
+            }
+        }
+        const uint32_t j = warp_append(walk_count, walk);
+        if (walk)
+            walks[j] = i;
+    }
+}
+
+// Walks of the queue, a step of every lane's walk at a time; once KS_WALK_REFILL lanes are idle they take new
+// walks.  Few hits walk, and a walk takes 1 to 256 steps (16 on average): run where the hits lie they kept 2 or
+// 3 lanes of a warp busy (subsurface box and sphere, 256 x 256 x 16: 13.4 ms a frame, 10.3 with the queue).  What
+// is left is latency: the longest walk's 256 steps one after the other, about 4.5 us each, so neither the
+// refill (4, 8, 16 idle lanes: 11.1, 11.0, 11.0 ms) nor more CTAs (5, 6, 8 per SM: 11.5, 12.6, 13.3 ms) helps.
+#ifndef KS_WALK_REFILL
+#define KS_WALK_REFILL 8
+#endif
+__global__ void __launch_bounds__(128) k_subsurface_walk(const __grid_constant__ SceneView sv,
+                                                         const __grid_constant__ RenderParams rp, PathBuf cur,
+                                                         float4 *hits, const uint32_t *walks,
+                                                         const uint32_t *walk_count, uint32_t *fetch, int *overflow)
+{
+    const uint32_t count = *walk_count;
+    SsWalk s;
+    uint32_t i = ~0u, mesh = 0;
+    bool drained = false;
+    int of = 0;
+    auto cast = [&](const RayQuery &ray, WalkExit &e) {
+        Hit hh;
+        traverse<false>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, ray, 2, hh, of, nullptr,
+                        MeshOnly{sv.tri_mesh, mesh});
+        if (hh.tri == ~0u)
+            return false;
+        e = WalkExit{hh.slot, hh.t, hh.b1, hh.b2};
+        return true;
+    };
+    auto finish = [&](bool hit) {
         const float4 bp = cur.beta_pix[i];
-        const uint32_t pix = bits(bp.w), smp = bits(cur.L_smp[i].w);
-        SobolSampler sob = SobolSampler::start(pix % (uint32_t)rp.W, pix / (uint32_t)rp.W, smp, rp.log2_spp,
-                                               rp.n_digits, (uint32_t)rp.seed, dim);
-        const float u_sel = sob.next();
-        d4.w = fbits(((uint32_t)(dim + 1) << 16) | bounce);
-        f3 beta = mk(bp.x, bp.y, bp.z);
-        if (u_sel < 0.5f) {
-            beta *= 2.0f;
-        } else {
+        f3 beta = mk(0, 0, 0);
+        if (hit) {
+            beta = mk(bp.x, bp.y, bp.z) * s.throughput;
+            hits[i] = make_float4(-1.0f, s.exit.b1, s.exit.b2, fbits(s.exit.slot));
+            cur.d_info[i] = make_float4(s.ray.d.x, s.ray.d.y, s.ray.d.z, cur.d_info[i].w);
+        }
+        cur.beta_pix[i] = make_float4(beta.x, beta.y, beta.z, bp.w);
+        i = ~0u;
+    };
+    while (true) {
+        const uint32_t q = warp_fetch(fetch, count, i == ~0u, drained);
+        if (q != ~0u) {
+            i = walks[q];
+            const float4 h = hits[i];
+            const float4 *pt = sv.prim_tris + 3 * (size_t)bits(h.w);
+            const float4 v0 = __ldg(pt), v1 = __ldg(pt + 1), v2 = __ldg(pt + 2);
+            const uint32_t tri = bits(v0.w);
+            mesh = __ldg(&sv.tri_mesh[tri]);
+            const MaterialGPU &mat = sv.materials[__ldg(&sv.mesh_material[mesh])];
+            const float4 d4 = cur.d_info[i];
+            const uint32_t bounce = bits(d4.w) & 0xffffu;
+            const uint32_t pix = bits(cur.beta_pix[i].w), smp = bits(cur.L_smp[i].w);
             f3 tp = mk(2.0f, 2.0f, 2.0f);
             tp /= sqr(mat.ss_ior);
+            s.throughput = tp;
             const f3 p0 = mk(v0.x, v0.y, v0.z), p1 = mk(v1.x, v1.y, v1.z), p2 = mk(v2.x, v2.y, v2.z);
             const int flags = __ldg(&sv.mesh_flags[mesh]);
             ShadeFrame it = hit_frame<true>(sv, tri, flags, p0, p1, p2, h.y, h.z, mk(d4.x, d4.y, d4.z), nullptr);
             if (mat.tex_flags & kMatNormalMap)
                 (void)textured_material(sv, mat, tri, flags, h.y, h.z, it);
-            SsProfile prof;
-            prof.albedo = mk(mat.ss_albedo[0], mat.ss_albedo[1], mat.ss_albedo[2]);
-            prof.radius = mk(mat.ss_radius[0], mat.ss_radius[1], mat.ss_radius[2]);
-            prof.g = mat.ss_g;
-            prof.ior = mat.ss_ior;
-            prof.rfr_entry_prob = mat.ss_rfr;
-            Pcg32 rng = subsurface_stream(pix % (uint32_t)rp.W, pix / (uint32_t)rp.W, (uint32_t)rp.seed, smp, bounce);
-            int of = 0;
-            auto cast = [&](const RayQuery &ray, WalkExit &e) {
-                Hit hh;
-                traverse<false>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, ray, 2, hh, of,
-                                nullptr, MeshOnly{sv.tri_mesh, mesh});
-                if (hh.tri == ~0u)
-                    return false;
-                e = WalkExit{hh.slot, hh.t, hh.b1, hh.b2};
-                return true;
-            };
-            WalkExit ex;
-            f3 wi;
-            if (subsurface_walk(prof, it.p, it.sn, it.n, rng, cast, tp, ex, wi)) {
-                beta = beta * tp;
-                hits[i] = make_float4(-1.0f, ex.b1, ex.b2, fbits(ex.slot));
-                d4.x = wi.x;
-                d4.y = wi.y;
-                d4.z = wi.z;
-            } else {
-                beta = mk(0, 0, 0);
-            }
-            if (of)
-                atomicOr(overflow, 1);
+            s.prof.albedo = mk(mat.ss_albedo[0], mat.ss_albedo[1], mat.ss_albedo[2]);
+            s.prof.radius = mk(mat.ss_radius[0], mat.ss_radius[1], mat.ss_radius[2]);
+            s.prof.g = mat.ss_g;
+            s.prof.ior = mat.ss_ior;
+            s.prof.rfr_entry_prob = mat.ss_rfr;
+            s.rng = subsurface_stream(pix % (uint32_t)rp.W, pix / (uint32_t)rp.W, (uint32_t)rp.seed, smp, bounce);
+            s.P = it.p;
+            s.N = it.sn;
+            if (!subsurface_begin(s, it.n))
+                finish(false);
         }
-        cur.d_info[i] = d4;
-        cur.beta_pix[i] = make_float4(beta.x, beta.y, beta.z, bp.w);
+        if (__ballot_sync(0xffffffffu, i != ~0u) == 0) {
+            if (drained)
+                break;
+            continue;
+        }
+        while (true) {
+            bool hit;
+            if (i != ~0u && !subsurface_step(s, cast, hit))
+                finish(hit);
+            const int n_idle = __popc(__ballot_sync(0xffffffffu, i == ~0u));
+            if (n_idle == 32 || (!drained && n_idle >= KS_WALK_REFILL))
+                break;
+        }
     }
+    if (of)
+        atomicOr(overflow, 1);
 }
 
-void launch_subsurface(unsigned grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp, PathBuf cur,
-                       float4 *hits, const uint32_t *queue, const uint32_t *queue_count, int *overflow)
+void launch_subsurface(unsigned grid, unsigned sm_count, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
+                       PathBuf cur, float4 *hits, const uint32_t *queue, const uint32_t *queue_count, uint32_t *walks,
+                       uint32_t *walk_counts, int *overflow)
 {
-    k_subsurface<<<grid, 128, 0, st>>>(sv, rp, cur, hits, queue, queue_count, overflow);
+    k_subsurface_select<<<grid, 128, 0, st>>>(sv, rp, cur, hits, queue, queue_count, walks, walk_counts);
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subsurface_walk, 128, 0);
+    k_subsurface_walk<<<std::min(grid, (unsigned)std::max(per_sm, 1) * sm_count), 128, 0, st>>>(
+        sv, rp, cur, hits, walks, walk_counts, walk_counts + 1, overflow);
 }
 
 void launch_sample(bool batch, unsigned grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp,

@@ -206,16 +206,34 @@ struct WalkExit
     float t, b1, b2;
 };
 
-// subsurface_random_walk (subsurface.cpp:222-500) from an entry point P with shading normal N and
-// geometric normal Ng (the hit frame's).  cast(o, d, tmax, exit) is the mesh-local closest-hit
-// query (LocalGeometry::intersect1: only the entry mesh's triangles).  The walk starts with D = 0,
-// as BSSRDF::sample calls it (material.cpp:136-140): the refractive entry then reads a zero wo and
-// ends the walk (with probability rfr_entry_prob), else the entry direction is cosine-distributed
-// about -N.  On success the exit, the last direction (wi) and the throughput are returned.
-template <class Cast>
-KS_D bool subsurface_walk(SsProfile prof, f3 P, f3 N, f3 Ng, Pcg32 &rng, const Cast &cast, f3 &throughput,
-                          WalkExit &exit, f3 &wi)
+// subsurface_random_walk (subsurface.cpp:222-500) cut into its entry (begin) and its steps, so that a
+// warp can give a lane whose walk is over another one: walks take 1 to 256 steps.
+struct SsWalk
 {
+    SsProfile prof;
+    f3 P, N;            // entry point and shading normal
+    RayQuery ray;       // position and direction
+    Pcg32 rng;
+    f3 throughput;
+    f3 sigma_t, alpha;
+    float diffusion_length, phase_log, guided_fraction;
+    bool have_opposite;
+    float opposite_distance;
+    int bounce;
+    WalkExit exit;
+};
+
+// From an entry point P with shading normal N and geometric normal Ng (the hit frame's); false when the
+// walk ends at once.  The walk starts with D = 0, as BSSRDF::sample calls it (material.cpp:136-140): the
+// refractive entry then reads a zero wo and ends the walk (with probability rfr_entry_prob), else the
+// entry direction is cosine-distributed about -N.  rng and throughput are set by the caller.
+KS_D bool subsurface_begin(SsWalk &s, f3 Ng)
+{
+    SsProfile &prof = s.prof;
+    const f3 P = s.P, N = s.N;
+    Pcg32 &rng = s.rng;
+    f3 &throughput = s.throughput;
+    RayQuery &ray = s.ray;
     // bssrdf_setup_radius (subsurface.cpp:202-216)
     {
         const float eta = prof.ior, inv_eta = 1.0f / eta;
@@ -233,7 +251,6 @@ KS_D bool subsurface_walk(SsProfile prof, f3 P, f3 N, f3 Ng, Pcg32 &rng, const C
     f3 D = cosine_about(e0, e1, -N);
     if (-dot(Ng, D) <= 0.0f)
         return false;
-    RayQuery ray;
     ray.o = wave::spawn_origin(P, D, Ng);
     ray.d = D;
     ray.tmin = 0.0f;
@@ -242,7 +259,9 @@ KS_D bool subsurface_walk(SsProfile prof, f3 P, f3 N, f3 Ng, Pcg32 &rng, const C
     float st[3], al[3];
     for (int c = 0; c < 3; ++c)
         ss_remap(f3_get(prof.albedo, c), f3_get(prof.radius, c), prof.g, st[c], al[c]);
-    f3 sigma_t = mk(st[0], st[1], st[2]), alpha = mk(al[0], al[1], al[2]);
+    s.sigma_t = mk(st[0], st[1], st[2]);
+    f3 &alpha = s.alpha;
+    alpha = mk(al[0], al[1], al[2]);
     const float min_alpha = 0.2f;
     if (alpha.x < min_alpha) {
         throughput.x *= alpha.x / min_alpha;
@@ -256,23 +275,46 @@ KS_D bool subsurface_walk(SsProfile prof, f3 P, f3 N, f3 Ng, Pcg32 &rng, const C
         throughput.z *= alpha.z / min_alpha;
         alpha.z = min_alpha;
     }
-    const f3 sigma_s = mk(sigma_t.x * alpha.x, sigma_t.y * alpha.y, sigma_t.z * alpha.z);
     // diffusion_length_dwivedi (subsurface.cpp:121-125) of the largest alpha
     const float amax = fmaxf(alpha.x, fmaxf(alpha.y, alpha.z));
     const float diffusion_length = 1.0f / sqrtf(1.0f - powf(amax, 2.44294f - 0.0215813f * amax + 0.578637f / amax));
     if (diffusion_length == 1.0f)
         return false;
-    const float phase_log = logf((diffusion_length + 1.0f) / (diffusion_length - 1.0f));
-    bool hit = false, have_opposite = false;
-    float opposite_distance = 0.0f;
-    const float guided_fraction_org = 1.0f - fmaxf(0.5f, powf(fabsf(prof.g), 0.125f));
+    s.diffusion_length = diffusion_length;
+    s.phase_log = logf((diffusion_length + 1.0f) / (diffusion_length - 1.0f));
+    s.guided_fraction = 1.0f - fmaxf(0.5f, powf(fabsf(prof.g), 0.125f));
+    s.have_opposite = false;
+    s.opposite_distance = 0.0f;
+    s.bounce = 0;
+    return true;
+}
+
+// One step; cast(ray, exit) is the mesh-local closest-hit query (LocalGeometry::intersect1: only the entry
+// mesh's triangles).  True when the walk goes on; else `hit` says whether it left the mesh (s.exit, the last
+// direction s.ray.d and s.throughput then hold).
+template <class Cast>
+KS_D bool subsurface_step(SsWalk &s, const Cast &cast, bool &hit)
+{
+    const SsProfile &prof = s.prof;
+    const f3 P = s.P, N = s.N;
+    Pcg32 &rng = s.rng;
+    f3 &throughput = s.throughput;
+    RayQuery &ray = s.ray;
+    const f3 sigma_t = s.sigma_t, alpha = s.alpha;
+    const float diffusion_length = s.diffusion_length, phase_log = s.phase_log;
+    bool &have_opposite = s.have_opposite;
+    float &opposite_distance = s.opposite_distance;
+    WalkExit &exit = s.exit;
+    const int bounce = s.bounce;
+    const f3 sigma_s = mk(sigma_t.x * alpha.x, sigma_t.y * alpha.y, sigma_t.z * alpha.z);
     // the similarity relation past bounce 9 (SUBSURFACE_RANDOM_WALK_SIMILARITY_LEVEL)
     const f3 sigma_s_star = sigma_s * (1.0f - prof.g);
     const f3 sigma_t_star = sigma_t - sigma_s + sigma_s_star;
-    for (int bounce = 0; bounce < 256; ++bounce) {
+    hit = false;
+    {
         const bool late = bounce > 9;
         const float g = late ? 0.0f : prof.g;
-        const float guided_fraction = late ? 0.75f : guided_fraction_org;
+        const float guided_fraction = late ? 0.75f : s.guided_fraction;
         const f3 s_t = late ? sigma_t_star : sigma_t;
         const f3 s_s = late ? sigma_s_star : sigma_s;
         // volume_sample_channel (subsurface.cpp:17-42)
@@ -360,13 +402,10 @@ KS_D bool subsurface_walk(SsProfile prof, f3 P, f3 N, f3 Ng, Pcg32 &rng, const C
         const f3 num = hit ? transmittance : s_s * transmittance;
         const float den = f3_sum(channel_pdf * pdf);
         throughput = throughput * (num / den);
-        if (hit)
-            break;
-        if (fmaxf(throughput.x, fmaxf(throughput.y, throughput.z)) < 1e-6f)
-            break;
+        if (hit || fmaxf(throughput.x, fmaxf(throughput.y, throughput.z)) < 1e-6f)
+            return false;
     }
-    wi = ray.d;
-    return hit;
+    return ++s.bounce < 256;
 }
 
 } // namespace ksb
