@@ -55,6 +55,13 @@ using namespace wave;
 #define KS_WAVE_LOG2 25
 #endif
 
+// Queues of at most this many rays are traced by groups of lanes (k_extend_group, k_shadow_group): from
+// the start of a 641 x 359 pass's late bounces (preview 2.76 -> 2.23 ms; with 8 K rays 2.31, with 128 K 2.24,
+// where the box room goes from 7.05 to 7.27).
+#ifndef KS_GROUP_RAYS
+#define KS_GROUP_RAYS 32768u
+#endif
+
 // Per-iteration counters: paths continuing, shadow rays, hit queue, miss queue, extension-ray
 // fetch, shadow-ray fetch, subsurface walks, walk fetch.
 constexpr uint32_t kCounters = 8;
@@ -243,8 +250,11 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
                                                    float4 *hits, uint32_t *fetch, int *overflow,
                                                    unsigned long long *work, BatchView bv)
 {
-    if constexpr (kBatch)
+    if constexpr (kBatch) {
         count = bv.state->count;
+        if (!kDeep && count <= KS_GROUP_RAYS)
+            return; // k_extend_group's
+    }
     TravCount tc;
     KS_TRAV_STACK(stack);
     using View = TreeOf<kDeep>;
@@ -361,6 +371,18 @@ KS_D void shadow_done(const ShadowBuf &sb, uint32_t i, bool occ, PathBuf nxt, do
     }
 }
 
+// Shadow ray i.
+KS_D RayQuery shadow_ray(const ShadowBuf &sb, uint32_t i)
+{
+    const float4 a = sb.o_tmax[i], b = sb.d_target[i];
+    RayQuery q;
+    q.o = mk(a.x, a.y, a.z);
+    q.d = mk(b.x, b.y, b.z);
+    q.tmin = 0.0f;
+    q.tmax = a.w;
+    return q;
+}
+
 // Any-hit traversal of the NEE shadow rays with dynamic ray fetch (flat scenes); each ray is
 // finished by shadow_done as soon as its traversal ends.
 template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
@@ -370,6 +392,8 @@ __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const _
                                                    unsigned long long *work, GuideView gv, BatchView bv)
 {
     const uint32_t count = *shadow_count;
+    if (kBatch && !kDeep && count <= KS_GROUP_RAYS)
+        return; // k_shadow_group's
     TravCount tc;
     KS_TRAV_STACK(stack);
     using View = TreeOf<kDeep>;
@@ -390,13 +414,7 @@ __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const _
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
             tree = View::tree(sv);
             tris = sv.prim_tris;
-            float4 a = sb.o_tmax[id], b = sb.d_target[id];
-            RayQuery q;
-            q.o = mk(a.x, a.y, a.z);
-            q.d = mk(b.x, b.y, b.z);
-            q.tmin = 0.0f;
-            q.tmax = a.w;
-            if (trav_begin(s, q, View::root(sv), sv.root_count, sv.bmin, sv.bmax))
+            if (trav_begin(s, shadow_ray(sb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
             else
                 shadow_done<kBatch>(sb, id, false, nxt, accum_in, weights_in, gv, bv);
@@ -418,6 +436,77 @@ __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const _
     }
     if (of)
         atomicOr(overflow, 1);
+    flush_counts(tc, work);
+}
+
+// ---- short queues: one ray per group of 4 lanes (ks_traverse4.cuh) ------------------------------
+// Rays go round the warps first, so that few rays share a warp with none.
+#ifndef KS_GROUP_MIN_BLOCKS
+#define KS_GROUP_MIN_BLOCKS 6
+#endif
+KS_D uint32_t group_first_ray()
+{
+    const uint32_t warps = gridDim.x * (kTravBlock / 32), warp = blockIdx.x * (kTravBlock / 32) + (threadIdx.x >> 5);
+    return ((threadIdx.x & 31u) / kGroup) * warps + warp;
+}
+
+// kBatch: paths of many jobs; the count is the device's, and so is the choice between these kernels and the
+// persistent ones (both are launched, one returns).
+template <bool kBatch = false, bool kAlpha = false>
+__global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_extend_group(
+    const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count, float4 *hits, unsigned long long *work,
+    BatchView bv)
+{
+    if constexpr (kBatch) {
+        count = bv.state->count;
+        if (count > KS_GROUP_RAYS)
+            return;
+    }
+    TravCount tc;
+    KS_GROUP_STACK(stack);
+    const uint32_t mask = ((1u << kGroup) - 1u) << (threadIdx.x & 31u & ~(kGroup - 1u));
+    std::conditional_t<kAlpha, SceneAlpha, NoAlpha> filter;
+    if constexpr (kAlpha)
+        filter.sv = &sv_in;
+    const uint32_t stride = gridDim.x * (kTravBlock / kGroup);
+    for (uint32_t i = group_first_ray(); i < count; i += stride) {
+        const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
+        const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+        Trav4 s;
+        if (trav_begin(s, path_ray(pb, i), 0u, sv.root_count, sv.bmin, sv.bmax))
+            group_trace<false>(Tree4{sv.wide, sv.leaf_box}, sv.prim_tris, s, stack, mask, 2, &tc, filter);
+        if ((threadIdx.x & (kGroup - 1u)) == 0)
+            hits[i] = hit_record(s.hit, ambiguous(s));
+    }
+    __syncwarp();
+    flush_counts(tc, work);
+}
+
+template <bool kBatch = false, bool kAlpha = false>
+__global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_shadow_group(
+    const __grid_constant__ SceneView sv_in, ShadowBuf sb, const uint32_t *shadow_count, PathBuf nxt, double *accum,
+    double *weights, unsigned long long *work, GuideView gv, BatchView bv)
+{
+    const uint32_t count = *shadow_count;
+    if (kBatch && count > KS_GROUP_RAYS)
+        return;
+    TravCount tc;
+    KS_GROUP_STACK(stack);
+    const uint32_t mask = ((1u << kGroup) - 1u) << (threadIdx.x & 31u & ~(kGroup - 1u));
+    std::conditional_t<kAlpha, SceneAlpha, NoAlpha> filter;
+    if constexpr (kAlpha)
+        filter.sv = &sv_in;
+    const uint32_t stride = gridDim.x * (kTravBlock / kGroup);
+    for (uint32_t i = group_first_ray(); i < count; i += stride) {
+        const uint32_t job = kBatch ? bits(sb.contrib[i].w) : 0u;
+        const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+        Trav4 s;
+        if (trav_begin(s, shadow_ray(sb, i), 0u, sv.root_count, sv.bmin, sv.bmax))
+            group_trace<true>(Tree4{sv.wide, sv.leaf_box}, sv.prim_tris, s, stack, mask, 2, &tc, filter);
+        if ((threadIdx.x & (kGroup - 1u)) == 0)
+            shadow_done<kBatch>(sb, i, s.hit.tri != ~0u, nxt, accum, weights, gv, bv);
+    }
+    __syncwarp();
     flush_counts(tc, work);
 }
 
@@ -486,13 +575,7 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_shadow_inst_pt(cons
     while (true) {
         const uint32_t id = warp_fetch(fetch, count, ray == ~0u, drained);
         if (id != ~0u) {
-            float4 a = sb.o_tmax[id], b = sb.d_target[id];
-            RayQuery q;
-            q.o = mk(a.x, a.y, a.z);
-            q.d = mk(b.x, b.y, b.z);
-            q.tmin = 0.0f;
-            q.tmax = a.w;
-            if (inst_begin(s, sv.inst, q))
+            if (inst_begin(s, sv.inst, shadow_ray(sb, id)))
                 ray = id;
             else
                 shadow_done<false>(sb, id, false, nxt, accum, weights, gv, BatchView{});
@@ -944,6 +1027,9 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                                                  : resident_grid(ext_kernel, 128, ctx->sm_count);
     const unsigned shadow_grid = scene->n_instances ? resident_grid(k_shadow_inst_pt, 128, ctx->sm_count)
                                                     : resident_grid(shadow_kernel, 128, ctx->sm_count);
+    const auto ext_group = alpha ? k_extend_group<false, true> : k_extend_group<>;
+    const auto shadow_group = alpha ? k_shadow_group<false, true> : k_shadow_group<>;
+    const unsigned ext_group_grid = resident_grid(ext_group, kTravBlock, ctx->sm_count);
     int cur = 0;
     cudaError_t err = cudaSuccess;
     std::vector<double> cb_acc, cb_w;
@@ -980,10 +1066,14 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             // counters: [0] next paths, [1] shadow rays, [2] hit queue, [3] miss queue, [4], [5] ray fetch
             cudaMemsetAsync(w.counters.ptr, 0, sizeof(uint32_t) * kCounters, st);
             unsigned grid = std::min<unsigned>((count + 127) / 128, max_grid);
+            const bool grouped = !scene->n_instances && !scene->deep && count <= KS_GROUP_RAYS;
+            const unsigned group_grid = std::min<unsigned>((count + 3) / 4, ext_group_grid);
             cudaEventRecord(ev[1], st);
             if (scene->n_instances)
                 k_extend_inst_pt<<<std::min(grid, ext_grid), 128, 0, st>>>(
                     sv, pb[cur], count, w.hits.ptr, w.hit_inst.ptr, w.counters.ptr + 4, w.overflow.ptr, work.ptr);
+            else if (grouped)
+                ext_group<<<group_grid, kTravBlock, 0, st>>>(sv, pb[cur], count, w.hits.ptr, work.ptr, BatchView{});
             else
                 ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, w.counters.ptr + 4,
                                                                      w.overflow.ptr, work.ptr, BatchView{});
@@ -1037,6 +1127,9 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                 k_shadow_inst_pt<<<std::min(grid, shadow_grid), 128, 0, st>>>(
                     sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
                     work.ptr + 2, gv);
+            else if (grouped)
+                shadow_group<<<group_grid, kTravBlock, 0, st>>>(sv, sb, w.counters.ptr + 1, pb[1 - cur], d_accum,
+                                                                d_weights, work.ptr + 2, gv, BatchView{});
             else
                 shadow_kernel<<<std::min(grid, shadow_grid), 128, 0, st>>>(
                     sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
@@ -1167,7 +1260,7 @@ struct BatchWork
     DevBuf<unsigned long long> path_begin;
     DevBuf<BatchState> state_dev;
     DevBuf<float> filters; // the jobs' pixel-filter sample tables, concatenated
-    unsigned ext_grid = 0, shadow_grid = 0; // one wave of resident CTAs of the traversal kernels
+    unsigned ext_grid = 0, shadow_grid = 0, group_grid = 0; // one wave of resident CTAs of the traversal kernels
     int variant = kShadePlain;              // the shading kernel variant of the most demanding job
     bool deep = false;                      // some job's tree is too deep for the 4-wide view
 };
@@ -1263,6 +1356,8 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     const auto shadow_kernel = w.deep ? k_shadow_pt<true, false, true> : k_shadow_pt<true>;
     ext_kernel<<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, cnt + 4, w.overflow.ptr,
                                                 w.work.ptr, bv);
+    if (!w.deep)
+        k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, w.work.ptr, bv);
     k_build_queues<true><<<grid, 256, 0, st>>>(SceneView{}, pb[cur], w.hits.ptr, 0u, w.queue[0].ptr,
                                                w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, bv);
     launch_sample(true, grid, st, SceneView{}, RenderParams{}, pb[cur], w.hits.ptr, nullptr, w.queue[0].ptr, cnt + 2,
@@ -1273,6 +1368,9 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
                      gv, bv);
     shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
                                                    w.overflow.ptr, w.work.ptr + 2, gv, bv);
+    if (!w.deep)
+        k_shadow_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, sb, cnt + 1, pb[1 - cur], nullptr, nullptr,
+                                                                  w.work.ptr + 2, gv, bv);
     k_batch_advance<<<1, 32, 0, st>>>(bv.state, cnt, handle, use_graph);
 }
 
@@ -1294,6 +1392,7 @@ static ks_status batch_render(ks_context *ctx, const ks_batch_job *jobs, uint32_
                         : resident_grid(k_extend_pt<true>, 128, ctx->sm_count);
     w.shadow_grid = w.deep ? resident_grid(k_shadow_pt<true, false, true>, 128, ctx->sm_count)
                            : resident_grid(k_shadow_pt<true>, 128, ctx->sm_count);
+    w.group_grid = resident_grid(k_extend_group<true>, kTravBlock, ctx->sm_count);
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < 4; ++f)
             KS_CUDA_TRY(ctx, w.state[b][f].alloc(capacity));

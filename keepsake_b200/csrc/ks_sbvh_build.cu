@@ -1062,7 +1062,9 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     KS_CUDA_TRY(ctx, cudaMemcpyAsync(&n_trav, interior_scan.ptr + n_nodes, 4, cudaMemcpyDeviceToHost, st));
     KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     KS_CUDA_TRY(ctx, out.trav.alloc(n_trav > 0 ? n_trav : 1));
-    KS_CUDA_TRY(ctx, out.prim_tris.alloc((size_t)pool_used * 3));
+    // records past the end are read (not used) with the last leaf, by the lanes of a group (ks_traverse4.cuh)
+    KS_CUDA_TRY(ctx, out.prim_tris.alloc(((size_t)pool_used + kPrimPad) * 3));
+    KS_CUDA_TRY(ctx, cudaMemsetAsync(out.prim_tris.ptr + 3 * (size_t)pool_used, 0, sizeof(float4) * 3 * kPrimPad, st));
     KS_CUDA_TRY(ctx, out.leaf_box.alloc((size_t)pool_used * 2));
     k_prim_tris<<<grid_for(pool_used, 256), 256, 0, st>>>(out.prims.ptr, pool_used, verts, indices, recs.ptr,
                                                           out.prim_tris.ptr, out.leaf_box.ptr);

@@ -31,6 +31,7 @@ struct TravNode
 constexpr uint32_t kLeafBit = 0x80000000u;
 // Bits of v1.w in a primitive's record (3 float4: v0 + triangle id, v1 + this mark, v2) that ends a leaf.
 constexpr uint32_t kLastPrim = 0x3f800000u;
+constexpr uint32_t kPrimPad = 4; // records of padding after the last
 
 // A node of the exact traversal's 4-wide steps (ks_traverse.cuh): the children of an interior node, each
 // interior child replaced by its own two children (2 to 4 slots, in order).  Slot boxes are the SBVH's

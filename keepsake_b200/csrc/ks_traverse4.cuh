@@ -234,6 +234,22 @@ KS_D bool leaf_reached(const float4 *__restrict__ leaf_box, const Trav4 &s, uint
     return slab(s.ray, exact_helper(s), bmin, bmax, entry, t1) && t1 > s.ray.tmin && entry < s.ray.tmax;
 }
 
+// Takes note of a closest-hit ray's hit on a triangle of a leaf that the ray enters at `entry`.
+KS_D void trav4_take(Trav4 &s, const Hit &h, float entry)
+{
+    if (h.tri == s.hit.tri) {
+        s.entry = fminf(s.entry, entry); // the same triangle through another of its leaves
+    } else if (s.hit.tri == ~0u || h.t < s.hit.t) {
+        if (s.hit.tri != ~0u)
+            s.second = fminf(s.second, s.hit.t);
+        s.entry = entry;
+        s.limit = fminf(s.ray.tmax, h.t + fabsf(h.t) * kPruneSlack);
+        s.hit = h;
+    } else {
+        s.second = fminf(s.second, h.t);
+    }
+}
+
 // Tests the leaf at hand; true when an any-hit query found an occluder.
 template <bool kAnyHit, class Alpha>
 KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restrict__ tris, Trav4 &s, int culling,
@@ -261,22 +277,7 @@ KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restri
                     return true;
                 }
             } else if (t < s.limit && leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
-                if (tri == s.hit.tri) {
-                    s.entry = fminf(s.entry, entry); // the same triangle through another of its leaves
-                } else if (s.hit.tri == ~0u || t < s.hit.t) {
-                    if (s.hit.tri != ~0u)
-                        s.second = fminf(s.second, s.hit.t);
-                    s.entry = entry;
-                    s.limit = fminf(s.ray.tmax, t + fabsf(t) * kPruneSlack);
-                    s.hit.tri = tri;
-                    s.hit.slot = slot;
-                    s.hit.t = t;
-                    s.hit.b0 = b0;
-                    s.hit.b1 = b1;
-                    s.hit.b2 = b2;
-                } else {
-                    s.second = fminf(s.second, t);
-                }
+                trav4_take(s, Hit{tri, slot, t, b0, b1, b2}, entry);
             }
         }
         ++slot;
@@ -297,6 +298,127 @@ KS_D bool trav_step(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 &s
             return false;
     }
     return !trav4_pop<kAnyHit>(tree.nodes, s, stack);
+}
+
+// ---- one ray per group of 4 lanes -------------------------------------------------------------
+// A queue shorter than the GPU takes the time of its longest ray, whatever the throughput: some hundred
+// rays along a bumpy surface took 100 to 170 us a launch, one dependent step after the other.  Here the 4
+// lanes of a group follow one ray: a lane tests one slot of a node or one triangle of a leaf, so a step's
+// chain is that of one box instead of four, a sort and three pushes.  Every lane holds the ray's state
+// (the same values); the same tests make the same hits.  The stack is the group's, in shared memory.
+constexpr int kGroup = 4, kGroupStack = kWideStackDepth; // entries of (ref, entry time)
+
+struct GroupStack
+{
+    uint2 *e;
+};
+#define KS_GROUP_STACK(name)                                                                                     \
+    __shared__ uint2 name##_smem[kTravBlock / kGroup][kGroupStack];                                             \
+    const GroupStack name{name##_smem[threadIdx.x / kGroup]}
+
+// One ray from trav_begin to its end; `mask`: the group's lanes.
+template <bool kAnyHit, class Alpha>
+KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 &s, const GroupStack &stack,
+                      uint32_t mask, int culling, TravCount *count, const Alpha &alpha)
+{
+    const uint32_t lane = threadIdx.x & 31u, k = lane & (kGroup - 1u), shift = lane & ~(kGroup - 1u);
+    while (true) {
+        if (!s.at_leaf()) {
+            if (k == 0)
+                count->nodes += 2;
+            const float *n = reinterpret_cast<const float *>(tree.nodes + s.ref) + k;
+            const int ux = s.inv.x < 0.0f ? 4 : 0, uy = s.inv.y < 0.0f ? 4 : 0, uz = s.inv.z < 0.0f ? 4 : 0;
+            const float ex = __ldg(n + ux), ey = __ldg(n + 8 + uy), ez = __ldg(n + 16 + uz);
+            const float lx = __ldg(n + 4 - ux), ly = __ldg(n + 12 - uy), lz = __ldg(n + 20 - uz);
+            const uint32_t ref = __float_as_uint(__ldg(n + 24));
+            const float t_in = max3f(fmaf(ex, s.inv.x, -s.o_in.x), fmaf(ey, s.inv.y, -s.o_in.y),
+                                     fmaxf(fmaf(ez, s.inv.z, -s.o_in.z), s.ray.tmin));
+            const float t_out = min3f(fmaf(lx, s.inv_out.x, -s.o_out.x), fmaf(ly, s.inv_out.y, -s.o_out.y),
+                                      fminf(fmaf(lz, s.inv_out.z, -s.o_out.z), s.limit));
+            const bool ok = t_in <= t_out;
+            const uint32_t hits = (__ballot_sync(mask, ok) >> shift) & ((1u << kGroup) - 1u);
+            if (hits) {
+                const int n_hit = __popc(hits);
+                int rank; // among the slots hit: by time, any-hit queries by slot
+                if constexpr (kAnyHit) {
+                    rank = __popc(hits & ((1u << k) - 1u));
+                } else {
+                    const uint32_t key = ok ? ((__float_as_uint(t_in) & ~3u) | k) : ~0u;
+                    rank = 0;
+#pragma unroll
+                    for (int x = 1; x < kGroup; ++x)
+                        rank += __shfl_xor_sync(mask, key, x) < key ? 1 : 0;
+                }
+                if (ok && rank > 0)
+                    stack.e[s.sp + n_hit - 1 - rank] = make_uint2(ref, __float_as_uint(t_in));
+                const uint32_t first = (__ballot_sync(mask, ok && rank == 0) >> shift) & ((1u << kGroup) - 1u);
+                s.ref = __shfl_sync(mask, ref, (int)(shift + __ffs(first) - 1u));
+                s.sp += n_hit - 1;
+                __syncwarp(mask);
+                continue;
+            }
+        } else {
+            const uint32_t first = s.ref & ~kLeafBit;
+            uint32_t base = first;
+            bool last = false;
+            while (!last) {
+                // the record past the leaf's last is another leaf's or the array's padding: read, not used
+                const uint32_t slot = base + k;
+                const float4 *p = tris + 3 * (size_t)slot;
+                const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+                const uint32_t ends =
+                    (__ballot_sync(mask, __float_as_uint(b.w) != 0u) >> shift) & ((1u << kGroup) - 1u);
+                last = ends != 0u;
+                const bool mine = !last || (int)k < __ffs(ends);
+                const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
+                RayQuery q = s.ray;
+                q.tmax = s.limit;
+                Hit h;
+                h.tri = __float_as_uint(a.w);
+                h.slot = slot;
+                float entry = 0.0f;
+                bool take = false;
+                if (mine) {
+                    count->tris++;
+                    take = !cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, h.t, h.b0, h.b1, h.b2) &&
+                           (kAnyHit || h.t < s.limit) && leaf_reached(tree.leaf_box, s, first, entry) &&
+                           alpha(h.tri, h.b1, h.b2, s.ray);
+                }
+                uint32_t found = (__ballot_sync(mask, take) >> shift) & ((1u << kGroup) - 1u);
+                if constexpr (kAnyHit) {
+                    if (found) {
+                        s.hit.tri = 0u;
+                        return;
+                    }
+                } else {
+                    for (; found; found &= found - 1u) { // in the leaf's order, as one lane would
+                        const int src = (int)(shift + __ffs(found) - 1u);
+                        Hit g;
+                        g.tri = __shfl_sync(mask, h.tri, src);
+                        g.slot = __shfl_sync(mask, h.slot, src);
+                        g.t = __shfl_sync(mask, h.t, src);
+                        g.b0 = __shfl_sync(mask, h.b0, src);
+                        g.b1 = __shfl_sync(mask, h.b1, src);
+                        g.b2 = __shfl_sync(mask, h.b2, src);
+                        const float at = __shfl_sync(mask, entry, src);
+                        if (g.t < s.limit)
+                            trav4_take(s, g, at);
+                    }
+                }
+                base += kGroup;
+            }
+        }
+        // the next pending child
+        bool more = false;
+        while (s.sp > 0 && !more) {
+            const uint2 e = stack.e[--s.sp];
+            s.ref = e.x;
+            more = kAnyHit || __uint_as_float(e.y) <= s.limit;
+        }
+        __syncwarp(mask);
+        if (!more)
+            return;
+    }
 }
 
 // The closest hit by the exact traversal's own order: the 4-wide steps over boxes read from the

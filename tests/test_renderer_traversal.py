@@ -57,3 +57,43 @@ def test_wide_traversal_matches_binary(ctx, kind, n, culling):
     if kind not in ("flat", "copies"):  # no coplanar or repeated triangles: ties are rare
         assert (~same).mean() < 1e-3 and (off <= 8 * 2.0 ** -23).all()
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(1, 1), (181, 181), (182, 182), (600, 400)])
+@pytest.mark.parametrize("batch", [False, True])
+def test_short_queues_render_the_same(ctx, W, H, batch):
+    """Queues of up to 2^15 rays are traced by groups of lanes, longer ones by a lane per ray: a frame
+    rendered whole equals, pixel by pixel, the same frame rendered in crops whose queues are shorter
+    (181 x 181 is the largest square below the limit, 182 x 182 the first above it).  Both ways make the
+    same tests, so the sums differ by the order of FP64 additions only."""
+    import torch
+
+    import keepsake_b200 as ks
+    g = ks.Generated("icosphere", 3, level=5, sky=(128, 64), resolution=(W, H))
+    s = ks.Scene(ctx, g.desc)
+    s.build_bvh()
+    cam = ks.camera_perspective(g.camera_to_world, g.vfov, g.aspect)
+    size = dict(render_width=W, render_height=H, spp=1, bounces=6)
+
+    def render(**crop):
+        acc = torch.zeros((H, W, 3), dtype=torch.float64, device="cuda")
+        wts = torch.zeros((H, W, 2), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        p = ks.SmallPTParams.make(**size, **crop)
+        if batch:
+            ks.batch_render(ctx, [(s, cam, p, acc.data_ptr(), wts.data_ptr())])
+        else:
+            s.render_device(cam, p, acc.data_ptr(), wts.data_ptr())
+        return acc.cpu().numpy(), wts.cpu().numpy()
+
+    acc, wts = render()
+    rows = max(1, 8192 // W)
+    acc_c, wts_c = np.zeros_like(acc), np.zeros_like(wts)
+    for y in range(0, H, rows):
+        a, w = render(crop_start_x=0, crop_start_y=y, crop_width=W, crop_height=min(rows, H - y))
+        acc_c += a
+        wts_c += w
+    assert np.array_equal(wts, wts_c)
+    assert np.allclose(acc, acc_c, rtol=1e-14, atol=0)
+    s.close()
