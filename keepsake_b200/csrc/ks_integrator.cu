@@ -63,8 +63,8 @@ using namespace wave;
 #endif
 
 // Per-iteration counters: paths continuing, shadow rays, hit queue, miss queue, extension-ray
-// fetch, shadow-ray fetch, subsurface walks, walk fetch.
-constexpr uint32_t kCounters = 8;
+// fetch, shadow-ray fetch, subsurface walks, walk fetch, simple hits, general hits.
+constexpr uint32_t kCounters = 10;
 
 // ---- kernels --------------------------------------------------------------------------------
 
@@ -303,11 +303,15 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
 // Hit and miss queues from the per-ray results of k_extend_pt, one CTA-aggregated append per
 // kind (queue order follows the path index within each CTA's tile).  The few rays whose closest hit
 // depends on the visiting order are traced again here first.
-template <bool kBatch = false>
+// kSplit: a scene (of some job) with materials of both kinds; the hits also go to one of two queues by the
+// shading variant their material needs (simple_queue at 0, general ones at split_cap).  Mixed in one queue,
+// the warps of an SM ran all BSDF kinds at once and waited for instructions 28 of 45 cycles.
+template <bool kBatch = false, bool kSplit = false>
 __global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__ SceneView sv_in, PathBuf pb, float4 *hits,
                                                       uint32_t count, uint32_t *hit_queue,
                                                       uint32_t *miss_queue, uint32_t *queue_counts, int *overflow,
-                                                      int alpha, BatchView bv)
+                                                      int alpha, uint32_t *split_queue, uint32_t split_cap,
+                                                      uint32_t *split_counts, BatchView bv)
 {
     if constexpr (kBatch)
         count = bv.state->count;
@@ -339,6 +343,19 @@ __global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__
                 hit_queue[jh] = i;
             else
                 miss_queue[jm] = i;
+        }
+        if constexpr (kSplit) {
+            bool general = false;
+            if (is_hit) {
+                const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
+                const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+                const uint32_t tri = bits(__ldg(&sv.prim_tris[3 * (size_t)slot].w));
+                general = (__ldg(&sv.mesh_flags[__ldg(&sv.tri_mesh[tri])]) & kMeshGeneral) != 0;
+            }
+            uint32_t js, jg;
+            block_append2(split_counts, is_hit && !general, split_counts + 1, general, js, jg);
+            if (is_hit)
+                split_queue[general ? (size_t)split_cap + jg : (size_t)js] = i;
         }
     }
 }
@@ -686,6 +703,7 @@ struct RenderWork
     DevBuf<uint32_t> counters; // [next, shadow, hit queue, miss queue, extension fetch, shadow fetch]
     DevBuf<uint32_t> queue[2]; // hit / miss path indices
     DevBuf<uint32_t> walks;    // scenes with subsurface materials: paths that walk this bounce
+    DevBuf<uint32_t> split;    // scenes of mixed materials: simple hits, then (at the capacity) general ones
     DevBuf<int> overflow;
     DevBuf<float> filter; // the pixel filter's sample table (Gaussian / Blackman-Harris)
     uint32_t capacity = 0;
@@ -925,6 +943,9 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
         KS_CUDA_TRY(ctx, w.hit_inst.reserve(w.capacity));
     if (scene->any_subsurface)
         KS_CUDA_TRY(ctx, w.walks.reserve(w.capacity));
+    const bool split = scene->mixed_materials;
+    if (split)
+        KS_CUDA_TRY(ctx, w.split.reserve(2 * (size_t)w.capacity));
     KS_CUDA_TRY(ctx, w.samples.reserve(4 * (size_t)w.capacity));
     if (rp.filter_n) {
         KS_CUDA_TRY(ctx, w.filter.reserve(ftab.size()));
@@ -1077,9 +1098,10 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             else
                 ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, w.counters.ptr + 4,
                                                                      w.overflow.ptr, work.ptr, BatchView{});
-            k_build_queues<false><<<std::min((count + 255) / 256, max_grid), 256, 0, st>>>(
-                sv, pb[cur], w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2,
-                w.overflow.ptr, alpha, BatchView{});
+            (split ? k_build_queues<false, true> : k_build_queues<false>)<<<std::min((count + 255) / 256, max_grid), 256, 0,
+                                                                             st>>>(
+                sv, pb[cur], w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2, w.overflow.ptr, alpha,
+                w.split.ptr, w.capacity, w.counters.ptr + 8, BatchView{});
             stats.kernel_launches++;
             cudaEventRecord(ev[2], st);
             const bool guiding = guide && gv.active;
@@ -1115,12 +1137,20 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             launch_sample(false, grid, st, sv, rp, pb[cur], w.hits.ptr, w.hit_inst.ptr, w.queue[0].ptr,
                           w.counters.ptr + 2, w.samples.ptr, BatchView{});
             // misses first (they do not read the guide), then the hits once the guide has joined
-            for (int miss = 1; miss >= 0; --miss) {
-                if (!miss && guiding)
-                    cudaStreamWaitEvent(st, ev_join, 0);
-                launch_shade(miss != 0, guide != nullptr, false, variant, grid, st, sv, rp, pb[cur], pb[1 - cur], w.hits.ptr,
-                             w.hit_inst.ptr, w.samples.ptr, w.queue[miss].ptr, w.counters.ptr + 2 + miss,
-                             w.counters.ptr, sb, w.counters.ptr + 1, d_accum, d_weights, gv, BatchView{});
+            auto shade = [&](bool miss, int kernel_variant, const uint32_t *queue, const uint32_t *n) {
+                launch_shade(miss, guide != nullptr, false, kernel_variant, grid, st, sv, rp, pb[cur], pb[1 - cur],
+                             w.hits.ptr, w.hit_inst.ptr, w.samples.ptr, queue, n, w.counters.ptr, sb, w.counters.ptr + 1,
+                             d_accum, d_weights, gv, BatchView{});
+            };
+            shade(true, variant, w.queue[1].ptr, w.counters.ptr + 3);
+            if (guiding)
+                cudaStreamWaitEvent(st, ev_join, 0);
+            if (split) {
+                shade(false, sv.simple_variant, w.split.ptr, w.counters.ptr + 8);
+                shade(false, variant, w.split.ptr + w.capacity, w.counters.ptr + 9);
+                stats.kernel_launches++;
+            } else {
+                shade(false, variant, w.queue[0].ptr, w.counters.ptr + 2);
             }
             cudaEventRecord(ev[3], st);
             if (scene->n_instances)
@@ -1251,7 +1281,7 @@ struct BatchWork
 {
     DevBuf<float4> state[2][4];
     DevBuf<float4> hits, samples, shadow[4];
-    DevBuf<uint32_t> counters, queue[2];
+    DevBuf<uint32_t> counters, queue[2], split;
     DevBuf<int> overflow;
     DevBuf<unsigned long long> work;
     DevBuf<SceneView> views;
@@ -1262,6 +1292,8 @@ struct BatchWork
     DevBuf<float> filters; // the jobs' pixel-filter sample tables, concatenated
     unsigned ext_grid = 0, shadow_grid = 0, group_grid = 0; // one wave of resident CTAs of the traversal kernels
     int variant = kShadePlain;              // the shading kernel variant of the most demanding job
+    int simple_variant = kShadePlain;       // ... and of the hits that do not need the general one
+    bool any_simple = false;                // some job has such hits
     bool deep = false;                      // some job's tree is too deep for the 4-wide view
 };
 
@@ -1278,7 +1310,8 @@ static ks_status batch_tables(ks_context *ctx, const ks_batch_job *jobs, uint32_
     std::vector<float> filter_host;
     std::vector<size_t> filter_off(n, 0);
     *max_bounces = 0;
-    w.variant = kShadePlain;
+    w.variant = w.simple_variant = kShadePlain;
+    w.any_simple = false;
     w.deep = false;
     for (uint32_t j = 0; j < n; ++j) {
         const ks_batch_job &jb = jobs[j];
@@ -1313,6 +1346,8 @@ static ks_status batch_tables(ks_context *ctx, const ks_batch_job *jobs, uint32_
                                                      "with ks_small_pt_render)");
         views[j] = make_view(jb.scene);
         w.variant = std::max(w.variant, views[j].shade_variant);
+        w.simple_variant = std::max(w.simple_variant, views[j].simple_variant);
+        w.any_simple = w.any_simple || jb.scene->mixed_materials || views[j].shade_variant != kShadeGeneral;
         w.deep = w.deep || jb.scene->deep;
         acc[j] = jb.accum_rgb_device;
         wts[j] = jb.weights_device;
@@ -1358,14 +1393,23 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
                                                 w.work.ptr, bv);
     if (!w.deep)
         k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, w.work.ptr, bv);
-    k_build_queues<true><<<grid, 256, 0, st>>>(SceneView{}, pb[cur], w.hits.ptr, 0u, w.queue[0].ptr,
-                                               w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, bv);
+    const bool split = w.split.ptr != nullptr;
+    (split ? k_build_queues<true, true> : k_build_queues<true>)<<<grid, 256, 0, st>>>(
+        SceneView{}, pb[cur], w.hits.ptr, 0u, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, w.split.ptr,
+        capacity, cnt + 8, bv);
     launch_sample(true, grid, st, SceneView{}, RenderParams{}, pb[cur], w.hits.ptr, nullptr, w.queue[0].ptr, cnt + 2,
                   w.samples.ptr, bv);
-    for (int miss = 0; miss < 2; ++miss)
-        launch_shade(miss != 0, false, true, w.variant, grid, st, SceneView{}, RenderParams{}, pb[cur], pb[1 - cur], w.hits.ptr,
-                     nullptr, w.samples.ptr, w.queue[miss].ptr, cnt + 2 + miss, cnt, sb, cnt + 1, nullptr, nullptr,
-                     gv, bv);
+    auto shade = [&](bool miss, int kernel_variant, const uint32_t *queue, const uint32_t *n) {
+        launch_shade(miss, false, true, kernel_variant, grid, st, SceneView{}, RenderParams{}, pb[cur], pb[1 - cur],
+                     w.hits.ptr, nullptr, w.samples.ptr, queue, n, cnt, sb, cnt + 1, nullptr, nullptr, gv, bv);
+    };
+    if (split) {
+        shade(false, w.simple_variant, w.split.ptr, cnt + 8);
+        shade(false, w.variant, w.split.ptr + capacity, cnt + 9);
+    } else {
+        shade(false, w.variant, w.queue[0].ptr, cnt + 2);
+    }
+    shade(true, w.variant, w.queue[1].ptr, cnt + 3);
     shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
                                                    w.overflow.ptr, w.work.ptr + 2, gv, bv);
     if (!w.deep)
@@ -1400,6 +1444,8 @@ static ks_status batch_render(ks_context *ctx, const ks_batch_job *jobs, uint32_
     KS_CUDA_TRY(ctx, w.samples.alloc(4 * (size_t)capacity));
     for (auto &q : w.queue)
         KS_CUDA_TRY(ctx, q.alloc(capacity));
+    if (w.variant == kShadeGeneral && w.any_simple)
+        KS_CUDA_TRY(ctx, w.split.alloc(2 * (size_t)capacity));
     for (auto &f : w.shadow)
         KS_CUDA_TRY(ctx, f.alloc(capacity));
     KS_CUDA_TRY(ctx, w.counters.alloc(kCounters));

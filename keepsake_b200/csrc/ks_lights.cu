@@ -461,9 +461,8 @@ SceneView make_view(const ks_scene *s)
     v.tex_texels = s->tex_texels.ptr;
     v.tex_info = s->tex_info.ptr;
     v.bindings = s->bindings.ptr;
-    v.shade_variant = (s->ext_materials || s->any_bindings) ? kShadeGeneral
-                      : (s->normals.ptr != nullptr || s->texcoords.ptr != nullptr) ? kShadeAttribs
-                                                                                     : kShadePlain;
+    v.simple_variant = (s->normals.ptr != nullptr || s->texcoords.ptr != nullptr) ? kShadeAttribs : kShadePlain;
+    v.shade_variant = (s->ext_materials || s->any_bindings) ? kShadeGeneral : v.simple_variant;
     v.light_count = s->light_count;
     v.n_nonmesh = s->n_nonmesh;
     v.n_sky = (s->sky_desc.kind >= 1 && s->sky_desc.kind <= 3) ? 1u : 0u;

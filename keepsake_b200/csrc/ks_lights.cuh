@@ -36,7 +36,7 @@ struct SceneView
     float bmin[3], bmax[3];
     const uint32_t *tri_mesh;
     const uint32_t *mesh_material;
-    const int *mesh_flags;   // per mesh: kMeshTwosided | kMeshSmooth | kMeshTexcoords
+    const int *mesh_flags;   // per mesh: kMeshTwosided | kMeshSmooth | kMeshTexcoords | kMeshGeneral
     const float *normals;    // global vertex normals (3 floats each; null when no mesh shades smooth)
     const float *texcoords;  // global texture coordinates (2 floats each; null when no mesh has them)
     const MaterialGPU *materials;
@@ -46,6 +46,7 @@ struct SceneView
     // the shading kernel variant the scene needs: kShadePlain; kShadeAttribs for vertex normals or
     // texcoords; kShadeGeneral for a material other than the GGX PrincipledBSDF
     int shade_variant;
+    int simple_variant; // ... and the one that its meshes without kMeshGeneral need
     // lights
     uint32_t light_count;
     uint32_t n_nonmesh; // the sky (light 0, when there is one) and the point / directional lights

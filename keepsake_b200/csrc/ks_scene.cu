@@ -692,6 +692,15 @@ ks_status ks_scene_create(ks_context *ctx, const ks_scene_desc *desc, ks_scene *
         s->any_emission_map |= (mats[m].tex_flags & kMatEmissionMap) != 0;
     }
     s->any_bindings = !binds.empty();
+    size_t general = 0;
+    for (size_t k = 0; k < s->host.mesh_flags.size(); ++k) {
+        const ks_material_desc &m = desc->materials[s->host.mesh_material[k]];
+        if (m.bsdf != 0 || m.microfacet != 0 || m.has_subsurface != 0 || mats[s->host.mesh_material[k]].bind_count) {
+            s->host.mesh_flags[k] |= kMeshGeneral;
+            ++general;
+        }
+    }
+    s->mixed_materials = general > 0 && general < s->host.mesh_flags.size();
     if (s->any_emission_map) {
         s->emit_tex.texels = texels;
         s->emit_tex.info = tex_info;

@@ -65,7 +65,8 @@ enum : int
 {
     kMeshTwosided = 1,
     kMeshSmooth = 2,
-    kMeshTexcoords = 4
+    kMeshTexcoords = 4,
+    kMeshGeneral = 8 // its material needs the general shading variant (kShadeGeneral)
 };
 
 // Device copy of one material (constant principled fields + emission).
@@ -138,6 +139,7 @@ struct ks_scene
     ksb::DevBuf<uint32_t> mesh_material;
     ksb::DevBuf<int> mesh_flags;
     bool ext_materials = false; // some material is not a GGX PrincipledBSDF
+    bool mixed_materials = false; // some meshes need the general shading variant and some do not
     // textures (linear float texels, 4 per texel), their sizes, the bindings grouped by material
     ksb::DevBuf<float4> tex_texels;
     ksb::DevBuf<ksb::TexInfo> tex_info;
