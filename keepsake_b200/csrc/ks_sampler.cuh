@@ -104,16 +104,6 @@ KS_HD float sobol_sample_01(uint64_t a, int dim, uint32_t seed)
     return f < kOneMinusEps ? f : kOneMinusEps;
 }
 
-// mix_bits (hash.h:206-214) of a value below 2^32, then (>> 24) % 24 as in sobol.h:209.
-KS_HD int digit_perm_index(uint32_t x)
-{
-    uint64_t v = mix_bits64((uint64_t)x);
-    uint64_t y = v >> 24; // < 2^40
-    // y % 24 without a 64-bit division: 2^32 = 16 (mod 24)
-    uint32_t hi = (uint32_t)(y >> 32), lo = (uint32_t)y;
-    return (int)((hi * 16u + lo % 24u) % 24u);
-}
-
 KS_HD uint32_t part1by1(uint32_t x)
 {
     x &= 0x0000ffffu;
@@ -124,21 +114,42 @@ KS_HD uint32_t part1by1(uint32_t x)
     return x;
 }
 
-// All 24 orderings of {0,1,2,3}, in the order the reference enumerates them (sobol.h:169-199).
-KS_HD int digit_permutation(int p, int digit)
+// The 24 orderings of {0, 1, 2, 3} in the order the reference enumerates them (sobol.h:169-199), by digit:
+// 2 bits per ordering p (ordering 0 in the low bits), 8 orderings to a 16-bit word, so that the word of
+// p / 8 shifted right by 2 (p % 8) has the digit's image in its low bits.
+struct DigitTable
 {
-    // Packed: 2 bits per entry (entry 0 in the low bits), one byte per permutation, 8 bytes per
-    // 64-bit word, so the lookup stays in registers.  Bytes, permutation 0 first:
-    //   E4 B4 D8 78 6C 9C E1 B1 | C9 39 2D 8D C6 36 D2 72 | 4E 1E 27 87 1B 4B 63 93
-    constexpr uint64_t w0 = 0xB1E19C6C78D8B4E4ull, w1 = 0x72D236C68D2D39C9ull, w2 = 0x93634B1B87271E4Eull;
-    const uint64_t w = p < 8 ? w0 : (p < 16 ? w1 : w2);
-#ifdef __CUDA_ARCH__
-    // byte p & 7 of the word in the low byte (one byte-permute instead of a 64-bit shift)
-    const uint32_t byte = __byte_perm((uint32_t)w, (uint32_t)(w >> 32), (uint32_t)(p & 7));
-#else
-    const uint32_t byte = (uint32_t)(w >> (8 * (p & 7))) & 0xffu;
-#endif
-    return (int)((byte >> (2 * digit)) & 3u);
+    uint32_t w[3];
+};
+KS_HD DigitTable digit_table(uint32_t digit)
+{
+    // per digit: words p / 8 = 0 and 1 packed in 32 bits, then word 2
+    constexpr uint32_t w01[4] = {0xaa555000u, 0x05fa0fa5u, 0xdc2ce6deu, 0x7383b97bu}, w2[4] = {0xfffau, 0x0a5fu, 0x6124u, 0x9481u};
+    const uint32_t a = digit < 2 ? (digit == 0 ? w01[0] : w01[1]) : (digit == 2 ? w01[2] : w01[3]);
+    const uint32_t c = digit < 2 ? (digit == 0 ? w2[0] : w2[1]) : (digit == 2 ? w2[2] : w2[3]);
+    return DigitTable{{a, a >> 16, c}};
+}
+
+// The image of the table's digit under ordering (mix_bits(x) >> 24) % 24 (sobol.h:209; x below 2^32).
+// mix_bits in 32-bit halves, as far as its bits are used; with v >> 24 = 8 z + r, the ordering is
+// 8 (z % 3) + r, and z % 3 (z < 2^37) comes from z's digits in base 2^16, each 1 mod 3: a small sum n whose
+// product with 1/3 mod 2^32 lies in the first, last or middle third for n % 3 = 0, 1, 2.
+KS_HD uint32_t permuted_digit(const DigitTable &t, uint32_t x)
+{
+    const uint64_t m1 = 0x7fb5d329728ea185ull, m2 = 0x81dadef4bc2dd44dull;
+    const uint32_t v0 = x ^ (x >> 31);
+    uint64_t p = (uint64_t)v0 * (uint32_t)m1;
+    uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32) + v0 * (uint32_t)(m1 >> 32);
+    lo ^= (lo >> 27) | (hi << 5); // v ^= v >> 27
+    hi ^= hi >> 27;
+    p = (uint64_t)lo * (uint32_t)m2;
+    hi = (uint32_t)(p >> 32) + lo * (uint32_t)(m2 >> 32) + hi * (uint32_t)m2;
+    lo = (uint32_t)p ^ (hi >> 1); // v ^= v >> 33
+    const uint32_t z = (lo >> 27) | (hi << 5), z_hi = hi >> 27;
+    const uint32_t n = (z & 0xffffu) + (z >> 16) + z_hi;
+    const uint32_t third = n * 0xaaaaaaabu;
+    const uint32_t w = third <= 0x55555555u ? t.w[0] : (third > 0xaaaaaaaau ? t.w[1] : t.w[2]);
+    return (w >> ((lo >> 23) & 14u)) & 3u;
 }
 
 struct SobolSampler
@@ -173,28 +184,41 @@ struct SobolSampler
     template <int N>
     KS_HD void sample_indices(const uint32_t (&dim_mix)[N], uint64_t (&out)[N]) const
     {
+        // up to 16 digits (1024 x 1024 at 4096 samples) an index has 32 bits
+        if (n_base4_digits <= 16)
+            permute<N, uint32_t>(dim_mix, out);
+        else
+            permute<N, uint64_t>(dim_mix, out);
+    }
+
+    template <int N, class Index>
+    KS_HD void permute(const uint32_t (&dim_mix)[N], uint64_t (&out)[N]) const
+    {
         const uint32_t m = (uint32_t)morton_index;
         const bool pow2 = (log2_spp & 1) != 0;
         const int last_digit = pow2 ? 1 : 0;
+        Index a[N];
 #pragma unroll
         for (int k = 0; k < N; ++k)
-            out[k] = 0;
+            a[k] = 0;
         for (int i = n_base4_digits - 1; i >= last_digit; --i) {
             int shift = 2 * i - (pow2 ? 1 : 0);
             uint32_t digit = shift >= 32 ? 0u : ((m >> shift) & 3u);
             uint32_t higher = shift + 2 >= 32 ? 0u : (m >> (shift + 2));
+            const DigitTable t = digit_table(digit);
 #pragma unroll
             for (int k = 0; k < N; ++k)
-                out[k] = (out[k] << 2) |
-                         (uint64_t)digit_permutation(digit_perm_index(higher ^ dim_mix[k]), (int)digit);
+                a[k] = (a[k] << 2) | (Index)permuted_digit(t, higher ^ dim_mix[k]);
         }
         if (pow2) {
             uint32_t digit = m & 1u;
 #pragma unroll
             for (int k = 0; k < N; ++k)
-                out[k] = (out[k] << 1) |
-                         (uint64_t)(digit ^ (uint32_t)(mix_bits64((uint64_t)((m >> 1) ^ dim_mix[k])) & 1u));
+                a[k] = (a[k] << 1) | (Index)(digit ^ (uint32_t)(mix_bits64((uint64_t)((m >> 1) ^ dim_mix[k])) & 1u));
         }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            out[k] = a[k];
     }
 
     KS_HD uint64_t sample_index() const
