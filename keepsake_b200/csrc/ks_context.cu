@@ -2,6 +2,10 @@
 #include "ks_internal.h"
 #include "ks_sampler.cuh"
 
+#include <algorithm>
+#include <thread>
+#include <cstring>
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <new>
@@ -56,6 +60,69 @@ DevicePool *pool_of(int device)
 } // namespace pool_detail
 using pool_detail::DevicePool;
 using pool_detail::pool_of;
+
+cudaError_t staged_copy(ks_context *ctx, void *dst, const void *src, size_t bytes, bool to_device)
+{
+    const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    cudaStream_t st = ctx->stream;
+    if (bytes < kStageMin || ctx->stage.reserve(std::min(bytes, kStageBytes)) != cudaSuccess) {
+        cudaGetLastError();
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
+    cudaEvent_t done[kStageChunks] = {};
+    cudaError_t err = cudaSuccess;
+    for (auto &ev : done)
+        if (err == cudaSuccess)
+            err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    char *stage = static_cast<char *>(ctx->stage.ptr);
+    for (size_t off = 0; off < bytes && err == cudaSuccess; off += ctx->stage.bytes) {
+        const size_t part = std::min(bytes - off, ctx->stage.bytes), piece = (part + kStageChunks - 1) / kStageChunks;
+        auto begin = [&](size_t k) { return std::min(part, k * piece); };
+        auto issue = [&](size_t k) { // piece k over the link
+            const size_t b = begin(k), n = begin(k + 1) - b;
+            cudaError_t e = n ? (to_device ? cudaMemcpyAsync(static_cast<char *>(dst) + off + b, stage + b, n, kind, st)
+                                           : cudaMemcpyAsync(stage + b, static_cast<const char *>(src) + off + b, n, kind, st))
+                              : cudaSuccess;
+            return e == cudaSuccess ? cudaEventRecord(done[k], st) : e;
+        };
+        if (to_device) {
+            for (size_t k = 0; k < kStageChunks && err == cudaSuccess; ++k) {
+                const size_t b = begin(k);
+                host_parallel(begin(k + 1) - b, (size_t)1 << 20, [&](size_t i, size_t e) {
+                    std::memcpy(stage + b + i, static_cast<const char *>(src) + off + b + i, e - i);
+                });
+                err = issue(k);
+            }
+            const cudaError_t e = cudaStreamSynchronize(st);
+            err = err == cudaSuccess ? e : err;
+            continue;
+        }
+        for (size_t k = 0; k < kStageChunks && err == cudaSuccess; ++k)
+            err = issue(k);
+        // every thread copies its share of each piece as the piece arrives; the caller's waits for it
+        std::atomic<size_t> ready{0};
+        host_parallel(part, (size_t)1 << 20, [&](size_t i, size_t e) {
+            for (size_t k = 0; k < kStageChunks; ++k) {
+                if (i == 0) {
+                    const cudaError_t w = err == cudaSuccess ? cudaEventSynchronize(done[k]) : err;
+                    err = err == cudaSuccess ? w : err;
+                    ready.store(k + 1, std::memory_order_release);
+                }
+                while (ready.load(std::memory_order_acquire) <= k)
+                    std::this_thread::yield();
+                const size_t b = begin(k), n = begin(k + 1) - b;
+                const size_t lo = (size_t)((double)n * ((double)i / (double)part)),
+                             hi = e == part ? n : (size_t)((double)n * ((double)e / (double)part));
+                std::memcpy(static_cast<char *>(dst) + off + b + lo, stage + b + lo, hi - lo);
+            }
+        });
+    }
+    for (auto &ev : done)
+        if (ev)
+            cudaEventDestroy(ev);
+    return err;
+}
 
 cudaError_t pool_alloc(void **ptr, size_t bytes)
 {

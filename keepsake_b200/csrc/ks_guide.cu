@@ -585,6 +585,7 @@ struct ks_guide
     DevBuf<__half2> grid_h; // FP16 copy of grid for inference, refreshed with w_image
     DevBuf<int> err;
     DevBuf<double> loss;
+    DevBuf<float> rows;     // ks_guide_infer's and ks_guide_gradients' rows, kept between calls (up to kRowsKept)
     int iter = 0;
     bool packed = false;
     int grid_ctas = 148;
@@ -902,9 +903,9 @@ ks_status ks_guide_get_weights(ks_guide *g, float *mlp_weights, float *grid)
         return KS_ERR_INVALID_ARGUMENT;
     KS_CUDA_TRY(g->ctx, enter_device(g->ctx));
     if (mlp_weights)
-        KS_CUDA_TRY(g->ctx, cudaMemcpy(mlp_weights, g->w.ptr, g->w.bytes(), cudaMemcpyDeviceToHost));
+        KS_CUDA_TRY(g->ctx, staged_copy(g->ctx, mlp_weights, g->w.ptr, g->w.bytes(), false));
     if (grid)
-        KS_CUDA_TRY(g->ctx, cudaMemcpy(grid, g->grid.ptr, g->grid.bytes(), cudaMemcpyDeviceToHost));
+        KS_CUDA_TRY(g->ctx, staged_copy(g->ctx, grid, g->grid.ptr, g->grid.bytes(), false));
     return KS_OK;
 }
 
@@ -914,11 +915,21 @@ ks_status ks_guide_set_weights(ks_guide *g, const float *mlp_weights, const floa
         return KS_ERR_INVALID_ARGUMENT;
     KS_CUDA_TRY(g->ctx, enter_device(g->ctx));
     if (mlp_weights)
-        KS_CUDA_TRY(g->ctx, cudaMemcpy(g->w.ptr, mlp_weights, g->w.bytes(), cudaMemcpyHostToDevice));
+        KS_CUDA_TRY(g->ctx, staged_copy(g->ctx, g->w.ptr, mlp_weights, g->w.bytes(), true));
     if (grid)
-        KS_CUDA_TRY(g->ctx, cudaMemcpy(g->grid.ptr, grid, g->grid.bytes(), cudaMemcpyHostToDevice));
+        KS_CUDA_TRY(g->ctx, staged_copy(g->ctx, g->grid.ptr, grid, g->grid.bytes(), true));
     g->packed = false;
     return KS_OK;
+}
+
+// Room for n floats: the guide's own buffer, or `own` when that would keep too much.
+static cudaError_t row_buffer(ks_guide *g, size_t n, DevBuf<float> &own, float **out)
+{
+    constexpr size_t kRowsKept = (size_t)64 << 20; // floats
+    DevBuf<float> &buf = n <= kRowsKept ? g->rows : own;
+    const cudaError_t e = buf.reserve(n);
+    *out = buf.ptr;
+    return e;
 }
 
 ks_status ks_guide_infer(ks_guide *g, const float *pos, const float *wo, const float *normal, uint32_t n,
@@ -930,19 +941,17 @@ ks_status ks_guide_infer(ks_guide *g, const float *pos, const float *wo, const f
     KS_CUDA_TRY(ctx, enter_device(ctx));
     if (n == 0)
         return KS_OK;
-    DevBuf<float> dp, dw, dn, dout;
-    KS_CUDA_TRY(ctx, dp.alloc(3 * (size_t)n));
-    KS_CUDA_TRY(ctx, dw.alloc(3 * (size_t)n));
-    KS_CUDA_TRY(ctx, dn.alloc(3 * (size_t)n));
-    KS_CUDA_TRY(ctx, dout.alloc((size_t)kOut * n));
-    cudaStream_t st = ctx->stream;
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dp.ptr, pos, dp.bytes(), cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dw.ptr, wo, dw.bytes(), cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dn.ptr, normal, dn.bytes(), cudaMemcpyHostToDevice, st));
-    ks_status s = run_mlp(g, false, n, dp.ptr, dw.ptr, dn.ptr, nullptr, nullptr, dout.ptr);
+    DevBuf<float> own;
+    float *d = nullptr;
+    const size_t r3 = 3 * (size_t)n;
+    KS_CUDA_TRY(ctx, row_buffer(g, 3 * r3 + (size_t)kOut * n, own, &d));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, d, pos, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, d + r3, wo, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, d + 2 * r3, normal, r3 * sizeof(float), true));
+    ks_status s = run_mlp(g, false, n, d, d + r3, d + 2 * r3, nullptr, nullptr, d + 3 * r3);
     if (s != KS_OK)
         return s;
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(raw_out, dout.ptr, dout.bytes(), cudaMemcpyDeviceToHost, st));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, raw_out, d + 3 * r3, sizeof(float) * (size_t)kOut * n, false));
     return check_err(g);
 }
 
@@ -955,23 +964,21 @@ ks_status ks_guide_gradients(ks_guide *g, const float *pos, const float *wo, con
     ks_context *ctx = g->ctx;
     KS_CUDA_TRY(ctx, enter_device(ctx));
     cudaStream_t st = ctx->stream;
-    DevBuf<float> dp, dwo, dn, dwi, dt, dpb;
-    KS_CUDA_TRY(ctx, dn.alloc(3 * (size_t)n + 3));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dn.ptr, normal, 12 * (size_t)n, cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, dp.alloc(3 * (size_t)n + 3));
-    KS_CUDA_TRY(ctx, dwo.alloc(3 * (size_t)n + 3));
-    KS_CUDA_TRY(ctx, dwi.alloc(3 * (size_t)n + 3));
-    KS_CUDA_TRY(ctx, dt.alloc((size_t)n + 1));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dp.ptr, pos, 12 * (size_t)n, cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dwo.ptr, wo, 12 * (size_t)n, cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dwi.ptr, wi, 12 * (size_t)n, cudaMemcpyHostToDevice, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(dt.ptr, target, 4 * (size_t)n, cudaMemcpyHostToDevice, st));
-    if (bsdf_pdf) {
-        KS_CUDA_TRY(ctx, dpb.alloc((size_t)n + 1));
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(dpb.ptr, bsdf_pdf, 4 * (size_t)n, cudaMemcpyHostToDevice, st));
-    }
+    DevBuf<float> own;
+    float *d = nullptr;
+    const size_t r3 = 3 * (size_t)n;
+    KS_CUDA_TRY(ctx, row_buffer(g, 4 * r3 + 2 * (size_t)n + 1, own, &d));
+    float *dp = d, *dwo = d + r3, *dn = d + 2 * r3, *dwi = d + 3 * r3, *dt = d + 4 * r3;
+    float *dpb = bsdf_pdf ? dt + n : nullptr;
+    KS_CUDA_TRY(ctx, staged_copy(ctx, dn, normal, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, dp, pos, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, dwo, wo, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, dwi, wi, r3 * sizeof(float), true));
+    KS_CUDA_TRY(ctx, staged_copy(ctx, dt, target, n * sizeof(float), true));
+    if (bsdf_pdf)
+        KS_CUDA_TRY(ctx, staged_copy(ctx, dpb, bsdf_pdf, n * sizeof(float), true));
     KS_CUDA_TRY(ctx, cudaMemsetAsync(g->loss.ptr, 0, sizeof(double), st));
-    ks_status s = run_mlp(g, true, n, dp.ptr, dwo.ptr, dn.ptr, dwi.ptr, dt.ptr, nullptr, 3, dpb.ptr, 1);
+    ks_status s = run_mlp(g, true, n, dp, dwo, dn, dwi, dt, nullptr, 3, dpb, 1);
     if (s != KS_OK)
         return s;
     if (loss)
@@ -979,8 +986,7 @@ ks_status ks_guide_gradients(ks_guide *g, const float *pos, const float *wo, con
     if (mlp_grad)
         KS_CUDA_TRY(ctx, cudaMemcpyAsync(mlp_grad, g->w_grad.ptr, g->w_grad.bytes(), cudaMemcpyDeviceToHost, st));
     if (grid_grad)
-        KS_CUDA_TRY(ctx,
-                    cudaMemcpyAsync(grid_grad, g->grid_grad.ptr, g->grid_grad.bytes(), cudaMemcpyDeviceToHost, st));
+        KS_CUDA_TRY(ctx, staged_copy(ctx, grid_grad, g->grid_grad.ptr, g->grid_grad.bytes(), false));
     s = check_err(g);
     if (s != KS_OK)
         return s;

@@ -58,6 +58,8 @@ struct ks_context
     ks_context_limits limits{};
     // host side of ks_scene_create's uploads
     KsPinned upload;
+    // host side of staged_copy (at most kStageBytes)
+    KsPinned stage;
 };
 
 namespace ksb
@@ -93,6 +95,14 @@ void host_parallel(size_t n, size_t grain, F &&f)
     for (auto &t : pool)
         t.join();
 }
+
+// Copies between the caller's (pageable) host memory and the device on the context's stream, through pinned
+// memory the context keeps, in kStageChunks pieces so that the link and the host threads' copies overlap;
+// the call returns when host memory is done with (a download: filled; an upload: read).  Small copies go
+// straight.  Pageable copies of 64 MB into new memory took the driver some 11 ms: one thread copying from its
+// own staging while it meets a page fault every 4 KB.
+constexpr size_t kStageBytes = (size_t)64 << 20, kStageChunks = 8, kStageMin = (size_t)1 << 20;
+cudaError_t staged_copy(ks_context *ctx, void *dst, const void *src, size_t bytes, bool to_device);
 
 // Records a failure on the context and returns its status.
 inline ks_status fail(ks_context *ctx, ks_status s, const std::string &msg)
