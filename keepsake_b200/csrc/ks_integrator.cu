@@ -4,7 +4,9 @@
 //
 //   raygen  -> new camera paths fill the free queue slots (sample-major over the crop window),
 //   extend  -> closest-hit traversal of the SBVH's 4-wide view by persistent warps that fetch rays
-//              from a counter (ks_traverse.cuh), then hit and miss queues in path order,
+//              from a counter (ks_traverse4.cuh; instanced scenes and trees too deep for the view:
+//              ks_traverse.cuh), short queues by groups of 4 lanes per ray; then hit and miss queues
+//              in path order,
 //   sample  -> the bounce's Sobol values and the NEE light sample (ks_shade.cu),
 //   shade   -> miss/sky MIS, emitter MIS, BSDF eval of the light sample (Material::sample_with_nee,
 //              material.cpp:101-167; next_event_estimate, nee.cpp:11-57), BSDF sample, Russian
@@ -213,6 +215,16 @@ KS_D void flush_counts(const TravCount &c, unsigned long long *dst)
     }
 }
 
+// Paths of an iteration: the host's number, or the device's (the last iteration's count of continuing paths;
+// batches: their state).
+template <bool kBatch>
+KS_D uint32_t queue_size(uint32_t count, const uint32_t *count_ptr, const BatchView &bv)
+{
+    if constexpr (kBatch)
+        return bv.state->count;
+    return count_ptr ? *count_ptr : count;
+}
+
 // The extension ray of path slot i.
 KS_D RayQuery path_ray(const PathBuf &pb, uint32_t i)
 {
@@ -245,16 +257,16 @@ KS_D float4 hit_record(const Hit &h, bool retrace = false)
 // order.  kBatch: paths of many jobs, the count read from the batch state.
 // kAlpha: the scene has opacity maps; candidate hits go through their stochastic test (SceneAlpha).
 // kDeep: the tree (of some job) is too deep for the 4-wide view.
+// count_ptr: where the count lies on the device when the host does not know it yet (else null); choose: the
+// group kernel was launched too, and short queues are its.
 template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
 __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
-                                                   float4 *hits, uint32_t *fetch, int *overflow,
-                                                   unsigned long long *work, BatchView bv)
+                                                   const uint32_t *count_ptr, int choose, float4 *hits, uint32_t *fetch,
+                                                   int *overflow, unsigned long long *work, BatchView bv)
 {
-    if constexpr (kBatch) {
-        count = bv.state->count;
-        if (!kDeep && count <= KS_GROUP_RAYS)
-            return; // k_extend_group's
-    }
+    count = queue_size<kBatch>(count, count_ptr, bv);
+    if (!kDeep && choose && count <= KS_GROUP_RAYS)
+        return; // k_extend_group's
     TravCount tc;
     KS_TRAV_STACK(stack);
     using View = TreeOf<kDeep>;
@@ -308,13 +320,12 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
 // the warps of an SM ran all BSDF kinds at once and waited for instructions 28 of 45 cycles.
 template <bool kBatch = false, bool kSplit = false>
 __global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__ SceneView sv_in, PathBuf pb, float4 *hits,
-                                                      uint32_t count, uint32_t *hit_queue,
+                                                      uint32_t count, const uint32_t *count_ptr, uint32_t *hit_queue,
                                                       uint32_t *miss_queue, uint32_t *queue_counts, int *overflow,
                                                       int alpha, uint32_t *split_queue, uint32_t split_cap,
                                                       uint32_t *split_counts, BatchView bv)
 {
-    if constexpr (kBatch)
-        count = bv.state->count;
+    count = queue_size<kBatch>(count, count_ptr, bv);
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t *slots = reinterpret_cast<const uint32_t *>(hits) + 3;
     for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
@@ -404,12 +415,12 @@ KS_D RayQuery shadow_ray(const ShadowBuf &sb, uint32_t i)
 // finished by shadow_done as soon as its traversal ends.
 template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
 __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const __grid_constant__ SceneView sv_in, ShadowBuf sb,
-                                                   const uint32_t *shadow_count, uint32_t *fetch, PathBuf nxt,
+                                                   const uint32_t *shadow_count, int choose, uint32_t *fetch, PathBuf nxt,
                                                    double *accum_in, double *weights_in, int *overflow,
                                                    unsigned long long *work, GuideView gv, BatchView bv)
 {
     const uint32_t count = *shadow_count;
-    if (kBatch && !kDeep && count <= KS_GROUP_RAYS)
+    if (!kDeep && choose && count <= KS_GROUP_RAYS)
         return; // k_shadow_group's
     TravCount tc;
     KS_TRAV_STACK(stack);
@@ -467,18 +478,15 @@ KS_D uint32_t group_first_ray()
     return ((threadIdx.x & 31u) / kGroup) * warps + warp;
 }
 
-// kBatch: paths of many jobs; the count is the device's, and so is the choice between these kernels and the
-// persistent ones (both are launched, one returns).
+// kBatch: paths of many jobs.  choose: the persistent kernel was launched too, and takes longer queues.
 template <bool kBatch = false, bool kAlpha = false>
 __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_extend_group(
-    const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count, float4 *hits, unsigned long long *work,
-    BatchView bv)
+    const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count, const uint32_t *count_ptr, int choose,
+    float4 *hits, unsigned long long *work, BatchView bv)
 {
-    if constexpr (kBatch) {
-        count = bv.state->count;
-        if (count > KS_GROUP_RAYS)
-            return;
-    }
+    count = queue_size<kBatch>(count, count_ptr, bv);
+    if (choose && count > KS_GROUP_RAYS)
+        return;
     TravCount tc;
     KS_GROUP_STACK(stack);
     const uint32_t mask = ((1u << kGroup) - 1u) << (threadIdx.x & 31u & ~(kGroup - 1u));
@@ -501,11 +509,11 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_extend_grou
 
 template <bool kBatch = false, bool kAlpha = false>
 __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_shadow_group(
-    const __grid_constant__ SceneView sv_in, ShadowBuf sb, const uint32_t *shadow_count, PathBuf nxt, double *accum,
-    double *weights, unsigned long long *work, GuideView gv, BatchView bv)
+    const __grid_constant__ SceneView sv_in, ShadowBuf sb, const uint32_t *shadow_count, int choose, PathBuf nxt,
+    double *accum, double *weights, unsigned long long *work, GuideView gv, BatchView bv)
 {
     const uint32_t count = *shadow_count;
-    if (kBatch && count > KS_GROUP_RAYS)
+    if (choose && count > KS_GROUP_RAYS)
         return;
     TravCount tc;
     KS_GROUP_STACK(stack);
@@ -534,9 +542,10 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_shadow_grou
 // The same warp-level ray fetch as k_extend_pt / k_shadow_pt over inst_step (ks_traverse.cuh):
 // each ray makes the tests of traverse_instances, in resumable steps.
 __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_extend_inst_pt(const __grid_constant__ SceneView sv, PathBuf pb,
-                                                        uint32_t count, float4 *hits, uint32_t *hit_inst,
+                                                        uint32_t count, const uint32_t *count_ptr, float4 *hits, uint32_t *hit_inst,
                                                         uint32_t *fetch, int *overflow, unsigned long long *work)
 {
+    count = queue_size<false>(count, count_ptr, BatchView{});
     TravCount tc;
     KS_TRAV_STACK(stack);
     InstTravState s;
@@ -957,7 +966,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     KS_CUDA_TRY(ctx, w.queue[1].reserve(w.capacity));
     for (int f = 0; f < 4; ++f)
         KS_CUDA_TRY(ctx, w.shadow[f].reserve(w.capacity));
-    KS_CUDA_TRY(ctx, w.counters.reserve(kCounters));
+    KS_CUDA_TRY(ctx, w.counters.reserve(2 * kCounters));
     KS_CUDA_TRY(ctx, w.overflow.reserve(1));
     DevBuf<unsigned long long> work; // ext nodes, ext tris, shadow nodes, shadow tris
     KS_CUDA_TRY(ctx, work.alloc(4));
@@ -1012,25 +1021,41 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     // kept with the wavefront buffers: a pinned allocation and free per render cost milliseconds,
     // now and then far more
     if (!w.h_counts)
-        KS_CUDA_TRY(ctx, cudaMallocHost((void **)&w.h_counts, sizeof(uint32_t) * 4));
-    uint32_t *h_counts = w.h_counts;
-    h_counts[2] = 0;
+        KS_CUDA_TRY(ctx, cudaMallocHost((void **)&w.h_counts, sizeof(uint32_t) * 8));
     // guided renders: the guide's filter and inference run on a second stream, overlapping the
     // sampling and the miss shading, and join before the hit shading
     cudaStream_t aux = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_g0 = nullptr, ev_g1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     if (guide) {
         if (!rc.aux)
             KS_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&rc.aux, cudaStreamNonBlocking));
         aux = rc.aux;
         cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming);
-        cudaEventCreate(&ev_g0);
-        cudaEventCreate(&ev_g1);
     }
-    cudaEvent_t ev[6];
-    for (auto &e : ev)
-        cudaEventCreate(&e);
+    // Two iterations are in flight once all paths are issued: the next one is launched, its count still on the
+    // device, before the host has read the last one's.  The host's round trip left the GPU idle for about 30 us an
+    // iteration; without it a 64x48 thumbnail takes 0.94 -> 0.81 ms, a 641x359 preview 2.24 -> 1.94 and a 1024x1024 frame
+    // of 64 samples 83.3 -> 82.2.  While paths are still issued the host has to know the free slots, so those
+    // iterations are read one by one.
+    struct Flight
+    {
+        cudaEvent_t ev[6] = {}, g0 = nullptr, g1 = nullptr, done = nullptr;
+        uint32_t *counters = nullptr, *h_counts = nullptr; // device and pinned: next paths, shadow rays, guide rows
+        uint32_t bound = 0;                                // its paths, or more
+        int cur = 0;                                       // its path buffer
+    } flights[2];
+    for (int k = 0; k < 2; ++k) {
+        for (auto &e : flights[k].ev)
+            cudaEventCreate(&e);
+        cudaEventCreateWithFlags(&flights[k].done, cudaEventDisableTiming);
+        if (guide) {
+            cudaEventCreate(&flights[k].g0);
+            cudaEventCreate(&flights[k].g1);
+        }
+        flights[k].counters = w.counters.ptr + k * kCounters;
+        flights[k].h_counts = w.h_counts + 4 * k;
+    }
     cudaEvent_t t_begin, t_end;
     cudaEventCreate(&t_begin);
     cudaEventCreate(&t_end);
@@ -1068,130 +1093,177 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
         uint64_t watchdog = (total / w.capacity + 2) * (uint64_t)(in->bounces + 2) + 64;
         if (ctx->limits.wavefront_max_iterations)
             watchdog = std::min<uint64_t>(watchdog, ctx->limits.wavefront_max_iterations);
-        uint64_t it_interval = 0;
-        while ((issued < total || cur_count > 0) && err == cudaSuccess) {
-            if (++it_interval > watchdog) {
-                err = cudaErrorUnknown;
-                stats.iterations = 0xffffffffu;
-                break;
-            }
-            uint32_t n_new = (uint32_t)std::min<uint64_t>(w.capacity - cur_count, total - issued);
-            cudaEventRecord(ev[0], st);
+        uint64_t it_interval = 0, last_issue = 0;
+        const bool guiding = guide && gv.active;
+        // One iteration: the first n_old paths of its buffer (or as many as *count_ptr says, at most n_old) and
+        // n_new camera paths behind them.
+        auto launch = [&](Flight &f, uint32_t n_old, uint32_t n_new, const uint32_t *count_ptr) {
+            uint32_t *cnt = f.counters;
+            const uint32_t count = n_old + n_new;
+            f.bound = count;
+            cudaEventRecord(f.ev[0], st);
             if (n_new) {
-                k_raygen<<<(n_new + 255) / 256, 256, 0, st>>>(rp, pb[cur], cur_count, issued, n_new, s0, n_pix);
+                k_raygen<<<(n_new + 255) / 256, 256, 0, st>>>(rp, pb[f.cur], n_old, issued, n_new, s0, n_pix);
                 stats.kernel_launches++;
             }
-            issued += n_new;
-            uint32_t count = cur_count + n_new;
-            stats.extension_rays += count;
-            // counters: [0] next paths, [1] shadow rays, [2] hit queue, [3] miss queue, [4], [5] ray fetch
-            cudaMemsetAsync(w.counters.ptr, 0, sizeof(uint32_t) * kCounters, st);
-            unsigned grid = std::min<unsigned>((count + 127) / 128, max_grid);
-            const bool grouped = !scene->n_instances && !scene->deep && count <= KS_GROUP_RAYS;
+            cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * kCounters, st);
+            const unsigned grid = std::min<unsigned>((count + 127) / 128, max_grid);
+            // groups of lanes for short queues; where the count is not known to be short, or long, both kernels
+            // are launched and choose
+            const bool can_group = !scene->n_instances && !scene->deep;
+            const bool short_queue = can_group && count <= KS_GROUP_RAYS;
+            const bool ext_choose = can_group && !short_queue && count_ptr && count <= 16 * KS_GROUP_RAYS;
+            const bool shadow_choose = can_group && !short_queue && count <= 16 * KS_GROUP_RAYS;
             const unsigned group_grid = std::min<unsigned>((count + 3) / 4, ext_group_grid);
-            cudaEventRecord(ev[1], st);
+            cudaEventRecord(f.ev[1], st);
             if (scene->n_instances)
-                k_extend_inst_pt<<<std::min(grid, ext_grid), 128, 0, st>>>(
-                    sv, pb[cur], count, w.hits.ptr, w.hit_inst.ptr, w.counters.ptr + 4, w.overflow.ptr, work.ptr);
-            else if (grouped)
-                ext_group<<<group_grid, kTravBlock, 0, st>>>(sv, pb[cur], count, w.hits.ptr, work.ptr, BatchView{});
-            else
-                ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[cur], count, w.hits.ptr, w.counters.ptr + 4,
-                                                                     w.overflow.ptr, work.ptr, BatchView{});
+                k_extend_inst_pt<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[f.cur], count, count_ptr, w.hits.ptr,
+                                                                           w.hit_inst.ptr, cnt + 4, w.overflow.ptr,
+                                                                           work.ptr);
+            else if (!short_queue)
+                ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[f.cur], count, count_ptr, ext_choose,
+                                                                     w.hits.ptr, cnt + 4, w.overflow.ptr, work.ptr,
+                                                                     BatchView{});
+            if (short_queue || ext_choose)
+                ext_group<<<group_grid, kTravBlock, 0, st>>>(sv, pb[f.cur], count, count_ptr, ext_choose, w.hits.ptr,
+                                                             work.ptr, BatchView{});
             (split ? k_build_queues<false, true> : k_build_queues<false>)<<<std::min((count + 255) / 256, max_grid), 256, 0,
                                                                              st>>>(
-                sv, pb[cur], w.hits.ptr, count, w.queue[0].ptr, w.queue[1].ptr, w.counters.ptr + 2, w.overflow.ptr, alpha,
-                w.split.ptr, w.capacity, w.counters.ptr + 8, BatchView{});
+                sv, pb[f.cur], w.hits.ptr, count, count_ptr, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, alpha,
+                w.split.ptr, w.capacity, cnt + 8, BatchView{});
             stats.kernel_launches++;
-            cudaEventRecord(ev[2], st);
-            const bool guiding = guide && gv.active;
+            cudaEventRecord(f.ev[2], st);
             if (guiding) {
                 // the guide only at vertices that sample a direction with a rough enough BSDF
                 cudaEventRecord(ev_fork, st);
                 cudaStreamWaitEvent(aux, ev_fork, 0);
-                cudaEventRecord(ev_g0, aux);
+                cudaEventRecord(f.g0, aux);
                 cudaMemsetAsync(gw.gcount.ptr, 0, sizeof(uint32_t), aux);
                 k_guide_filter<<<grid, 128, 0, aux>>>(sv, std::min<int>(rp.bounces, (int)gv.rec_bounces),
-                                                      gv.min_roughness, pb[cur], w.hits.ptr,
-                                                      w.queue[0].ptr, w.counters.ptr + 2, gw.gqueue.ptr,
-                                                      gw.gcount.ptr, gw.lobes.ptr, w.capacity);
+                                                      gv.min_roughness, pb[f.cur], w.hits.ptr, w.queue[0].ptr, cnt + 2,
+                                                      gw.gqueue.ptr, gw.gcount.ptr, gw.lobes.ptr, w.capacity);
                 stats.kernel_launches++;
-                ks_status gs = guide_impl::infer_paths(guide, gw.gqueue.ptr, gw.gcount.ptr, pb[cur].o_pdf,
-                                                       pb[cur].d_info, w.hits.ptr, sv.prim_tris, w.hit_inst.ptr,
+                ks_status gs = guide_impl::infer_paths(guide, gw.gqueue.ptr, gw.gcount.ptr, pb[f.cur].o_pdf,
+                                                       pb[f.cur].d_info, w.hits.ptr, sv.prim_tris, w.hit_inst.ptr,
                                                        sv.inst.xf, gw.lobes.ptr, w.capacity, count, aux);
-                cudaEventRecord(ev_g1, aux);
+                cudaEventRecord(f.g1, aux);
                 cudaEventRecord(ev_join, aux);
                 if (gs != KS_OK) {
                     cudaStreamWaitEvent(st, ev_join, 0);
                     err = cudaErrorLaunchFailure;
-                    break;
+                    return;
                 }
                 stats.kernel_launches++;
             }
-            cudaEventRecord(ev[5], st);
+            cudaEventRecord(f.ev[5], st);
             if (scene->any_subsurface) {
-                launch_subsurface(grid, (unsigned)ctx->sm_count, st, sv, rp, pb[cur], w.hits.ptr, w.queue[0].ptr,
-                                  w.counters.ptr + 2, w.walks.ptr, w.counters.ptr + 6, w.overflow.ptr);
+                launch_subsurface(grid, (unsigned)ctx->sm_count, st, sv, rp, pb[f.cur], w.hits.ptr, w.queue[0].ptr, cnt + 2,
+                                  w.walks.ptr, cnt + 6, w.overflow.ptr);
                 stats.kernel_launches += 2;
             }
-            launch_sample(false, grid, st, sv, rp, pb[cur], w.hits.ptr, w.hit_inst.ptr, w.queue[0].ptr,
-                          w.counters.ptr + 2, w.samples.ptr, BatchView{});
+            launch_sample(false, grid, st, sv, rp, pb[f.cur], w.hits.ptr, w.hit_inst.ptr, w.queue[0].ptr, cnt + 2,
+                          w.samples.ptr, BatchView{});
             // misses first (they do not read the guide), then the hits once the guide has joined
             auto shade = [&](bool miss, int kernel_variant, const uint32_t *queue, const uint32_t *n) {
-                launch_shade(miss, guide != nullptr, false, kernel_variant, grid, st, sv, rp, pb[cur], pb[1 - cur],
-                             w.hits.ptr, w.hit_inst.ptr, w.samples.ptr, queue, n, w.counters.ptr, sb, w.counters.ptr + 1,
-                             d_accum, d_weights, gv, BatchView{});
+                launch_shade(miss, guide != nullptr, false, kernel_variant, grid, st, sv, rp, pb[f.cur], pb[1 - f.cur],
+                             w.hits.ptr, w.hit_inst.ptr, w.samples.ptr, queue, n, cnt, sb, cnt + 1, d_accum, d_weights, gv,
+                             BatchView{});
             };
-            shade(true, variant, w.queue[1].ptr, w.counters.ptr + 3);
+            shade(true, variant, w.queue[1].ptr, cnt + 3);
             if (guiding)
                 cudaStreamWaitEvent(st, ev_join, 0);
             if (split) {
-                shade(false, sv.simple_variant, w.split.ptr, w.counters.ptr + 8);
-                shade(false, variant, w.split.ptr + w.capacity, w.counters.ptr + 9);
+                shade(false, sv.simple_variant, w.split.ptr, cnt + 8);
+                shade(false, variant, w.split.ptr + w.capacity, cnt + 9);
                 stats.kernel_launches++;
             } else {
-                shade(false, variant, w.queue[0].ptr, w.counters.ptr + 2);
+                shade(false, variant, w.queue[0].ptr, cnt + 2);
             }
-            cudaEventRecord(ev[3], st);
+            cudaEventRecord(f.ev[3], st);
             if (scene->n_instances)
                 k_shadow_inst_pt<<<std::min(grid, shadow_grid), 128, 0, st>>>(
-                    sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
-                    work.ptr + 2, gv);
-            else if (grouped)
-                shadow_group<<<group_grid, kTravBlock, 0, st>>>(sv, sb, w.counters.ptr + 1, pb[1 - cur], d_accum,
+                    sv, sb, cnt + 1, cnt + 5, pb[1 - f.cur], d_accum, d_weights, w.overflow.ptr, work.ptr + 2, gv);
+            else if (!short_queue)
+                shadow_kernel<<<std::min(grid, shadow_grid), 128, 0, st>>>(sv, sb, cnt + 1, shadow_choose, cnt + 5,
+                                                                           pb[1 - f.cur], d_accum, d_weights,
+                                                                           w.overflow.ptr, work.ptr + 2, gv, BatchView{});
+            if (short_queue || shadow_choose)
+                shadow_group<<<group_grid, kTravBlock, 0, st>>>(sv, sb, cnt + 1, shadow_choose, pb[1 - f.cur], d_accum,
                                                                 d_weights, work.ptr + 2, gv, BatchView{});
-            else
-                shadow_kernel<<<std::min(grid, shadow_grid), 128, 0, st>>>(
-                    sv, sb, w.counters.ptr + 1, w.counters.ptr + 5, pb[1 - cur], d_accum, d_weights, w.overflow.ptr,
-                    work.ptr + 2, gv, BatchView{});
-            cudaEventRecord(ev[4], st);
-            stats.kernel_launches += 5;
-            cudaMemcpyAsync(h_counts, w.counters.ptr, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost, st);
-            if (guide && gv.active)
-                cudaMemcpyAsync(h_counts + 2, gw.gcount.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-            err = cudaStreamSynchronize(st);
-            if (err != cudaSuccess)
-                break;
+            stats.kernel_launches += 5u + ext_choose + shadow_choose;
+            cudaEventRecord(f.ev[4], st);
+            cudaMemcpyAsync(f.h_counts, cnt, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost, st);
+            if (guiding)
+                cudaMemcpyAsync(f.h_counts + 2, gw.gcount.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+            cudaEventRecord(f.done, st);
             err = cudaGetLastError();
+        };
+        // Waits for an iteration and books it.
+        auto finish = [&](Flight &f) {
+            err = cudaEventSynchronize(f.done);
+            if (err != cudaSuccess)
+                return;
             float ms;
-            cudaEventElapsedTime(&ms, ev[0], ev[1]);
+            cudaEventElapsedTime(&ms, f.ev[0], f.ev[1]);
             stats.ms_shade += ms;
-            cudaEventElapsedTime(&ms, ev[1], ev[2]);
+            cudaEventElapsedTime(&ms, f.ev[1], f.ev[2]);
             stats.ms_extend += ms;
             if (guiding) {
-                cudaEventElapsedTime(&ms, ev_g0, ev_g1);
+                cudaEventElapsedTime(&ms, f.g0, f.g1);
                 stats.ms_guide_infer += ms;
+                stats.guide_rows += f.h_counts[2];
             }
-            cudaEventElapsedTime(&ms, ev[5], ev[3]);
+            cudaEventElapsedTime(&ms, f.ev[5], f.ev[3]);
             stats.ms_shade += ms;
-            cudaEventElapsedTime(&ms, ev[3], ev[4]);
+            cudaEventElapsedTime(&ms, f.ev[3], f.ev[4]);
             stats.ms_shadow += ms;
-            stats.shadow_rays += h_counts[1];
-            if (guide && gv.active)
-                stats.guide_rows += h_counts[2];
+            stats.shadow_rays += f.h_counts[1];
             stats.iterations++;
-            cur_count = h_counts[0];
-            cur = 1 - cur;
+        };
+        Flight *pending = nullptr;
+        while (err == cudaSuccess) {
+            if (!pending) {
+                if (issued >= total && cur_count == 0)
+                    break;
+                if (++it_interval > watchdog) {
+                    err = cudaErrorUnknown;
+                    stats.iterations = 0xffffffffu;
+                    break;
+                }
+                const uint32_t n_new = (uint32_t)std::min<uint64_t>(w.capacity - cur_count, total - issued);
+                pending = &flights[cur];
+                pending->cur = cur;
+                launch(*pending, cur_count, n_new, nullptr);
+                if (n_new)
+                    last_issue = it_interval;
+                issued += n_new;
+                stats.extension_rays += cur_count + n_new;
+                cur = 1 - cur;
+            }
+            if (err != cudaSuccess)
+                break;
+            // a path takes at most bounces + 1 iterations: after those nothing is left to run ahead for
+            const bool ahead = issued == total && it_interval < watchdog &&
+                               it_interval - last_issue < (uint64_t)in->bounces;
+            Flight &next = flights[cur];
+            if (ahead) {
+                next.cur = cur;
+                launch(next, pending->bound, 0, pending->counters);
+                if (err != cudaSuccess)
+                    break;
+            }
+            finish(*pending);
+            if (err != cudaSuccess)
+                break;
+            cur_count = pending->h_counts[0];
+            pending = nullptr;
+            if (ahead && cur_count > 0) { // else the one launched ahead has no paths: nothing of it counts
+                ++it_interval;
+                next.bound = cur_count;
+                stats.extension_rays += cur_count;
+                pending = &next;
+                cur = 1 - cur;
+            }
         }
         stats.paths += total;
         if (err == cudaSuccess && recording) {
@@ -1204,20 +1276,20 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                 break;
             n_rec = std::min(n_rec, go.max_records);
             stats.guide_records += n_rec;
-            cudaEventRecord(ev[0], st);
+            cudaEventRecord(flights[0].ev[0], st);
             ks_status gs = guide_impl::train_rows(guide, n_rec, gw.rec_f4[0].ptr, gw.rec_f4[1].ptr, gw.rec_f4[4].ptr,
                                                   gw.rec_f4[2].ptr, gw.rec_t.ptr, go.train_batch,
                                                   &stats.guide_train_steps);
-            cudaEventRecord(ev[1], st);
+            cudaEventRecord(flights[0].ev[1], st);
             if (gs != KS_OK) {
                 err = cudaErrorLaunchFailure;
                 break;
             }
             err = cudaMemsetAsync(gw.rec_count.ptr, 0, sizeof(uint32_t), st);
             if (err == cudaSuccess)
-                err = cudaEventSynchronize(ev[1]);
+                err = cudaEventSynchronize(flights[0].ev[1]);
             float ms = 0.0f;
-            cudaEventElapsedTime(&ms, ev[0], ev[1]);
+            cudaEventElapsedTime(&ms, flights[0].ev[0], flights[0].ev[1]);
             stats.ms_guide_train += ms;
         }
         if (err == cudaSuccess && dcb) {
@@ -1247,9 +1319,14 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     cudaEventRecord(t_end, st);
     cudaEventSynchronize(t_end);
     cudaEventElapsedTime(&stats.ms_total, t_begin, t_end);
-    for (auto &e : ev)
-        cudaEventDestroy(e);
-    for (cudaEvent_t e : {ev_fork, ev_join, ev_g0, ev_g1})
+    for (Flight &f : flights) {
+        for (cudaEvent_t e : f.ev)
+            cudaEventDestroy(e);
+        for (cudaEvent_t e : {f.g0, f.g1, f.done})
+            if (e)
+                cudaEventDestroy(e);
+    }
+    for (cudaEvent_t e : {ev_fork, ev_join})
         if (e)
             cudaEventDestroy(e);
     cudaEventDestroy(t_begin);
@@ -1389,13 +1466,14 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     k_raygen_batch<<<(unsigned)ctx->sm_count * 8, 256, 0, st>>>(bv, pb[cur]);
     const auto ext_kernel = w.deep ? k_extend_pt<true, false, true> : k_extend_pt<true>;
     const auto shadow_kernel = w.deep ? k_shadow_pt<true, false, true> : k_shadow_pt<true>;
-    ext_kernel<<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, cnt + 4, w.overflow.ptr,
-                                                w.work.ptr, bv);
+    ext_kernel<<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, nullptr, 1, w.hits.ptr, cnt + 4, w.overflow.ptr,
+                                           w.work.ptr, bv);
     if (!w.deep)
-        k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, w.hits.ptr, w.work.ptr, bv);
+        k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, nullptr, 1, w.hits.ptr,
+                                                                  w.work.ptr, bv);
     const bool split = w.split.ptr != nullptr;
     (split ? k_build_queues<true, true> : k_build_queues<true>)<<<grid, 256, 0, st>>>(
-        SceneView{}, pb[cur], w.hits.ptr, 0u, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, w.split.ptr,
+        SceneView{}, pb[cur], w.hits.ptr, 0u, nullptr, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, w.split.ptr,
         capacity, cnt + 8, bv);
     launch_sample(true, grid, st, SceneView{}, RenderParams{}, pb[cur], w.hits.ptr, nullptr, w.queue[0].ptr, cnt + 2,
                   w.samples.ptr, bv);
@@ -1410,10 +1488,10 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
         shade(false, w.variant, w.queue[0].ptr, cnt + 2);
     }
     shade(true, w.variant, w.queue[1].ptr, cnt + 3);
-    shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
-                                                   w.overflow.ptr, w.work.ptr + 2, gv, bv);
+    shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
+                                                 w.overflow.ptr, w.work.ptr + 2, gv, bv);
     if (!w.deep)
-        k_shadow_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, sb, cnt + 1, pb[1 - cur], nullptr, nullptr,
+        k_shadow_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, sb, cnt + 1, 1, pb[1 - cur], nullptr, nullptr,
                                                                   w.work.ptr + 2, gv, bv);
     k_batch_advance<<<1, 32, 0, st>>>(bv.state, cnt, handle, use_graph);
 }
