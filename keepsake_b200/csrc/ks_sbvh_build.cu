@@ -30,7 +30,15 @@ namespace
 {
 
 constexpr int kMaxBuckets = 16;
-constexpr uint32_t kChunk = 1024; // references per work item (one warp each)
+// References per work item (one warp each).  The serial steps of a warp, not the bandwidth, bound the upper levels'
+// kernels.  Builds of 82 K, 328 K and 1.3 M triangles: items of 1024 4.1, 5.4 and 10.3 ms, 512 3.5, 4.6 and 9.7, 256 3.3,
+// 4.5 and 9.65, 128 3.1, 4.5 and 10.3 (more atomics on the nodes' tables).
+#ifndef KS_BUILD_CHUNK
+#define KS_BUILD_CHUNK 256
+#endif
+constexpr uint32_t kChunk = KS_BUILD_CHUNK;
+constexpr int kEvalLanes = 16; // lanes that evaluate a node's splits, one each
+static_assert(kMaxBuckets <= kEvalLanes, "a lane per split");
 constexpr int kWarpsPerBlock = 8;
 
 enum NodeKind : int
@@ -201,56 +209,41 @@ __global__ void k_init_refs(const float *verts, const uint32_t *idx, uint32_t tr
     refs[i].hi = make_float4(b[3], b[4], b[5], 0.0f);
 }
 
-__global__ void k_item_counts(const LevelNode *nodes, uint32_t n, uint32_t *counts)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        counts[i] = (nodes[i].ref_count + kChunk - 1) / kChunk;
-}
+KS_D uint32_t item_count(uint32_t refs) { return (refs + kChunk - 1) / kChunk; }
 
-__global__ void k_items_fill(LevelNode *nodes, uint32_t n, const uint32_t *item_off, Item *items)
+// The work items of every node, and its accumulators' start: kEvalLanes lanes a node.
+__global__ void k_items_fill(LevelNode *nodes, uint32_t n, const uint32_t *item_off, Item *items, uint32_t *bnd,
+                             uint32_t *obj, uint32_t *sp, NodeInfo *info, uint32_t buckets)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kEvalLanes, lane = threadIdx.x % kEvalLanes;
     if (i >= n)
         return;
-    LevelNode nd = nodes[i];
-    uint32_t first = item_off[i], cnt = item_off[i + 1] - first;
-    nodes[i].first_item = first;
-    for (uint32_t k = 0; k < cnt; ++k) {
+    const uint32_t ref_begin = nodes[i].ref_begin, ref_count = nodes[i].ref_count;
+    const uint32_t first = item_off[i], cnt = item_off[i + 1] - first;
+    for (uint32_t k = lane; k < cnt; k += kEvalLanes) {
         Item it;
         it.node = i;
-        it.begin = nd.ref_begin + k * kChunk;
-        uint32_t rem = nd.ref_count - k * kChunk;
+        it.begin = ref_begin + k * kChunk;
+        uint32_t rem = ref_count - k * kChunk;
         it.count = rem < kChunk ? rem : kChunk;
         it.single = cnt == 1;
         items[first + k] = it;
     }
-}
-
-__global__ void k_acc_init(const LevelNode *nodes, uint32_t *bnd, uint32_t *obj, uint32_t *sp, NodeInfo *info,
-                           uint32_t n, uint32_t buckets)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    info[i].cls[0] = info[i].cls[1] = info[i].cls[2] = 0;
-    if (nodes[i].ref_count <= kChunk)
+    if (lane == 0)
+        nodes[i].first_item = first;
+    if (lane < 3)
+        info[i].cls[lane] = 0;
+    if (cnt == 1)
         return; // single work item: every accumulator is written with plain stores
-    for (int k = 0; k < 12; ++k)
-        bnd[12 * i + k] = (k < 3 || (k >= 6 && k < 9)) ? kOInf : kONegInf;
-    for (uint32_t b = 0; b < buckets; ++b) {
-        uint32_t *o = obj + (size_t)(i * buckets + b) * 7;
-        o[0] = 0;
-        for (int k = 0; k < 3; ++k) {
-            o[1 + k] = kOInf;
-            o[4 + k] = kONegInf;
-        }
-        uint32_t *s = sp + (size_t)(i * buckets + b) * 8;
-        s[0] = s[1] = 0;
-        for (int k = 0; k < 3; ++k) {
-            s[2 + k] = kOInf;
-            s[5 + k] = kONegInf;
-        }
+    if (lane < 12)
+        bnd[12 * i + lane] = (lane < 3 || (lane >= 6 && lane < 9)) ? kOInf : kONegInf;
+    for (uint32_t k = lane; k < buckets * 7; k += kEvalLanes) {
+        const uint32_t f = k % 7;
+        obj[(size_t)i * buckets * 7 + k] = f == 0 ? 0u : (f < 4 ? kOInf : kONegInf);
+    }
+    for (uint32_t k = lane; k < buckets * 8; k += kEvalLanes) {
+        const uint32_t f = k % 8;
+        sp[(size_t)i * buckets * 8 + k] = f < 2 ? 0u : (f < 5 ? kOInf : kONegInf);
     }
 }
 
@@ -268,10 +261,10 @@ KS_D float warp_max(float v)
 }
 
 // Node bounds and centroid bounds (cuda/sbvh.cu:308-313, 330-333).
-__global__ void k_bounds(const Item *items, uint32_t n_items, const BRef *refs, uint32_t *bnd)
+__global__ void k_bounds(const Item *items, const uint32_t *n_items, const BRef *refs, uint32_t *bnd)
 {
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n_items)
+    if (w >= *n_items)
         return;
     Item it = items[w];
     float v[12];
@@ -351,13 +344,13 @@ __global__ void k_prep(const LevelNode *nodes, uint32_t n, const uint32_t *bnd, 
 }
 
 // Object-split bucket statistics (cuda/sbvh.cu:95-102).
-__global__ void k_obj_bins(const Item *items, uint32_t n_items, const BRef *refs, const NodeInfo *info,
+__global__ void k_obj_bins(const Item *items, const uint32_t *n_items, const BRef *refs, const NodeInfo *info,
                            uint32_t buckets, uint32_t *obj)
 {
     __shared__ uint32_t sbins[kWarpsPerBlock][kMaxBuckets * 7];
     uint32_t wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t w = blockIdx.x * kWarpsPerBlock + wl;
-    if (w >= n_items)
+    if (w >= *n_items)
         return;
     Item it = items[w];
     const NodeInfo &ni = info[it.node];
@@ -396,57 +389,73 @@ __global__ void k_obj_bins(const Item *items, uint32_t n_items, const BRef *refs
     }
 }
 
-// Picks the cheapest split of a bucket table (cuda/sbvh.cu:104-130, 190-216).
-// bins: per bucket [count-like for left, count-like for right, min xyz, max xyz] accessors.
+// Picks the cheapest split of a bucket table (cuda/sbvh.cu:104-130, 190-216) with kEvalLanes lanes, one split each,
+// and writes it (all lanes of the warp call; a group without a node passes its own flag).
+// lc, rc, box: a bucket's counts for the left and the right side, and its bounds.
+// Bound by the latency of its table reads: a thread per node went over the table 15 times (k_obj_eval and k_decide
+// 1.02 + 0.44 ms of the build of a level-7 icosphere's 327680 triangles, 21 us for the root alone; now 0.42 + 0.16).
 template <typename LeftCount, typename RightCount, typename BoxOf>
-KS_D void best_split(uint32_t buckets, float travw, float node_sa, LeftCount lc, RightCount rc, BoxOf box,
-                     int &best_bucket, float &best_cost, float bl[6], float br[6])
+KS_D void best_split(bool active, uint32_t lane, uint32_t buckets, float travw, float node_sa, LeftCount lc, RightCount rc,
+                     BoxOf box, int &best_bucket, float &best_cost, float bl[6], float br[6])
 {
-    for (uint32_t i = 0; i + 1 < buckets; ++i) {
-        float L[6], R[6];
-        box_empty(L);
-        box_empty(R);
+    float L[6], R[6], cost = kInf;
+    box_empty(L);
+    box_empty(R);
+    if (active && lane + 1 < buckets) {
         uint32_t c0 = 0, c1 = 0;
-        for (uint32_t j = 0; j <= i; ++j) {
+        for (uint32_t j = 0; j < buckets; ++j) {
             float b[6];
             box(j, b);
-            box_expand(L, b);
-            c0 += lc(j);
-        }
-        for (uint32_t j = i + 1; j < buckets; ++j) {
-            float b[6];
-            box(j, b);
-            box_expand(R, b);
-            c1 += rc(j);
-        }
-        float cost = travw + ((float)c0 * surface_area(L, L + 3) + (float)c1 * surface_area(R, R + 3)) / node_sa;
-        if (i == 0 || cost < best_cost) {
-            best_cost = cost;
-            best_bucket = (int)i;
-            for (int k = 0; k < 6; ++k) {
-                bl[k] = L[k];
-                br[k] = R[k];
+            if (j <= lane) {
+                box_expand(L, b);
+                c0 += lc(j);
+            } else {
+                box_expand(R, b);
+                c1 += rc(j);
             }
         }
+        cost = travw + ((float)c0 * surface_area(L, L + 3) + (float)c1 * surface_area(R, R + 3)) / node_sa;
+        // the first split stands even where its cost is not a number; a later one then never wins
+        if (lane > 0 && !(cost == cost))
+            cost = kInf;
     }
+    uint32_t best = lane;
+    float best_c = cost;
+    for (int o = 1; o < kEvalLanes; o <<= 1) {
+        const float c = __shfl_xor_sync(0xffffffffu, best_c, o);
+        const uint32_t l = __shfl_xor_sync(0xffffffffu, best, o);
+        // the lower split unless the higher one is cheaper
+        if (l > best ? c < best_c : !(best_c < c)) {
+            best = l;
+            best_c = c;
+        }
+    }
+    if (active && lane == best) {
+        best_bucket = (int)lane;
+        best_cost = cost;
+        for (int k = 0; k < 6; ++k) {
+            bl[k] = L[k];
+            br[k] = R[k];
+        }
+    }
+    __syncwarp();
 }
 
 __global__ void k_obj_eval(uint32_t n, const uint32_t *obj, NodeInfo *info, Params p)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    NodeInfo &ni = info[i];
-    if (ni.kind != kPending)
-        return;
-    const uint32_t *o = obj + (size_t)i * p.buckets * 7;
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kEvalLanes, lane = threadIdx.x % kEvalLanes;
+    const bool active = i < n && info[i].kind == kPending;
+    NodeInfo &ni = info[i < n ? i : 0];
+    const uint32_t *o = obj + (size_t)(i < n ? i : 0) * p.buckets * 7;
     float node_sa = surface_area(ni.bmin, ni.bmax);
     auto cnt = [&](uint32_t j) { return o[j * 7]; };
     auto box = [&](uint32_t j, float b[6]) {
         for (int k = 0; k < 6; ++k)
             b[k] = o2f(o[j * 7 + 1 + k]);
     };
-    best_split(p.buckets, p.trav_weight, node_sa, cnt, cnt, box, ni.os_bucket, ni.os_cost, ni.osL, ni.osR);
+    best_split(active, lane, p.buckets, p.trav_weight, node_sa, cnt, cnt, box, ni.os_bucket, ni.os_cost, ni.osL, ni.osR);
+    if (!active)
+        return;
     // skipSpatialSplit (cuda/sbvh.cu:132-134)
     float imn[3], imx[3];
     bool empty = false;
@@ -457,22 +466,24 @@ __global__ void k_obj_eval(uint32_t n, const uint32_t *obj, NodeInfo *info, Para
     if (imn[0] > imx[0] || imn[1] > imx[1] || imn[2] > imx[2])
         empty = true; // intersect() returns an empty AABB3, whose is_empty() is true
     float isa = empty ? 0.0f : surface_area(imn, imx);
-    ni.skip = (isa / g_root_sa <= p.alpha) ? 1 : 0;
-    if (!ni.skip) {
+    const int skip = (isa / g_root_sa <= p.alpha) ? 1 : 0;
+    if (lane == 0)
+        ni.skip = skip;
+    if (!skip) {
         int d = ni.dim;
-        for (uint32_t b = 0; b <= p.buckets; ++b)
+        for (uint32_t b = lane; b <= p.buckets; b += kEvalLanes)
             ni.clip[b] = std_lerp(ni.bmin[d], ni.bmax[d], (float)b / (float)p.buckets);
     }
 }
 
 // Spatial-split bucket statistics (cuda/sbvh.cu:154-176).
-__global__ void k_sp_bins(const Item *items, uint32_t n_items, const BRef *refs, const NodeInfo *info,
+__global__ void k_sp_bins(const Item *items, const uint32_t *n_items, const BRef *refs, const NodeInfo *info,
                           uint32_t buckets, uint32_t *sp)
 {
     __shared__ uint32_t sbins[kWarpsPerBlock][kMaxBuckets * 8];
     uint32_t wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t w = blockIdx.x * kWarpsPerBlock + wl;
-    if (w >= n_items)
+    if (w >= *n_items)
         return;
     Item it = items[w];
     const NodeInfo &ni = info[it.node];
@@ -526,30 +537,29 @@ __global__ void k_sp_bins(const Item *items, uint32_t n_items, const BRef *refs,
 // Spatial estimate + leaf/object/spatial decision (cuda/sbvh.cu:347-360).
 __global__ void k_decide(const LevelNode *nodes, uint32_t n, const uint32_t *sp, NodeInfo *info, Params p)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kEvalLanes, lane = threadIdx.x % kEvalLanes;
+    const bool active = i < n && info[i].kind == kPending;
+    NodeInfo &ni = info[i < n ? i : 0];
+    const bool skip = ni.skip;
+    const uint32_t *s = sp + (size_t)(i < n ? i : 0) * p.buckets * 8;
+    float node_sa = surface_area(ni.bmin, ni.bmax);
+    auto enter = [&](uint32_t j) { return s[j * 8 + 0]; };
+    auto exitc = [&](uint32_t j) { return s[j * 8 + 1]; };
+    auto box = [&](uint32_t j, float b[6]) {
+        for (int k = 0; k < 6; ++k)
+            b[k] = o2f(s[j * 8 + 2 + k]);
+    };
+    best_split(active && !skip, lane, p.buckets, p.trav_weight, node_sa, enter, exitc, box, ni.ss_bucket, ni.ss_cost, ni.ssL,
+               ni.ssR);
+    if (!active || lane)
         return;
-    NodeInfo &ni = info[i];
-    if (ni.kind != kPending)
-        return;
-    if (!ni.skip) {
-        const uint32_t *s = sp + (size_t)i * p.buckets * 8;
-        float node_sa = surface_area(ni.bmin, ni.bmax);
-        auto enter = [&](uint32_t j) { return s[j * 8 + 0]; };
-        auto exitc = [&](uint32_t j) { return s[j * 8 + 1]; };
-        auto box = [&](uint32_t j, float b[6]) {
-            for (int k = 0; k < 6; ++k)
-                b[k] = o2f(s[j * 8 + 2 + k]);
-        };
-        best_split(p.buckets, p.trav_weight, node_sa, enter, exitc, box, ni.ss_bucket, ni.ss_cost, ni.ssL, ni.ssR);
-    }
     uint32_t ref_count = nodes[i].ref_count;
     float leaf_cost = (float)ref_count;
-    if (ref_count <= p.max_prims && leaf_cost <= ni.os_cost && (ni.skip || leaf_cost <= ni.ss_cost)) {
+    if (ref_count <= p.max_prims && leaf_cost <= ni.os_cost && (skip || leaf_cost <= ni.ss_cost)) {
         ni.kind = kLeaf;
         return;
     }
-    if (ni.skip || ni.os_cost <= ni.ss_cost) {
+    if (skip || ni.os_cost <= ni.ss_cost) {
         ni.kind = kObject;
     } else {
         ni.kind = kSpatial;
@@ -559,10 +569,10 @@ __global__ void k_decide(const LevelNode *nodes, uint32_t n, const uint32_t *sp,
 }
 
 // Left / right / straddling counts of a spatial split (cuda/sbvh.cu:242-251).
-__global__ void k_sp_classes(const Item *items, uint32_t n_items, const BRef *refs, NodeInfo *info)
+__global__ void k_sp_classes(const Item *items, const uint32_t *n_items, const BRef *refs, NodeInfo *info)
 {
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n_items)
+    if (w >= *n_items)
         return;
     Item it = items[w];
     NodeInfo &ni = info[it.node];
@@ -604,21 +614,24 @@ __global__ void k_sp_costs(uint32_t n, NodeInfo *info)
     ni.full_cost = ni.saL * (float)ni.n1 + ni.saR * (float)ni.n2;
 }
 
-// Per work item: how many references go left, right, or into the leaf pool.
-__global__ void k_count(const Item *items, uint32_t n_items, const BRef *refs, const NodeInfo *info,
-                        uint32_t buckets, uint32_t *cl, uint32_t *cr, uint32_t *cp)
+// Per work item: how many references go left, right, or into the leaf pool: three arrays of n_max entries, zero past
+// the level's items.
+__global__ void k_count(const Item *items, const uint32_t *n_items, uint32_t n_max, const BRef *refs,
+                        const NodeInfo *info, uint32_t buckets, uint32_t *counts)
 {
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n_items)
+    if (w >= n_max)
         return;
-    Item it = items[w];
-    const NodeInfo &ni = info[it.node];
     uint32_t l = 0, r = 0, p = 0;
-    for (uint32_t j = lane; j < it.count; j += 32) {
-        int dst = ref_destination(refs[it.begin + j], ni, buckets);
-        l += dst & 1;
-        r += (dst >> 1) & 1;
-        p += (dst >> 2) & 1;
+    if (w < *n_items) {
+        const Item it = items[w];
+        const NodeInfo &ni = info[it.node];
+        for (uint32_t j = lane; j < it.count; j += 32) {
+            int dst = ref_destination(refs[it.begin + j], ni, buckets);
+            l += dst & 1;
+            r += (dst >> 1) & 1;
+            p += (dst >> 2) & 1;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -626,9 +639,9 @@ __global__ void k_count(const Item *items, uint32_t n_items, const BRef *refs, c
         p += __shfl_xor_sync(0xffffffffu, p, o);
     }
     if (lane == 0) {
-        cl[w] = l;
-        cr[w] = r;
-        cp[w] = p;
+        counts[w] = l;
+        counts[n_max + w] = r;
+        counts[2 * n_max + w] = p;
     }
 }
 
@@ -636,7 +649,7 @@ __global__ void k_count(const Item *items, uint32_t n_items, const BRef *refs, c
 // one side empty trips the reference's assertion (cuda/sbvh.cu:295); such a node falls back to
 // its object split and the level is recounted.
 __global__ void k_child_counts(uint32_t n, const uint32_t *item_off, const uint32_t *sl, const uint32_t *sr,
-                               NodeInfo *info, uint32_t *flag)
+                               NodeInfo *info, uint32_t *flag, uint32_t *split)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -649,14 +662,24 @@ __global__ void k_child_counts(uint32_t n, const uint32_t *item_off, const uint3
         ni.kind = kObject;
         atomicAdd(flag, 1u);
     }
+    split[i] = ni.kind != kLeaf;
 }
 
-__global__ void k_scatter(const Item *items, uint32_t n_items, const BRef *refs, const NodeInfo *info,
+// What the host reads of a level: references left and right, to leaves, splits, nodes that fell back.
+__global__ void k_totals(const uint32_t *sl, const uint32_t *sr, const uint32_t *spool, const uint32_t *split,
+                         const uint32_t *flag, uint32_t *out)
+{
+    const uint32_t *src[5] = {sl, sr, spool, split, flag};
+    if (threadIdx.x < 5)
+        out[threadIdx.x] = *src[threadIdx.x];
+}
+
+__global__ void k_scatter(const Item *items, const uint32_t *n_items, const BRef *refs, const NodeInfo *info,
                           uint32_t buckets, const uint32_t *sl, const uint32_t *sr, const uint32_t *spool,
                           uint32_t left_total, BRef *next, uint32_t pool_base, uint32_t *pool)
 {
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n_items)
+    if (w >= *n_items)
         return;
     Item it = items[w];
     const NodeInfo &ni = info[it.node];
@@ -708,17 +731,10 @@ __global__ void k_scatter(const Item *items, uint32_t n_items, const BRef *refs,
     }
 }
 
-__global__ void k_split_flags(const NodeInfo *info, uint32_t n, uint32_t *flags)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        flags[i] = (info[i].kind == kObject || info[i].kind == kSpatial) ? 1u : 0u;
-}
-
 __global__ void k_children(const LevelNode *nodes, uint32_t n, const NodeInfo *info, const uint32_t *split_scan,
                            uint32_t n_split, const uint32_t *sl, const uint32_t *sr, const uint32_t *spool,
                            uint32_t left_total, uint32_t pool_base, uint32_t next_build_base, BuildRec *recs,
-                           LevelNode *next_nodes)
+                           LevelNode *next_nodes, uint32_t *next_items)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -746,6 +762,8 @@ __global__ void k_children(const LevelNode *nodes, uint32_t n, const NodeInfo *i
     R.first_item = 0;
     next_nodes[k] = L;
     next_nodes[n_split + k] = R;
+    next_items[k] = item_count(L.ref_count);
+    next_items[n_split + k] = item_count(R.ref_count);
     rec.leaf = 0;
     rec.left = L.build_id;
     rec.right = R.build_id;
@@ -896,12 +914,18 @@ struct BuildScratch
     DevBuf<LevelNode> nodes_a, nodes_b;
     DevBuf<Item> items;
     DevBuf<NodeInfo> info;
-    DevBuf<uint32_t> bnd, obj, sp, item_cnt, item_off, cl, cr, cp, sl, sr, spool, split_flag, split_scan, pool, flag;
+    DevBuf<uint32_t> bnd, obj, sp, item_cnt, item_off, counts, count_scan, split_flag, split_scan, pool, flag, totals;
     DevBuf<uint32_t> interior_flag, interior_scan;
     DevBuf<uint32_t> wide_binary, wide_child, wide_level;
     DevBuf<float> wide_bound;
     DevBuf<BuildRec> recs;
     ScanScratch scan;
+    uint32_t *h_totals = nullptr; // pinned
+    ~BuildScratch()
+    {
+        if (h_totals)
+            cudaFreeHost(h_totals);
+    }
 };
 
 static BuildScratch &build_scratch(ks_context *ctx)
@@ -921,7 +945,7 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     auto &items = bs.items;
     auto &info = bs.info;
     auto &bnd = bs.bnd, &obj = bs.obj, &sp = bs.sp, &item_cnt = bs.item_cnt, &item_off = bs.item_off;
-    auto &cl = bs.cl, &cr = bs.cr, &cp = bs.cp, &sl = bs.sl, &sr = bs.sr, &spool = bs.spool;
+    auto &counts = bs.counts, &count_scan = bs.count_scan;
     auto &split_flag = bs.split_flag, &split_scan = bs.split_scan, &pool = bs.pool, &flag = bs.flag;
     auto &recs = bs.recs;
     auto &scan = bs.scan;
@@ -933,11 +957,17 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
     size_t rec_cap = (size_t)n_tris * 4 + 1024;
     KS_CUDA_TRY(ctx, recs.reserve(rec_cap));
     KS_CUDA_TRY(ctx, flag.reserve(1));
+    KS_CUDA_TRY(ctx, bs.totals.reserve(5));
+    if (!bs.h_totals)
+        KS_CUDA_TRY(ctx, cudaMallocHost((void **)&bs.h_totals, sizeof(uint32_t) * 5));
 
     k_init_refs<<<grid_for(n_tris, 256), 256, 0, st>>>(verts, indices, tri_begin, n_tris, refs_a.ptr);
     LevelNode root{0, n_tris, 0, 0};
     KS_CUDA_TRY(ctx, nodes_a.reserve(1));
     KS_CUDA_TRY(ctx, cudaMemcpyAsync(nodes_a.ptr, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+    const uint32_t root_items = (n_tris + kChunk - 1) / kChunk;
+    KS_CUDA_TRY(ctx, item_cnt.reserve(1));
+    KS_CUDA_TRY(ctx, cudaMemcpyAsync(item_cnt.ptr, &root_items, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
 
     uint32_t n_active = 1, n_refs = n_tris, build_base = 0, pool_used = 0;
     std::vector<uint32_t> level_begin;
@@ -949,67 +979,53 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
         level_begin.push_back(build_base);
         if ((size_t)build_base + n_active > rec_cap)
             return fail(ctx, KS_ERR_OUT_OF_MEMORY, "sbvh build: node record capacity exceeded");
-        // work items
-        KS_CUDA_TRY(ctx, item_cnt.reserve(n_active));
+        // work items (the last kernel of the level before counted them); the host knows no more than their bound
         KS_CUDA_TRY(ctx, item_off.reserve(n_active + 1));
-        k_item_counts<<<grid_for(n_active, 256), 256, 0, st>>>(cur_nodes->ptr, n_active, item_cnt.ptr);
         KS_CUDA_TRY(ctx, exclusive_scan(item_cnt.ptr, item_off.ptr, n_active, scan, st));
-        uint32_t n_items = 0;
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(&n_items, item_off.ptr + n_active, 4, cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-        KS_CUDA_TRY(ctx, items.reserve(n_items));
-        k_items_fill<<<grid_for(n_active, 256), 256, 0, st>>>(cur_nodes->ptr, n_active, item_off.ptr, items.ptr);
-        // accumulators
+        const uint32_t max_items = n_active + n_refs / kChunk;
+        const uint32_t *n_items = item_off.ptr + n_active;
+        KS_CUDA_TRY(ctx, items.reserve(max_items));
         KS_CUDA_TRY(ctx, info.reserve(n_active));
         KS_CUDA_TRY(ctx, bnd.reserve((size_t)n_active * 12));
         KS_CUDA_TRY(ctx, obj.reserve((size_t)n_active * p.buckets * 7));
         KS_CUDA_TRY(ctx, sp.reserve((size_t)n_active * p.buckets * 8));
-        k_acc_init<<<grid_for(n_active, 128), 128, 0, st>>>(cur_nodes->ptr, bnd.ptr, obj.ptr, sp.ptr, info.ptr,
-                                                            n_active, p.buckets);
-        unsigned wgrid = grid_for((uint64_t)n_items * 32, 256);
-        unsigned wgrid8 = grid_for(n_items, kWarpsPerBlock);
+        const unsigned wgrid = grid_for((uint64_t)max_items * 32, 256);
+        const unsigned wgrid8 = grid_for(max_items, kWarpsPerBlock);
+        const unsigned eval_grid = grid_for((uint64_t)n_active * kEvalLanes, 128);
+        k_items_fill<<<eval_grid, 128, 0, st>>>(cur_nodes->ptr, n_active, item_off.ptr, items.ptr, bnd.ptr, obj.ptr, sp.ptr,
+                                                info.ptr, p.buckets);
         k_bounds<<<wgrid, 256, 0, st>>>(items.ptr, n_items, cur, bnd.ptr);
         k_prep<<<grid_for(n_active, 128), 128, 0, st>>>(cur_nodes->ptr, n_active, bnd.ptr, info.ptr, recs.ptr + 0,
                                                         level == 0);
         k_obj_bins<<<wgrid8, kWarpsPerBlock * 32, 0, st>>>(items.ptr, n_items, cur, info.ptr, p.buckets, obj.ptr);
-        k_obj_eval<<<grid_for(n_active, 128), 128, 0, st>>>(n_active, obj.ptr, info.ptr, p);
+        k_obj_eval<<<eval_grid, 128, 0, st>>>(n_active, obj.ptr, info.ptr, p);
         k_sp_bins<<<wgrid8, kWarpsPerBlock * 32, 0, st>>>(items.ptr, n_items, cur, info.ptr, p.buckets, sp.ptr);
-        k_decide<<<grid_for(n_active, 128), 128, 0, st>>>(cur_nodes->ptr, n_active, sp.ptr, info.ptr, p);
+        k_decide<<<eval_grid, 128, 0, st>>>(cur_nodes->ptr, n_active, sp.ptr, info.ptr, p);
         k_sp_classes<<<wgrid, 256, 0, st>>>(items.ptr, n_items, cur, info.ptr);
         k_sp_costs<<<grid_for(n_active, 128), 128, 0, st>>>(n_active, info.ptr);
-        KS_CUDA_TRY(ctx, cl.reserve(n_items));
-        KS_CUDA_TRY(ctx, cr.reserve(n_items));
-        KS_CUDA_TRY(ctx, cp.reserve(n_items));
-        KS_CUDA_TRY(ctx, sl.reserve(n_items + 1));
-        KS_CUDA_TRY(ctx, sr.reserve(n_items + 1));
-        KS_CUDA_TRY(ctx, spool.reserve(n_items + 1));
+        KS_CUDA_TRY(ctx, counts.reserve((size_t)max_items * 3));
+        KS_CUDA_TRY(ctx, count_scan.reserve(((size_t)max_items + 1) * 3));
+        KS_CUDA_TRY(ctx, split_flag.reserve(n_active));
+        KS_CUDA_TRY(ctx, split_scan.reserve(n_active + 1));
+        const uint32_t *sl = count_scan.ptr, *sr = sl + max_items + 1, *spool = sr + max_items + 1;
         for (int pass = 0;; ++pass) {
-            k_count<<<wgrid, 256, 0, st>>>(items.ptr, n_items, cur, info.ptr, p.buckets, cl.ptr, cr.ptr, cp.ptr);
-            KS_CUDA_TRY(ctx, exclusive_scan(cl.ptr, sl.ptr, n_items, scan, st));
-            KS_CUDA_TRY(ctx, exclusive_scan(cr.ptr, sr.ptr, n_items, scan, st));
-            KS_CUDA_TRY(ctx, exclusive_scan(cp.ptr, spool.ptr, n_items, scan, st));
+            k_count<<<wgrid, 256, 0, st>>>(items.ptr, n_items, max_items, cur, info.ptr, p.buckets, counts.ptr);
+            KS_CUDA_TRY(ctx, exclusive_scan(counts.ptr, count_scan.ptr, max_items, scan, st, 3));
             KS_CUDA_TRY(ctx, cudaMemsetAsync(flag.ptr, 0, 4, st));
-            k_child_counts<<<grid_for(n_active, 128), 128, 0, st>>>(n_active, item_off.ptr, sl.ptr, sr.ptr, info.ptr,
-                                                                    flag.ptr);
-            uint32_t changed = 0;
-            KS_CUDA_TRY(ctx, cudaMemcpyAsync(&changed, flag.ptr, 4, cudaMemcpyDeviceToHost, st));
+            k_child_counts<<<grid_for(n_active, 128), 128, 0, st>>>(n_active, item_off.ptr, sl, sr, info.ptr, flag.ptr,
+                                                                    split_flag.ptr);
+            KS_CUDA_TRY(ctx, exclusive_scan(split_flag.ptr, split_scan.ptr, n_active, scan, st));
+            k_totals<<<1, 32, 0, st>>>(sl + max_items, sr + max_items, spool + max_items, split_scan.ptr + n_active,
+                                       flag.ptr, bs.totals.ptr);
+            KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.h_totals, bs.totals.ptr, sizeof(uint32_t) * 5, cudaMemcpyDeviceToHost, st));
             KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-            if (!changed)
+            if (!bs.h_totals[4])
                 break;
             if (pass > 0)
                 return fail(ctx, KS_ERR_INVALID_ARGUMENT, "sbvh build: degenerate split could not be resolved");
         }
-        KS_CUDA_TRY(ctx, split_flag.reserve(n_active));
-        KS_CUDA_TRY(ctx, split_scan.reserve(n_active + 1));
-        k_split_flags<<<grid_for(n_active, 256), 256, 0, st>>>(info.ptr, n_active, split_flag.ptr);
-        KS_CUDA_TRY(ctx, exclusive_scan(split_flag.ptr, split_scan.ptr, n_active, scan, st));
-        uint32_t totals[4] = {0, 0, 0, 0};
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(&totals[0], sl.ptr + n_items, 4, cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(&totals[1], sr.ptr + n_items, 4, cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(&totals[2], spool.ptr + n_items, 4, cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(&totals[3], split_scan.ptr + n_active, 4, cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-        uint32_t left_total = totals[0], right_total = totals[1], leaf_total = totals[2], n_split = totals[3];
+        const uint32_t left_total = bs.h_totals[0], right_total = bs.h_totals[1], leaf_total = bs.h_totals[2];
+        const uint32_t n_split = bs.h_totals[3];
         size_t next_refs = (size_t)left_total + right_total;
         if (next_refs > nxt_buf->count) {
             // grow the next-level buffer (contents are rewritten by the scatter)
@@ -1018,13 +1034,13 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
         }
         if ((size_t)pool_used + leaf_total > pool.count)
             return fail(ctx, KS_ERR_OUT_OF_MEMORY, "sbvh build: leaf pool capacity exceeded");
-        k_scatter<<<wgrid, 256, 0, st>>>(items.ptr, n_items, cur, info.ptr, p.buckets, sl.ptr, sr.ptr, spool.ptr,
-                                         left_total, nxt, pool_used, pool.ptr);
+        k_scatter<<<wgrid, 256, 0, st>>>(items.ptr, n_items, cur, info.ptr, p.buckets, sl, sr, spool, left_total, nxt, pool_used, pool.ptr);
         KS_CUDA_TRY(ctx, nxt_nodes->reserve((size_t)2 * n_split + 1));
+        KS_CUDA_TRY(ctx, item_cnt.reserve((size_t)2 * n_split + 1));
         uint32_t next_build_base = build_base + n_active;
         k_children<<<grid_for(n_active, 128), 128, 0, st>>>(cur_nodes->ptr, n_active, info.ptr, split_scan.ptr, n_split,
-                                                            sl.ptr, sr.ptr, spool.ptr, left_total, pool_used,
-                                                            next_build_base, recs.ptr, nxt_nodes->ptr);
+                                                            sl, sr, spool, left_total, pool_used, next_build_base,
+                                                            recs.ptr, nxt_nodes->ptr, item_cnt.ptr);
         // the level's node list is read by k_children above; keep the swap after it
         KS_CUDA_TRY(ctx, cudaGetLastError());
         pool_used += leaf_total;
@@ -1038,7 +1054,6 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
         if ((uint32_t)level > (ctx->limits.sbvh_max_levels ? ctx->limits.sbvh_max_levels : 4096u))
             return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: level limit reached");
     }
-    (void)n_refs;
     const uint32_t n_nodes = build_base;
     level_begin.push_back(build_base);
     // subtree sizes bottom-up, DFS numbering top-down
