@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_shadow_grou
 
 // ---- persistent two-level traversal (instanced scenes) ----------------------------------------
 #ifndef KS_INST_MIN_BLOCKS
-#define KS_INST_MIN_BLOCKS 1
+#define KS_INST_MIN_BLOCKS 5 // see inst_warp_step
 #endif
 // The same warp-level ray fetch as k_extend_pt / k_shadow_pt over inst_step (ks_traverse.cuh):
 // each ray makes the tests of traverse_instances, in resumable steps.

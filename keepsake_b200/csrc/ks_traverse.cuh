@@ -680,13 +680,9 @@ KS_D bool trav_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
 // instead of with the two or three that reach a leaf in the same step.  Any-hit queries step without
 // waiting: holding back a leaf that may end the ray costs them more than the batching saves.  Returns
 // true when this lane's ray is over.  Leaf batches of 8, 12, 16 lanes: mesh frame (1.3 M triangles,
-// 1024 x 1024 x 64) 38.9, 37.7, 37.5 ms of closest hits, box room 1.80, 1.71, 1.65; instanced scenes
-// (whose lanes also wait at the upper level) 21.9, 22.8, 24.0.
+// 1024 x 1024 x 64) 38.9, 37.7, 37.5 ms of closest hits, box room 1.80, 1.71, 1.65.
 #ifndef KS_LEAF_BATCH
 #define KS_LEAF_BATCH 12
-#endif
-#ifndef KS_LEAF_BATCH_INST
-#define KS_LEAF_BATCH_INST 8
 #endif
 #ifndef KS_LEAF_BATCH_ANY
 #define KS_LEAF_BATCH_ANY 0
@@ -1008,25 +1004,47 @@ KS_D bool inst_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
 }
 
 // Warp-wide step of the two-level traversal (every lane calls it; busy: the lane holds a ray).
-// Closest-hit queries batch their BLAS leaf tests like trav_warp_step: a lane whose BLAS node is
-// a leaf waits until KS_LEAF_BATCH_INST lanes (or all busy lanes) are at one.  Each ray's own sequence
-// of tests is that of inst_step.
+// Closest-hit queries take one of four kinds of step at a time (leaf tests of a prototype, the start of an
+// instance, a TLAS node, a node of a prototype), the first that KS_INST_LANES lanes wait for, instead of one after the
+// other in each warp step with a few lanes each; each ray's own sequence of tests is that of inst_step.  The kernel
+// is bound by the instructions it issues.  400 instances of 8 prototypes, 1920 x 1080 x 4: closest hits 21.2 ms with
+// leaf tests alone batched, 20.1 with these; 18.0 at the 20 warps an SM that 102 registers allow (118 before; at 24
+// warps the spills cost more: 21.0).  Lanes: 4 20.7, 8 20.1, 12 21.7 (at 118 registers); nodes first at 1 lane 18.6, 4
+// 17.9, 8 18.0.  Any-hit queries end early and gain nothing: 10.9 ms either way.
+#ifndef KS_INST_LANES
+#define KS_INST_LANES 8
+#endif
+#ifndef KS_INST_NODE_LANES
+#define KS_INST_NODE_LANES 4
+#endif
 template <bool kAnyHit, class Node>
 KS_D bool inst_warp_step(const Node *__restrict__ nodes, const float4 *__restrict__ tris, const InstanceView &iv,
                          InstTravState &s, uint4 *tstack, TravStack &blas_stack, int culling, int &overflow,
                          TravCount *count, bool busy)
 {
-    if constexpr (kAnyHit || KS_LEAF_BATCH_INST == 0) {
-        return busy && inst_step<kAnyHit>(nodes, tris, iv, s, tstack, blas_stack, culling, overflow, count);
-    } else {
-        const bool at_leaf = busy && s.in_blas && s.blas.at_leaf();
-        const uint32_t leaves = __ballot_sync(0xffffffffu, at_leaf);
-        const uint32_t others = __ballot_sync(0xffffffffu, busy && !at_leaf);
-        const bool leaf_phase = __popc(leaves) >= KS_LEAF_BATCH_INST || others == 0;
-        if (leaf_phase ? !at_leaf : (!busy || at_leaf))
-            return false;
-        return inst_step<false>(nodes, tris, iv, s, tstack, blas_stack, culling, overflow, count);
+    bool run = busy;
+    if constexpr (!kAnyHit) {
+        const bool top = busy && !s.in_blas;
+        const bool start = top && (s.ref & kLeafBit) && s.item < s.cnt;
+        const bool tlas = top && !start;
+        const bool leaf = busy && s.in_blas && s.blas.at_leaf();
+        const bool node = busy && s.in_blas && !leaf;
+        const int n_leaf = __popc(__ballot_sync(0xffffffffu, leaf));
+        const int n_start = __popc(__ballot_sync(0xffffffffu, start));
+        const int n_tlas = __popc(__ballot_sync(0xffffffffu, tlas));
+        const int n_node = __popc(__ballot_sync(0xffffffffu, node));
+        if (n_leaf >= KS_INST_LANES)
+            run = leaf;
+        else if (n_start >= KS_INST_LANES)
+            run = start;
+        else if (n_tlas >= KS_INST_LANES)
+            run = tlas;
+        else if (n_node >= KS_INST_NODE_LANES)
+            run = node;
+        else // few lanes are left: any kind that has one
+            run = n_tlas ? tlas : (n_start ? start : (n_node ? node : leaf));
     }
+    return run && inst_step<kAnyHit>(nodes, tris, iv, s, tstack, blas_stack, culling, overflow, count);
 }
 
 } // namespace ksb
