@@ -646,8 +646,11 @@ __global__ void __launch_bounds__(128) k_subsurface_select(const __grid_constant
 // Walks of the queue, a step of every lane's walk at a time; once KS_WALK_REFILL lanes are idle they take new
 // walks.  Few hits walk, and a walk takes 1 to 256 steps (16 on average): run where the hits lie they kept 2 or
 // 3 lanes of a warp busy (subsurface box and sphere, 256 x 256 x 16: 13.4 ms a frame, 10.3 with the queue).  What
-// is left is latency: the longest walk's 256 steps one after the other, about 4.5 us each, so neither the
-// refill (4, 8, 16 idle lanes: 11.1, 11.0, 11.0 ms) nor more CTAs (5, 6, 8 per SM: 11.5, 12.6, 13.3 ms) helps.
+// is left is latency: the longest walk's 256 steps one after the other, so neither the refill (4, 8, 16 idle
+// lanes: 11.1, 11.0, 11.0 ms) nor more CTAs per SM (5, 6, 8: 11.5, 12.6, 13.3 ms; by a register cap, 4 and 5 instead of 3:
+// 9.2 and 10.7 against 8.9) helps, but a shorter step does: rays through the 4-wide view, which halves
+// the nodes met, took the frame from 12.0 to 8.2 ms.  A ray with nearly equal hits, and every ray of a tree too
+// deep for the view, takes the exact traversal.
 #ifndef KS_WALK_REFILL
 #define KS_WALK_REFILL 8
 #endif
@@ -661,10 +664,24 @@ __global__ void __launch_bounds__(128) k_subsurface_walk(const __grid_constant__
     uint32_t i = ~0u, mesh = 0;
     bool drained = false;
     int of = 0;
+    KS_TRAV_STACK(stack);
     auto cast = [&](const RayQuery &ray, WalkExit &e) {
         Hit hh;
-        traverse<false>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, ray, 2, hh, of, nullptr,
-                        MeshOnly{sv.tri_mesh, mesh});
+        hh.tri = ~0u;
+        bool exact = sv.deep;
+        if (!exact) {
+            Trav4 t;
+            if (trav_begin(t, ray, 0u, sv.root_count, sv.bmin, sv.bmax)) {
+                const Tree4 tree{sv.wide, sv.leaf_box};
+                while (!trav_step<false>(tree, sv.prim_tris, t, stack, 2, of, nullptr, MeshOnly{sv.tri_mesh, mesh})) {
+                }
+                exact = ambiguous(t);
+                hh = t.hit;
+            }
+        }
+        if (exact)
+            traverse<false>(sv.nodes, sv.prim_tris, sv.root_ref, sv.root_count, sv.bmin, sv.bmax, ray, 2, hh, of, nullptr,
+                            MeshOnly{sv.tri_mesh, mesh});
         if (hh.tri == ~0u)
             return false;
         e = WalkExit{hh.slot, hh.t, hh.b1, hh.b2};
