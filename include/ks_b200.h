@@ -308,13 +308,12 @@ ks_status ks_trace_rays(ks_scene *scene, const float *rays, uint32_t n, int any_
                         float *t, float *bary);
 
 /* The same queries through the renderer's traversal kernels.  Flat scenes: a 4-wide view of the
- * same SBVH (each node with its interior children replaced by theirs, boxes tested with the same
- * slab test), nearest slot first; it reaches the same leaves, so the result equals
- * ks_trace_rays' except where two triangles are hit at exactly the same distance (the visiting
- * order then picks one of them).  Instanced scenes: the persistent two-level traversal over the
- * TLAS and the 4-wide view of the BLAS nodes, the same except at exact ties.  Replaces the same
- * reference calls as
- * ks_trace_rays (cuda/sbvh.cu:512-603); exists to test the rendering traversal. */
+ * same SBVH with conservative boxes, nearest slot first; a hit counts when the exact slab test accepts
+ * its leaf's box, so the result equals ks_trace_rays' except where two triangles are hit at
+ * exactly the same distance (the visiting order then picks one of them).  Instanced scenes: the
+ * persistent two-level traversal over the TLAS and 4-wide steps of the BLAS nodes, the same except
+ * at exact ties.  Replaces the same reference calls as ks_trace_rays (cuda/sbvh.cu:512-603);
+ * exists to test the rendering traversal. */
 ks_status ks_trace_rays_wide(ks_scene *scene, const float *rays, uint32_t n, int any_hit, int culling,
                              uint32_t *tri_idx, float *t, float *bary);
 

@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128, KS_SHADE_MIN_BLOCKS) k_shade(const __grid
                     finish = true;
                 } else {
                     f3 wo = -normalize(rd);
-                    // a random walk's exit (k_subsurface marks its hit distance negative) shades with the
+                    // a random walk's exit (k_subsurface_walk marks its hit distance negative) shades with the
                     // Lambertian exit lobe
                     const std::conditional_t<kVariant == kShadeGeneral, AnyBsdf, Principled> bsdf{
                         kVariant == kShadeGeneral && h.x < 0.0f ? subsurface_exit_closure(mat.ss_ior) : make_closure(mat)};
