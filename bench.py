@@ -15,8 +15,9 @@ render, FP64 image download every step).
 
 Roofline of the closest-hit traversal kernel: algorithmic bytes per query as the CPU oracle counts
 them on the same frame (32 B per SBVH node whose bound the reference traversal tests, 48 B per
-triangle tested, 48 B of ray and hit I/O), over the kernel's CUDA-event time; beside it the
-kernel's own fetch count (128 B per 4-wide node, 48 B per triangle).
+triangle tested, 48 B of ray and hit I/O; only where the oracle traces through the reference's SBVH),
+over the kernel's CUDA-event time; beside it, or instead, the kernel's own fetch count (128 B per
+4-wide node, 48 B per triangle).
 
 time_to_relmse: the glossy scene behind an occluder (the same icosphere made glossy-heavy,
 roughness U[0.02,0.2], with an opaque slab between it and the sun) at 1920x1080, depth 12.  The
@@ -34,7 +35,8 @@ instanced scene (400 instances, 3840x2160, 1024 spp, depth 16) plain and guided.
 --impl reference runs the CPU implementation of the path on all host cores (the oracle's
 restatement of small_pt over the reference's own SBVH traversal, with the scene, camera and
 parameters made by the oracle library, without loading the CUDA library) on the same frame and
-configuration, each step one 16-spp interval of the 256-spp render of the full frame.
+configuration, each step one 16-spp interval of the 256-spp render of the full frame; where the
+reference's SBVH is not built (no reference tree) it prints that it is unavailable.
 """
 import argparse
 import ctypes
@@ -553,6 +555,10 @@ def reference_arm(args):
         return 0
     ol = oracle_module()
     orc = ol.load()
+    if not orc.rays_are_reference():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's ray queries (cuda/sbvh.cu) are not "
+                          "built: no reference tree on this machine"}), flush=True)
+        return 0
     g = orc.generate("icosphere", 0, level=8, sky=(2048, 1024), resolution=(W_RES, H_RES))
     params = orc.params(render_width=W_RES, render_height=H_RES, spp=SPP, bounces=BOUNCES, rng_seed=0)
     threads = os.cpu_count() or 1
@@ -661,8 +667,10 @@ def main():
         threads = os.cpu_count() or 1
         r = run_cpu(orc, g.desc, cam, params, 1, 0, threads)
         cpu = {"value": r["rays"] / r["seconds"] / 1e6, "unit": "Mrays/s", "cores": threads, "kind": "port",
-               "sample": r["sample"] + "; oracle restatement of small_pt over the reference cuda/sbvh.cu traversal"}
-        owork = oracle_work(r["scene"], cam, params, threads)
+               "sample": r["sample"] + "; oracle restatement of small_pt over " +
+                         ("the reference cuda/sbvh.cu traversal" if orc.rays_are_reference() else "its own binary tree")}
+        if orc.rays_are_reference():
+            owork = oracle_work(r["scene"], cam, params, threads)
 
     # roofline of the dominant kernel (closest-hit traversal).  Algorithmic bytes per query as the
     # oracle counts them on this frame: 32 B per node whose bound the reference traversal tests +
@@ -698,7 +706,7 @@ def main():
     else:
         roofline.update(achieved=achieved_kernel, frac=achieved_kernel / peak,
                         algorithmic_bytes_per_launch=kernel_bytes / launches,
-                        bytes_model="the kernel's own fetch count (no CPU leg in this run)")
+                        bytes_model="the kernel's own fetch count (no count of the reference traversal in this run)")
 
     # ---- end to end through the host-buffer C ABI ----
     e2e_steps = args.e2e_steps if args.e2e_steps is not None else args.steps

@@ -14,12 +14,14 @@
 //   DistribTable / DistribTable2D distrib.cpp:9-107
 //   RenderTarget2::add / add_miss render_target.cpp:82-107 (FP64 accumulation)
 //
-// Ray queries go through the reference's own SBVH (cuda/sbvh.cu, oracle/_ref).
+// Ray queries go through the reference's own SBVH (cuda/sbvh.cu, oracle/_ref) or, without it, the
+// oracle's own tree (o_rays.h).
 // The two float atomics of the reference (the sky luminance threshold light.cpp:35-48 and the
 // sky power light.cpp:136-159) have no fixed order there; here both are summed in a fixed order
 // (rows sequentially in double) so the product can reproduce them exactly.
 #include "../../include/ks_b200.h"
 #include "o_bsdf.h"
+#include "o_rays.h"
 #include "o_texture.h"
 #include "o_subsurface.h"
 #include "o_math.h"
@@ -33,16 +35,6 @@
 #include <numeric>
 #include <thread>
 #include <vector>
-
-extern "C" {
-int ksref_sbvh_build(const float *, uint32_t, const uint32_t *, uint32_t, uint32_t, uint32_t, float, float, void **,
-                     uint32_t *, uint32_t *);
-uint32_t ksref_sbvh_intersect1(void *, const float *, int, float *, float *);
-uint32_t ksref_sbvh_intersect1_counted(void *, const float *, int, int, float *, float *, uint64_t *,
-                                       int (*)(void *, uint32_t, float, float), void *);
-void ksref_sbvh_bound(void *, float *);
-void ksref_sbvh_destroy(void *);
-}
 
 namespace oracle
 {
@@ -586,7 +578,7 @@ struct Scene
     std::vector<Texture> textures;
     std::vector<std::vector<Binding>> mat_bindings; // per material, in the order given
     bool any_opacity = false;
-    void *bvh = nullptr;
+    std::unique_ptr<rays::Tree> bvh;
     float bound[6];
     std::unique_ptr<Sky> sky;
     std::vector<MeshLight> mesh_lights;
@@ -597,11 +589,6 @@ struct Scene
     uint32_t light_count = 0;
     std::vector<float> powers;
 
-    ~Scene()
-    {
-        if (bvh)
-            ksref_sbvh_destroy(bvh);
-    }
     V3 vert(uint32_t v) const { return V3(verts[3 * v], verts[3 * v + 1], verts[3 * v + 2]); }
     V3 tri_vert(uint32_t t, int k) const { return vert(idx[3 * t + k]); }
 
@@ -844,13 +831,13 @@ inline bool intersect(const Scene &s, V3 o, V3 d, float tmax, uint32_t &tri, flo
         // the reference's SBVH queries take no filter: its traversal restated, with the filter
         AlphaFilter f{&s, o, d};
         uint64_t dummy[3] = {0, 0, 0};
-        tri = ksref_sbvh_intersect1_counted(s.bvh, r, 0, 2, &t, bary, work ? work->ext : dummy, AlphaFilter::call, &f);
+        tri = s.bvh->query(r, false, &t, bary, work ? work->ext : dummy, AlphaFilter::call, &f);
         return tri != ~0u;
     }
-    tri = ksref_sbvh_intersect1(s.bvh, r, 0, &t, bary);
+    tri = s.bvh->query_plain(r, false, &t, bary);
     if (work) {
         float t2 = 0.0f, b2[3] = {0, 0, 0};
-        uint32_t tri2 = ksref_sbvh_intersect1_counted(s.bvh, r, 0, 2, &t2, b2, work->ext, nullptr, nullptr);
+        uint32_t tri2 = s.bvh->query(r, false, &t2, b2, work->ext, nullptr, nullptr);
         if (tri2 != tri || (tri != ~0u && std::memcmp(&t2, &t, sizeof(float)) != 0))
             ++work->mismatches;
     }
@@ -862,12 +849,10 @@ inline bool occluded(const Scene &s, V3 o, V3 d, float tmax, Work *work = nullpt
     if (s.any_opacity) {
         AlphaFilter f{&s, o, d};
         uint64_t dummy[3] = {0, 0, 0};
-        return ksref_sbvh_intersect1_counted(s.bvh, r, 1, 2, nullptr, nullptr, work ? work->shadow : dummy,
-                                             AlphaFilter::call, &f) != 0;
+        return s.bvh->query(r, true, nullptr, nullptr, work ? work->shadow : dummy, AlphaFilter::call, &f) != 0;
     }
-    const bool occ = ksref_sbvh_intersect1(s.bvh, r, 1, nullptr, nullptr) != 0;
-    if (work && (ksref_sbvh_intersect1_counted(s.bvh, r, 1, 2, nullptr, nullptr, work->shadow, nullptr, nullptr) !=
-                 0) != occ)
+    const bool occ = s.bvh->query_plain(r, true, nullptr, nullptr) != 0;
+    if (work && (s.bvh->query(r, true, nullptr, nullptr, work->shadow, nullptr, nullptr) != 0) != occ)
         ++work->mismatches;
     return occ;
 }
@@ -1284,8 +1269,7 @@ struct Tracer
                         } mf{&s, mesh};
                         float bary[3];
                         uint64_t dummy[3] = {0, 0, 0};
-                        tri_out = ksref_sbvh_intersect1_counted(s.bvh, r, 0, 2, &t_out, bary, dummy, MeshFilter::call,
-                                                                &mf);
+                        tri_out = s.bvh->query(r, false, &t_out, bary, dummy, MeshFilter::call, &mf);
                         b1 = bary[1];
                         b2 = bary[2];
                         return tri_out != ~0u;
@@ -1379,11 +1363,11 @@ Scene *create_scene(const ks_scene_desc *d, const ks_sbvh_options *opts)
     ks_sbvh_options o{4, 12, 1.0f, 1e-5f};
     if (opts)
         o = *opts;
-    uint32_t nn, np;
-    if (ksref_sbvh_build(s->verts.data(), vo, s->idx.data(), (uint32_t)s->tri_mesh.size(), o.max_prims_in_node,
-                         o.bucket_count, o.trav_weight, o.alpha, &s->bvh, &nn, &np) != 0)
+    s->bvh.reset(rays::build(s->verts.data(), vo, s->idx.data(), (uint32_t)s->tri_mesh.size(), o.max_prims_in_node,
+                             o.bucket_count, o.trav_weight, o.alpha));
+    if (!s->bvh)
         return nullptr;
-    ksref_sbvh_bound(s->bvh, s->bound);
+    s->bvh->bound(s->bound);
 
     // sky light (light.cpp:19-57)
     const ks_sky_desc &sd = d->sky;
@@ -1546,6 +1530,19 @@ void *oracle_scene_create(const ks_scene_desc *desc, const ks_sbvh_options *opts
 }
 
 void oracle_scene_destroy(void *s) { delete (Scene *)s; }
+
+// Whether the ray queries are the reference's own SBVH's.
+int oracle_rays_are_reference() { return oracle::rays::is_reference() ? 1 : 0; }
+
+// The queries themselves, laid out as ks_trace_rays' (8 floats a ray: origin, tmin, direction, tmax).
+void oracle_trace_rays(void *sp, const float *rays, uint32_t n, int any_hit, uint32_t *tri, float *t, float *bary)
+{
+    const Scene *s = (const Scene *)sp;
+    for (uint32_t i = 0; i < n; ++i) {
+        t[i] = bary[3 * i] = bary[3 * i + 1] = bary[3 * i + 2] = 0.0f;
+        tri[i] = s->bvh->query_plain(rays + 8 * (size_t)i, any_hit != 0, t + i, bary + 3 * (size_t)i);
+    }
+}
 
 // Light tables for parity checks: powers (light_count floats) and the power CDF
 // (light_count + 1 floats); returns light_count.

@@ -51,6 +51,9 @@ class Oracle:
         L.oracle_scene_create.restype = _vp
         L.oracle_scene_destroy.argtypes = [_vp]
         L.oracle_scene_destroy.restype = None
+        L.oracle_rays_are_reference.restype = ctypes.c_int
+        L.oracle_trace_rays.argtypes = [_vp, _vp, _u32, ctypes.c_int, _vp, _vp, _vp]
+        L.oracle_trace_rays.restype = None
         L.oracle_light_table.argtypes = [_vp, _vp, _vp]
         L.oracle_light_table.restype = _u32
         L.oracle_sky_tables.argtypes = [_vp, _vp, _vp]
@@ -95,6 +98,10 @@ class Oracle:
             else:
                 setattr(p, k, v)
         return p
+
+    def rays_are_reference(self):
+        """Whether the oracle traces its rays through the reference's own SBVH (else its own tree)."""
+        return bool(self.lib.oracle_rays_are_reference())
 
     def scene(self, desc, keepalive=None):
         return OracleScene(self, desc, keepalive)
@@ -143,6 +150,14 @@ class OracleScene:
             dp = ctypes.cast(ctypes.pointer(desc), _vp)
         self.h = oracle.lib.oracle_scene_create(dp, None)
         assert self.h, "oracle_scene_create failed"
+
+    def trace(self, rays, any_hit=False):
+        """The oracle's ray queries, both sides of every triangle: as Scene.trace."""
+        rays = np.ascontiguousarray(rays, np.float32).reshape(-1, 8)
+        n = len(rays)
+        tri, t, bary = np.empty(n, np.uint32), np.empty(n, np.float32), np.empty((n, 3), np.float32)
+        self.o.lib.oracle_trace_rays(self.h, P(rays), n, int(any_hit), P(tri), P(t), P(bary))
+        return (tri.astype(bool), None, None) if any_hit else (tri, t, bary)
 
     def light_table(self):
         n = self.o.lib.oracle_light_table(self.h, None, None)
@@ -309,4 +324,8 @@ def load():
 
 
 def ref_sbvh():
+    """The reference's SBVH; skips the calling test where it was not built (no reference tree)."""
+    if not os.path.exists(REF_SO):
+        import pytest
+        pytest.skip("the reference's SBVH (oracle/_ref) is not built: no reference tree")
     return RefSBVH()
