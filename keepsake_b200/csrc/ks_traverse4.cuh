@@ -40,9 +40,11 @@ KS_D float min3f(float a, float b, float c)
     return r;
 }
 
-// Relative slack of the box test, of the pruning distance and of the tie test (Trav4).
+// Relative slack of the box test, of the ray's end, of the pruning distance and of the tie test (Trav4).
+// An entry time that is compared with the ray's end may lie above slab()'s by 3 roundings (2^-24 each; the
+// padding by the origin vanishes at the origin) and, on the stack, by the slot number in its last two bits (3 ulp).
 constexpr float kMaxInv = 1e30f; // 1 / d is clamped to it
-constexpr float kBoxSlack = 0x1p-20f, kPruneSlack = 0x1p-12f, kTieSlack = 0x1p-20f;
+constexpr float kBoxSlack = 0x1p-20f, kRangeSlack = 0x1p-18f, kPruneSlack = 0x1p-12f, kTieSlack = 0x1p-20f;
 
 // What the traversal reads: the nodes, and per leaf (at its first primitive slot) its box, 2 float4.
 struct Tree4
@@ -59,7 +61,7 @@ struct Trav4
     f3 o_in, inv_out, o_out; // t of an entry plane: b inv - o_in; of an exit plane: b inv_out - o_out
     uint32_t ref;            // the node or leaf to visit
     int sp;
-    float limit;             // boxes and triangles beyond it are skipped
+    float limit;             // boxes and triangles beyond it are skipped: no less than what ends the query
     Hit hit;
     float entry;             // entry time of the hit's leaf
     float second;            // distance of the closest other hit seen
@@ -115,7 +117,7 @@ KS_D bool trav_begin(Trav4 &s, const RayQuery &ray, uint32_t root, uint32_t root
     s.ray = ray;
     s.th = make_tri_helper(ray.d);
     s.set_ray(ray.d);
-    s.limit = ray.tmax;
+    s.limit = ray.tmax + fabsf(ray.tmax) * kRangeSlack;
     s.entry = 0.0f;
     s.second = kInf;
     s.sp = 0;
@@ -243,7 +245,7 @@ KS_D void trav4_take(Trav4 &s, const Hit &h, float entry)
         if (s.hit.tri != ~0u)
             s.second = fminf(s.second, s.hit.t);
         s.entry = entry;
-        s.limit = fminf(s.ray.tmax, h.t + fabsf(h.t) * kPruneSlack);
+        s.limit = fminf(s.limit, h.t + fabsf(h.t) * kPruneSlack);
         s.hit = h;
     } else {
         s.second = fminf(s.second, h.t);
@@ -267,7 +269,7 @@ KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restri
         const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
         const uint32_t tri = __float_as_uint(a.w);
         RayQuery q = s.ray;
-        q.tmax = s.limit;
+        q.tmax = fminf(q.tmax, s.limit);
         float t, b0, b1, b2;
         if (!cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, t, b0, b1, b2)) {
             float entry;
@@ -276,7 +278,7 @@ KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restri
                     s.hit.tri = tri;
                     return true;
                 }
-            } else if (t < s.limit && leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
+            } else if (t < q.tmax && leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
                 trav4_take(s, Hit{tri, slot, t, b0, b1, b2}, entry);
             }
         }
@@ -372,7 +374,7 @@ KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 
                 const bool mine = !last || (int)k < __ffs(ends);
                 const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
                 RayQuery q = s.ray;
-                q.tmax = s.limit;
+                q.tmax = fminf(q.tmax, s.limit);
                 Hit h;
                 h.tri = __float_as_uint(a.w);
                 h.slot = slot;
@@ -381,7 +383,7 @@ KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 
                 if (mine) {
                     count->tris++;
                     take = !cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, h.t, h.b0, h.b1, h.b2) &&
-                           (kAnyHit || h.t < s.limit) && leaf_reached(tree.leaf_box, s, first, entry) &&
+                           (kAnyHit || h.t < q.tmax) && leaf_reached(tree.leaf_box, s, first, entry) &&
                            alpha(h.tri, h.b1, h.b2, s.ray);
                 }
                 uint32_t found = (__ballot_sync(mask, take) >> shift) & ((1u << kGroup) - 1u);

@@ -97,3 +97,44 @@ def test_short_queues_render_the_same(ctx, W, H, batch):
     assert np.array_equal(wts, wts_c)
     assert np.allclose(acc, acc_c, rtol=1e-14, atol=0)
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_prims", [1, 4])
+def test_hits_just_within_the_range(ctx, max_prims):
+    """Rays that end within 8 ulp beyond a hit: flat triangles across the axes, so that their boxes are entered at
+    the hit's distance, each in a plane of its own (no ties), among triangles that are passed by.  Axis rays
+    from points with few bits meet the planes exactly; oblique ones start at 0, where the box test's
+    padding by the origin vanishes."""
+    import keepsake_b200 as ks
+    rng = np.random.default_rng(5)
+    n, m = 240, 4000
+    axis, plane = np.arange(n) % 3, (1 + rng.permutation(n)).astype(np.float32) / 64
+    v = rng.integers(-256, 257, (n, 3, 3)).astype(np.float32) / 64
+    v[np.arange(n), :, axis] = plane[:, None]
+    desc, keep = ks.triangle_soup_desc(v.reshape(-1, 3), np.arange(3 * n, dtype=np.uint32).reshape(-1, 3))
+    s = ks.Scene(ctx, desc, keep)
+    s.build_bvh(max_prims=max_prims)
+    r = np.zeros((2 * m, 8), np.float32)
+    r[:m, 0:3] = rng.integers(-200, 200, (m, 3)) / 64 + 1 / 256
+    k = rng.integers(0, 3, m)
+    r[np.arange(m), k] = 0.0
+    r[np.arange(m), 4 + k] = 1.0
+    r[m:, 4:7] = np.abs(rng.normal(size=(m, 3))) + 1e-3
+    r[:, 7] = np.inf
+    tri0, t0, _ = s.trace(r)
+    r = r[tri0 != 0xFFFFFFFF]
+    t0 = t0[tri0 != 0xFFFFFFFF]
+    assert len(r) > m // 2
+    end = t0
+    hits = []
+    for ulp in range(0, 9):
+        r[:, 7] = end
+        tri, t, _ = s.trace(r)
+        wtri, wt, _ = s.trace(r, wide=True)
+        assert np.array_equal(tri, wtri) and np.array_equal(t[tri != 0xFFFFFFFF], wt[tri != 0xFFFFFFFF]), ulp
+        assert np.array_equal(s.trace(r, any_hit=True)[0], s.trace(r, any_hit=True, wide=True)[0]), ulp
+        end = np.nextafter(end, np.float32(np.inf))
+        hits.append((tri != 0xFFFFFFFF).sum())
+    assert hits[0] < hits[-1]  # the sweep crosses the ends that matter
+    s.close()
