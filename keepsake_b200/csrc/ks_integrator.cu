@@ -65,8 +65,9 @@ using namespace wave;
 #endif
 
 // Per-iteration counters: paths continuing, shadow rays, hit queue, miss queue, extension-ray
-// fetch, shadow-ray fetch, subsurface walks, walk fetch, simple hits, general hits.
-constexpr uint32_t kCounters = 10;
+// fetch, shadow-ray fetch, subsurface walks, walk fetch, simple hits, general hits, fetch of a batch's rays in
+// deep trees.
+constexpr uint32_t kCounters = 12;
 
 // ---- kernels --------------------------------------------------------------------------------
 
@@ -256,10 +257,11 @@ KS_D float4 hit_record(const Hit &h, bool retrace = false)
 // paths into the hit and miss queues in index order, so that shading reads the path state in
 // order.  kBatch: paths of many jobs, the count read from the batch state.
 // kAlpha: the scene has opacity maps; candidate hits go through their stochastic test (SceneAlpha).
-// kDeep: the tree (of some job) is too deep for the 4-wide view.
+// kDeep: the tree is too deep for the 4-wide view.  kMixed: a batch of which some job's is; its rays go to the
+// variant that their job's tree takes (the check cost a batch without such jobs 1.6 %).
 // count_ptr: where the count lies on the device when the host does not know it yet (else null); choose: the
 // group kernel was launched too, and short queues are its.
-template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
+template <bool kBatch = false, bool kAlpha = false, bool kDeep = false, bool kMixed = false>
 __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
                                                    const uint32_t *count_ptr, int choose, float4 *hits, uint32_t *fetch,
                                                    int *overflow, unsigned long long *work, BatchView bv)
@@ -287,7 +289,9 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
             tree = View::tree(sv);
             tris = sv.prim_tris;
-            if (trav_begin(s, path_ray(pb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
+            if (kMixed && (sv.deep != 0) != kDeep) {
+                // the other variant's
+            } else if (trav_begin(s, path_ray(pb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
             else
                 hits[id] = make_float4(0, 0, 0, fbits(~0u));
@@ -413,7 +417,7 @@ KS_D RayQuery shadow_ray(const ShadowBuf &sb, uint32_t i)
 
 // Any-hit traversal of the NEE shadow rays with dynamic ray fetch (flat scenes); each ray is
 // finished by shadow_done as soon as its traversal ends.
-template <bool kBatch = false, bool kAlpha = false, bool kDeep = false>
+template <bool kBatch = false, bool kAlpha = false, bool kDeep = false, bool kMixed = false>
 __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const __grid_constant__ SceneView sv_in, ShadowBuf sb,
                                                    const uint32_t *shadow_count, int choose, uint32_t *fetch, PathBuf nxt,
                                                    double *accum_in, double *weights_in, int *overflow,
@@ -442,7 +446,9 @@ __global__ void __launch_bounds__(128, KS_SHADOW_MIN_BLOCKS) k_shadow_pt(const _
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
             tree = View::tree(sv);
             tris = sv.prim_tris;
-            if (trav_begin(s, shadow_ray(sb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
+            if (kMixed && (sv.deep != 0) != kDeep) {
+                // the other variant's
+            } else if (trav_begin(s, shadow_ray(sb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
             else
                 shadow_done<kBatch>(sb, id, false, nxt, accum_in, weights_in, gv, bv);
@@ -497,6 +503,8 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_extend_grou
     for (uint32_t i = group_first_ray(); i < count; i += stride) {
         const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
         const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+        if (kBatch && sv.deep)
+            continue; // k_extend_pt's
         Trav4 s;
         if (trav_begin(s, path_ray(pb, i), 0u, sv.root_count, sv.bmin, sv.bmax))
             group_trace<false>(Tree4{sv.wide, sv.leaf_box}, sv.prim_tris, s, stack, mask, 2, &tc, filter);
@@ -525,6 +533,8 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_shadow_grou
     for (uint32_t i = group_first_ray(); i < count; i += stride) {
         const uint32_t job = kBatch ? bits(sb.contrib[i].w) : 0u;
         const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
+        if (kBatch && sv.deep)
+            continue; // k_shadow_pt's
         Trav4 s;
         if (trav_begin(s, shadow_ray(sb, i), 0u, sv.root_count, sv.bmin, sv.bmax))
             group_trace<true>(Tree4{sv.wide, sv.leaf_box}, sv.prim_tris, s, stack, mask, 2, &tc, filter);
@@ -569,7 +579,7 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_extend_inst_pt(cons
             continue;
         }
         while (true) {
-            if (inst_warp_step<false>(sv.inst_wide, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc,
+            if (inst_warp_step<false>(sv.wide_steps, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc,
                                       ray != ~0u)) {
                 hits[ray] = hit_record(s.hit);
                 hit_inst[ray] = s.hit_inst;
@@ -613,7 +623,7 @@ __global__ void __launch_bounds__(128, KS_INST_MIN_BLOCKS) k_shadow_inst_pt(cons
         }
         while (true) {
             if (ray != ~0u &&
-                inst_step<true>(sv.inst_wide, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc)) {
+                inst_step<true>(sv.wide_steps, sv.prim_tris, sv.inst, s, tstack, stack, 2, of, &tc)) {
                 shadow_done<false>(sb, ray, s.hit.tri != ~0u, nxt, accum, weights, gv, BatchView{});
                 ray = ~0u;
             }
@@ -1367,7 +1377,8 @@ struct BatchWork
     DevBuf<unsigned long long> path_begin;
     DevBuf<BatchState> state_dev;
     DevBuf<float> filters; // the jobs' pixel-filter sample tables, concatenated
-    unsigned ext_grid = 0, shadow_grid = 0, group_grid = 0; // one wave of resident CTAs of the traversal kernels
+    // one wave of resident CTAs of the traversal kernels
+    unsigned ext_grid = 0, shadow_grid = 0, group_grid = 0, deep_ext_grid = 0, deep_shadow_grid = 0;
     int variant = kShadePlain;              // the shading kernel variant of the most demanding job
     int simple_variant = kShadePlain;       // ... and of the hits that do not need the general one
     bool any_simple = false;                // some job has such hits
@@ -1464,13 +1475,15 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     const GuideView gv{};
     k_batch_prep<<<1, 32, 0, st>>>(bv.state, cnt, capacity);
     k_raygen_batch<<<(unsigned)ctx->sm_count * 8, 256, 0, st>>>(bv, pb[cur]);
-    const auto ext_kernel = w.deep ? k_extend_pt<true, false, true> : k_extend_pt<true>;
-    const auto shadow_kernel = w.deep ? k_shadow_pt<true, false, true> : k_shadow_pt<true>;
+    const auto ext_kernel = w.deep ? k_extend_pt<true, false, false, true> : k_extend_pt<true>;
+    const auto shadow_kernel = w.deep ? k_shadow_pt<true, false, false, true> : k_shadow_pt<true>;
     ext_kernel<<<w.ext_grid, 128, 0, st>>>(SceneView{}, pb[cur], 0u, nullptr, 1, w.hits.ptr, cnt + 4, w.overflow.ptr,
                                            w.work.ptr, bv);
-    if (!w.deep)
-        k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, nullptr, 1, w.hits.ptr,
-                                                                  w.work.ptr, bv);
+    k_extend_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, pb[cur], 0u, nullptr, 1, w.hits.ptr,
+                                                              w.work.ptr, bv);
+    if (w.deep)
+        k_extend_pt<true, false, true, true><<<w.deep_ext_grid, 128, 0, st>>>(
+            SceneView{}, pb[cur], 0u, nullptr, 0, w.hits.ptr, cnt + 10, w.overflow.ptr, w.work.ptr, bv);
     const bool split = w.split.ptr != nullptr;
     (split ? k_build_queues<true, true> : k_build_queues<true>)<<<grid, 256, 0, st>>>(
         SceneView{}, pb[cur], w.hits.ptr, 0u, nullptr, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, w.split.ptr,
@@ -1490,9 +1503,11 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     shade(true, w.variant, w.queue[1].ptr, cnt + 3);
     shadow_kernel<<<w.shadow_grid, 128, 0, st>>>(SceneView{}, sb, cnt + 1, 1, cnt + 5, pb[1 - cur], nullptr, nullptr,
                                                  w.overflow.ptr, w.work.ptr + 2, gv, bv);
-    if (!w.deep)
-        k_shadow_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, sb, cnt + 1, 1, pb[1 - cur], nullptr, nullptr,
-                                                                  w.work.ptr + 2, gv, bv);
+    k_shadow_group<true><<<w.group_grid, kTravBlock, 0, st>>>(SceneView{}, sb, cnt + 1, 1, pb[1 - cur], nullptr, nullptr,
+                                                              w.work.ptr + 2, gv, bv);
+    if (w.deep)
+        k_shadow_pt<true, false, true, true><<<w.deep_shadow_grid, 128, 0, st>>>(
+            SceneView{}, sb, cnt + 1, 0, cnt + 11, pb[1 - cur], nullptr, nullptr, w.overflow.ptr, w.work.ptr + 2, gv, bv);
     k_batch_advance<<<1, 32, 0, st>>>(bv.state, cnt, handle, use_graph);
 }
 
@@ -1510,10 +1525,12 @@ static ks_status batch_render(ks_context *ctx, const ks_batch_job *jobs, uint32_
         (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(o.capacity ? o.capacity : 1u << 22,
                                                                                total));
     const unsigned grid = (unsigned)ctx->sm_count * (o.grid_per_sm ? std::min(o.grid_per_sm, 64u) : 16u);
-    w.ext_grid = w.deep ? resident_grid(k_extend_pt<true, false, true>, 128, ctx->sm_count)
-                        : resident_grid(k_extend_pt<true>, 128, ctx->sm_count);
-    w.shadow_grid = w.deep ? resident_grid(k_shadow_pt<true, false, true>, 128, ctx->sm_count)
-                           : resident_grid(k_shadow_pt<true>, 128, ctx->sm_count);
+    w.ext_grid = resident_grid(k_extend_pt<true>, 128, ctx->sm_count);
+    w.shadow_grid = resident_grid(k_shadow_pt<true>, 128, ctx->sm_count);
+    if (w.deep) {
+        w.deep_ext_grid = resident_grid(k_extend_pt<true, false, true, true>, 128, ctx->sm_count);
+        w.deep_shadow_grid = resident_grid(k_shadow_pt<true, false, true, true>, 128, ctx->sm_count);
+    }
     w.group_grid = resident_grid(k_extend_group<true>, kTravBlock, ctx->sm_count);
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < 4; ++f)

@@ -440,7 +440,7 @@ SceneView make_view(const ks_scene *s)
     v.inst_light_base = s->inst_light_base.ptr;
     v.nodes = s->trav_nodes.ptr;
     v.wide = s->wide_nodes.ptr;
-    v.inst_wide = s->inst_wide.ptr;
+    v.wide_steps = s->wide_steps.ptr;
     v.leaf_box = s->leaf_box.ptr;
     v.deep = s->deep ? 1 : 0;
     v.prim_tris = s->prim_tris.ptr;

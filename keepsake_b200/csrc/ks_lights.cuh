@@ -26,7 +26,7 @@ struct SceneView
     InstanceView inst; // instances (inst.n == 0: flat scene)
     const TravNode *nodes;
     const Wide4Node *wide;      // flat scenes: the renderer's 4-wide view of nodes
-    const WideNode *inst_wide;  // instanced scenes: 4-wide steps of the concatenated BLAS nodes
+    const WideNode *wide_steps; // instanced scenes: 4-wide steps of the concatenated BLAS nodes; deep ones: of nodes
     const float4 *leaf_box; // per leaf, at its first primitive slot: its box (2 float4)
     int deep;               // flat scene without the view (ks_scene::deep)
     const float4 *prim_tris;

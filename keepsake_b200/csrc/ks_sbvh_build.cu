@@ -1104,7 +1104,8 @@ static ks_status build_range(ks_context *ctx, const float *verts, const uint32_t
 
 // ---- the renderer's 4-wide view (Wide4Node) ----------------------------------------------------
 // Built from the binary nodes level by level.  A wide node opens its binary node: two children, then
-// the interior child of the largest area replaced by its own two, until there are 4 or only leaves.
+// the interior child of the largest area replaced by its own two, until there are 4 or only leaves
+// (`even`: each interior child replaced once instead).
 // k_wide4_alloc finds each node's interior children and gives them nodes of the next level (one atomic
 // per node); k_wide4_fill then writes all nodes at once, opening each the same way again.
 struct Opened4
@@ -1114,7 +1115,7 @@ struct Opened4
     int n;
 };
 
-__device__ __forceinline__ void open4(const TravNode *__restrict__ nodes, uint32_t ref, Opened4 &c)
+__device__ __forceinline__ void open4(const TravNode *__restrict__ nodes, uint32_t ref, bool even, Opened4 &c)
 {
     float area[4]; // of interior children
     auto put = [&](int at, const TravNode &t, int side) {
@@ -1135,11 +1136,19 @@ __device__ __forceinline__ void open4(const TravNode *__restrict__ nodes, uint32
         put(1, t, 1);
     }
     c.n = 2;
+    int next = 0; // even: the child to replace
     while (c.n < 4) {
         int best = -1;
-        for (int k = 0; k < c.n; ++k)
-            if (!(c.ref[k] & kLeafBit) && (best < 0 || area[k] > area[best]))
-                best = k;
+        if (even) {
+            while (next < c.n && (c.ref[next] & kLeafBit))
+                ++next;
+            best = next < c.n ? next : -1;
+            next += 2; // past what takes its place
+        } else {
+            for (int k = 0; k < c.n; ++k)
+                if (!(c.ref[k] & kLeafBit) && (best < 0 || area[k] > area[best]))
+                    best = k;
+        }
         if (best < 0)
             break;
         const TravNode t = nodes[c.ref[best]];
@@ -1159,8 +1168,8 @@ __device__ __forceinline__ void open4(const TravNode *__restrict__ nodes, uint32
 
 // Level `level` of the view: binary[i] is wide node i's binary node (kLeafBit: a tree that is one
 // leaf), level_n[l] the nodes of level l (complete below `level` + 1), child[i] the first child.
-__global__ void k_wide4_alloc(const TravNode *__restrict__ nodes, uint32_t level, uint32_t *level_n, uint32_t *binary,
-                              uint32_t *child)
+__global__ void k_wide4_alloc(const TravNode *__restrict__ nodes, uint32_t level, bool even, uint32_t *level_n,
+                              uint32_t *binary, uint32_t *child)
 {
     uint32_t begin = 0;
     for (uint32_t l = 0; l < level; ++l)
@@ -1173,7 +1182,7 @@ __global__ void k_wide4_alloc(const TravNode *__restrict__ nodes, uint32_t level
             continue;
         }
         Opened4 c;
-        open4(nodes, ref, c);
+        open4(nodes, ref, even, c);
         uint32_t inner = 0;
         for (int k = 0; k < c.n; ++k)
             inner += (c.ref[k] & kLeafBit) ? 0u : 1u;
@@ -1186,7 +1195,7 @@ __global__ void k_wide4_alloc(const TravNode *__restrict__ nodes, uint32_t level
 }
 
 // root_bound: the root's box, read when the tree is one leaf.
-__global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, const uint32_t *__restrict__ binary,
+__global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, bool even, const uint32_t *__restrict__ binary,
                              const uint32_t *__restrict__ child, const float *__restrict__ root_bound, Wide4Node *out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1202,7 +1211,7 @@ __global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, con
         }
         c.ref[0] = ref;
     } else {
-        open4(nodes, ref, c);
+        open4(nodes, ref, even, c);
     }
     Wide4Node w;
     float *plane = reinterpret_cast<float *>(w.plane);
@@ -1220,46 +1229,50 @@ __global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, con
 
 // The view of the tree over `nodes` whose root is root_ref with box root_bound (6 floats), into out (node 0:
 // the root).  Launches kWide4Chunk levels between two looks at the counts (a level without nodes costs its
-// launch); max_levels: levels of the binary tree.
+// launch); max_levels: levels of the binary tree, at most kMaxBinaryLevels.
 static ks_status build_wide4(ks_context *ctx, BuildScratch &bs, const TravNode *nodes, uint32_t n_trav, uint32_t root_ref,
-                             const float *root_bound, uint32_t max_levels, DevBuf<Wide4Node> &out, bool &too_deep)
+                             const float *root_bound, uint32_t max_levels, DevBuf<Wide4Node> &out)
 {
     constexpr uint32_t kWide4Chunk = 16;
     cudaStream_t st = ctx->stream;
-    const uint32_t levels = max_levels + kWide4Chunk + 1, one = 1;
+    const uint32_t levels = std::max(max_levels, kMaxWideLevels) + kWide4Chunk + 1, one = 1;
     KS_CUDA_TRY(ctx, bs.wide_binary.reserve((size_t)n_trav + 1));
     KS_CUDA_TRY(ctx, bs.wide_child.reserve((size_t)n_trav + 1));
     KS_CUDA_TRY(ctx, bs.wide_level.reserve(levels));
     KS_CUDA_TRY(ctx, bs.wide_bound.reserve(6));
-    KS_CUDA_TRY(ctx, cudaMemsetAsync(bs.wide_level.ptr, 0, sizeof(uint32_t) * levels, st));
-    KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_level.ptr, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_binary.ptr, &root_ref, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_bound.ptr, root_bound, sizeof(float) * 6, cudaMemcpyHostToDevice, st));
-    std::vector<uint32_t> count(levels, 0);
-    count[0] = 1;
-    uint32_t done = 0;
-    while (done < levels && count[done]) {
-        const uint32_t end = std::min(done + kWide4Chunk, levels - 1);
-        if (end == done)
-            return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: 4-wide level limit reached");
-        for (; done < end; ++done)
-            k_wide4_alloc<<<(unsigned)ctx->sm_count * 4, 128, 0, st>>>(nodes, done, bs.wide_level.ptr, bs.wide_binary.ptr,
-                                                                       bs.wide_child.ptr);
-        KS_CUDA_TRY(ctx, cudaMemcpyAsync(count.data(), bs.wide_level.ptr, sizeof(uint32_t) * levels,
-                                         cudaMemcpyDeviceToHost, st));
-        KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    std::vector<uint32_t> count;
+    bool even = false;
+    while (true) {
+        count.assign(levels, 0);
+        count[0] = 1;
+        KS_CUDA_TRY(ctx, cudaMemsetAsync(bs.wide_level.ptr, 0, sizeof(uint32_t) * levels, st));
+        KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_level.ptr, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+        uint32_t done = 0;
+        while (done < levels && count[done]) {
+            const uint32_t end = std::min(done + kWide4Chunk, levels - 1);
+            if (end == done)
+                return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: 4-wide level limit reached");
+            for (; done < end; ++done)
+                k_wide4_alloc<<<(unsigned)ctx->sm_count * 4, 128, 0, st>>>(nodes, done, even, bs.wide_level.ptr,
+                                                                           bs.wide_binary.ptr, bs.wide_child.ptr);
+            KS_CUDA_TRY(ctx, cudaMemcpyAsync(count.data(), bs.wide_level.ptr, sizeof(uint32_t) * levels,
+                                             cudaMemcpyDeviceToHost, st));
+            KS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        }
+        if (count[kMaxWideLevels] == 0)
+            break;
+        if (even)
+            return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: 4-wide levels exceed the traversal stack");
+        even = true;
     }
-    uint32_t n = 0, wide_levels = 0;
-    for (uint32_t c : count) {
+    uint32_t n = 0;
+    for (uint32_t c : count)
         n += c;
-        wide_levels += c ? 1 : 0;
-    }
-    too_deep = wide_levels > kMaxWideLevels;
-    if (too_deep)
-        return KS_OK;
     KS_CUDA_TRY(ctx, out.alloc(n));
-    k_wide4_fill<<<grid_for(n, 128), 128, 0, st>>>(nodes, n, bs.wide_binary.ptr, bs.wide_child.ptr, bs.wide_bound.ptr,
-                                                   out.ptr);
+    k_wide4_fill<<<grid_for(n, 128), 128, 0, st>>>(nodes, n, even, bs.wide_binary.ptr, bs.wide_child.ptr,
+                                                   bs.wide_bound.ptr, out.ptr);
     KS_CUDA_TRY(ctx, cudaGetLastError());
     return KS_OK;
 }
@@ -1432,9 +1445,9 @@ static ks_status build_instanced(ks_scene *scene, const Params &p)
     }
     KS_CUDA_TRY(ctx, cudaGetLastError());
     // 4-wide steps over the concatenated BLAS nodes (their refs are already global)
-    KS_CUDA_TRY(ctx, scene->inst_wide.alloc(total_trav > 0 ? total_trav : 1));
+    KS_CUDA_TRY(ctx, scene->wide_steps.alloc(total_trav > 0 ? total_trav : 1));
     if (total_trav > 0)
-        k_widen<<<grid_for(total_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, total_trav, scene->inst_wide.ptr);
+        k_widen<<<grid_for(total_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, total_trav, scene->wide_steps.ptr);
     // instance boxes: the 8 corners of the prototype box, transformed, padded by a relative epsilon
     TlasBuilder tb;
     for (uint32_t i = 0; i < scene->n_instances; ++i) {
@@ -1534,16 +1547,21 @@ ks_status build_sbvh(ks_scene *scene, const ks_sbvh_options &o, float *build_ms)
             scene->n_trav = r.n_trav;
             scene->root_count = r.n_prims;
             scene->root_ref = r.n_trav > 0 ? 0u : kLeafBit;
-            // the renderer's 4-wide view of the tree (timed with the build)
+            // the renderer's 4-wide view of the tree, or the exact traversal's steps (timed with the build)
             scene->deep = r.n_levels > kMaxBinaryLevels;
             scene->wide_nodes.release();
+            scene->wide_steps.release();
+            cudaEventRecord(ev2, st);
             if (!scene->deep) {
-                cudaEventRecord(ev2, st);
                 s = build_wide4(ctx, build_scratch(ctx), scene->trav_nodes.ptr, r.n_trav, scene->root_ref, r.bound,
-                                r.n_levels, scene->wide_nodes, scene->deep);
-                cudaEventRecord(ev3, st);
-                widened = s == KS_OK;
+                                r.n_levels, scene->wide_nodes);
+            } else if (scene->wide_steps.alloc(r.n_trav) != cudaSuccess) {
+                s = fail(ctx, KS_ERR_OUT_OF_MEMORY, "ks_scene_build_bvh: wide nodes");
+            } else {
+                k_widen<<<grid_for(r.n_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, r.n_trav, scene->wide_steps.ptr);
             }
+            cudaEventRecord(ev3, st);
+            widened = s == KS_OK;
         }
     }
     float ms = 0;

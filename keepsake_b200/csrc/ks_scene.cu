@@ -76,7 +76,7 @@ __global__ void trace_kernel(const TravNode *nodes, const float4 *tris, uint32_t
 
 // ks_trace_rays for flat scenes: the same queries as trace_kernel, traversed by trav_step with
 // dynamic ray fetch.  Tree = const TravNode *: each ray makes the same tests as traverse() (same triangle, t
-// and barycentrics); Tree = Tree4 or, in deep trees, const LazyWide * (ks_trace_rays_wide): the renderer's
+// and barycentrics); Tree = Tree4 or, in deep trees, const WideNode * (ks_trace_rays_wide): the renderer's
 // traversal, State its state; nodes_wide and root_wide are the tree it walks.
 template <class Tree, class State>
 __global__ void __launch_bounds__(128) trace_kernel_pt(const Tree nodes_wide, uint32_t root_wide, const TravNode *nodes,
@@ -907,7 +907,7 @@ static ks_status trace_rays_impl(ks_scene *scene, const float *rays, uint32_t n,
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_inst_kernel_pt, 128, 0);
         const unsigned grid = std::min<unsigned>((n + 127) / 128, (unsigned)std::max(per_sm, 1) * ctx->sm_count);
-        trace_inst_kernel_pt<<<grid, 128, 0, st>>>(scene->inst_wide.ptr, scene->prim_tris.ptr, make_view(scene).inst,
+        trace_inst_kernel_pt<<<grid, 128, 0, st>>>(scene->wide_steps.ptr, scene->prim_tris.ptr, make_view(scene).inst,
                                                    d_rays.ptr, n, any_hit, culling, d_tri.ptr, d_t.ptr, d_bary.ptr,
                                                    d_flag.ptr, d_fetch.ptr);
     } else if (scene->n_instances) {
@@ -931,8 +931,8 @@ static ks_status trace_rays_impl(ks_scene *scene, const float *rays, uint32_t n,
             run(trace_kernel_pt<const TravNode *, TravState>, static_cast<const TravNode *>(scene->trav_nodes.ptr),
                 scene->root_ref);
         else if (scene->deep)
-            run(trace_kernel_pt<const LazyWide *, TravState>,
-                reinterpret_cast<const LazyWide *>(scene->trav_nodes.ptr), scene->root_ref);
+            run(trace_kernel_pt<const WideNode *, TravState>, static_cast<const WideNode *>(scene->wide_steps.ptr),
+                scene->root_ref);
         else
             run(trace_kernel_pt<Tree4, Trav4>, Tree4{scene->wide_nodes.ptr, scene->leaf_box.ptr}, 0u);
     }

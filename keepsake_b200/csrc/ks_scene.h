@@ -36,8 +36,9 @@ constexpr uint32_t kPrimPad = 4; // records of padding after the last
 // A node of the exact traversal's 4-wide steps (ks_traverse.cuh): the children of an interior node, each
 // interior child replaced by its own two children (2 to 4 slots, in order).  Slot boxes are the SBVH's
 // boxes of those nodes; unused slots hold an empty box (lo +inf, hi -inf), which the slab test always
-// rejects.  Instanced scenes keep them for every interior node (indexed like the TravNode array, so child
-// refs need no renumbering; entries of nodes at odd depth are written but never read).
+// rejects.  Instanced scenes, and flat ones too deep for the view below, keep them for every interior node (indexed
+// like the TravNode array, so child refs need no renumbering; entries of nodes at odd depth are written but
+// never read).
 struct WideNode
 {
     float4 lo[3]; // per axis: the 4 slots' lower bounds
@@ -49,7 +50,9 @@ static_assert(sizeof(WideNode) == 128, "one 128-byte line per wide node");
 
 // The 4-wide view of the same SBVH that the renderer's traversal kernels read (ks_traverse4.cuh): a node
 // holds 1 to 4 nodes of the binary tree, found by replacing the largest interior child by its two
-// children until there are 4 (or leaves only), in their order.  Boxes are the SBVH's own; unused slots
+// children until there are 4 (or leaves only), in their order; where that gives more levels than the stack
+// holds (a small child that goes on beside large ones gains one binary level a level), by replacing each
+// interior child once, which halves the levels of any tree.  Boxes are the SBVH's own; unused slots
 // hold an empty box, never hit.  Every tree has a root node here, also one that is a single leaf.
 struct __align__(128) Wide4Node
 {
@@ -125,9 +128,9 @@ struct ks_scene
     // traversal layout
     ksb::DevBuf<ksb::TravNode> trav_nodes;
     ksb::DevBuf<ksb::Wide4Node> wide_nodes; // flat scenes: the renderer's 4-wide view of trav_nodes
-    ksb::DevBuf<ksb::WideNode> inst_wide;   // instanced scenes: 4-wide steps over trav_nodes
+    ksb::DevBuf<ksb::WideNode> wide_steps;  // instanced and deep scenes: 4-wide steps over trav_nodes
     ksb::DevBuf<float4> leaf_box; // per leaf, at its first primitive slot: its box (2 float4: lower, upper corner)
-    bool deep = false; // the tree is too deep for the view's stack: the exact traversal over trav_nodes
+    bool deep = false; // the tree is too deep for the view's stack: the exact traversal over wide_steps
     ksb::DevBuf<float4> prim_tris; // 3 float4 per primitive slot: v0 (+tri index bits in w), v1, v2
     uint32_t n_trav = 0;
     uint32_t root_ref = 0;   // ref of the root (leaf bit when the whole tree is one leaf)

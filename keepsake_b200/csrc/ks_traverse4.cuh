@@ -24,7 +24,10 @@ namespace ksb
 {
 
 // Deepest SBVH (levels) with this view: the exact traversal pushes at most 3 entries per two levels, so
-// up to here it never outgrows kWideStackDepth.  This one pushes at most 3 per level of the view.
+// up to here it never outgrows kWideStackDepth.  This one pushes at most 3 per level of the view; where opening
+// the largest child first gives more levels than that allows, the view opens evenly (build_wide4).  A sphere of
+// 81920 triangles, 512 x 512 x 4, beside nested clusters (58 levels) 3.3 ms, beside a chain (114 levels, the exact
+// steps) 3.9 ms; with both on binary nodes widened at each visit 9.6 and 10.2 ms.
 constexpr uint32_t kMaxBinaryLevels = 2 * (kWideStackDepth / 3), kMaxWideLevels = kWideStackDepth / 3;
 
 KS_D float max3f(float a, float b, float c)

@@ -422,8 +422,8 @@ KS_D f3 clamp_contrib(f3 v, int bounce_for_direct, const RenderParams &rp, bool 
     return v;
 }
 
-// What a flat scene's traversal kernel walks: the renderer's 4-wide view of the tree, or (kDeep) binary
-// nodes by the exact traversal's steps.
+// What a flat scene's traversal kernel walks: the renderer's 4-wide view of the tree, or (kDeep) the exact
+// traversal's 4-wide steps.
 template <bool kDeep>
 struct TreeOf
 {
@@ -436,8 +436,8 @@ template <>
 struct TreeOf<true>
 {
     using State = TravState;
-    using Tree = const LazyWide *;
-    KS_D static Tree tree(const SceneView &sv) { return reinterpret_cast<const LazyWide *>(sv.nodes); }
+    using Tree = const WideNode *;
+    KS_D static Tree tree(const SceneView &sv) { return sv.wide_steps; }
     KS_D static uint32_t root(const SceneView &sv) { return sv.root_ref; }
 };
 KS_D bool ambiguous(const TravState &) { return false; }
