@@ -66,8 +66,14 @@ using namespace wave;
 
 // Per-iteration counters: paths continuing, shadow rays, hit queue, miss queue, extension-ray
 // fetch, shadow-ray fetch, subsurface walks, walk fetch, simple hits, general hits, fetch of a batch's rays in
-// deep trees.
-constexpr uint32_t kCounters = 12;
+// deep trees (2), rays traced again.
+constexpr uint32_t kCounters = 13;
+
+// Rays traced again in an iteration (k_build_queues), as a share of its rays, from which the closest hits of a scene
+// are traced by the exact steps from then on: a ray that is traced again costs twice a ray of the 4-wide view, the
+// exact steps 1.2 to 1.4 times.  A box room with a second layer of 80,000 triangles in each wall's plane, 512 x 512
+// x 8: closest hits 2.0 ms by the exact steps, 5.4 with each ray traced again.
+constexpr uint32_t kAgainShare = 6, kAgainMin = 4096;
 
 // ---- kernels --------------------------------------------------------------------------------
 
@@ -317,8 +323,8 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
 }
 
 // Hit and miss queues from the per-ray results of k_extend_pt, one CTA-aggregated append per
-// kind (queue order follows the path index within each CTA's tile).  The few rays whose closest hit
-// depends on the visiting order are traced again here first.
+// kind (queue order follows the path index within each CTA's tile).  The rays whose closest hit depends on the
+// visiting order, few as a rule, are traced again here first, and counted.
 // kSplit: a scene (of some job) with materials of both kinds; the hits also go to one of two queues by the
 // shading variant their material needs (simple_queue at 0, general ones at split_cap).  Mixed in one queue,
 // the warps of an SM ran all BSDF kinds at once and waited for instructions 28 of 45 cycles.
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__
                                                       uint32_t count, const uint32_t *count_ptr, uint32_t *hit_queue,
                                                       uint32_t *miss_queue, uint32_t *queue_counts, int *overflow,
                                                       int alpha, uint32_t *split_queue, uint32_t split_cap,
-                                                      uint32_t *split_counts, BatchView bv)
+                                                      uint32_t *split_counts, uint32_t *again, BatchView bv)
 {
     count = queue_size<kBatch>(count, count_ptr, bv);
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -336,7 +342,10 @@ __global__ void __launch_bounds__(256, 4) k_build_queues(const __grid_constant__
         const uint32_t i = base + threadIdx.x;
         const bool valid = i < count;
         uint32_t slot = valid ? slots[4 * (size_t)i] : kNoHit;
+        const uint32_t retraced = __ballot_sync(0xffffffffu, slot == kRetrace);
         if (slot == kRetrace) {
+            if ((retraced & ((1u << (threadIdx.x & 31u)) - 1u)) == 0)
+                atomicAdd(again, (uint32_t)__popc(retraced));
             const uint32_t job = kBatch ? (bits(pb.beta_pix[i].w) >> kJobShift) : 0u;
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
             const RayQuery q = path_ray(pb, i);
@@ -719,7 +728,7 @@ struct RenderWork
     DevBuf<uint32_t> hit_inst; // instanced scenes: instance of each hit
     DevBuf<float4> samples; // 4 per path slot
     DevBuf<float4> shadow[4];
-    DevBuf<uint32_t> counters; // [next, shadow, hit queue, miss queue, extension fetch, shadow fetch]
+    DevBuf<uint32_t> counters; // two sets of kCounters
     DevBuf<uint32_t> queue[2]; // hit / miss path indices
     DevBuf<uint32_t> walks;    // scenes with subsurface materials: paths that walk this bounce
     DevBuf<uint32_t> split;    // scenes of mixed materials: simple hits, then (at the capacity) general ones
@@ -1031,7 +1040,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     // kept with the wavefront buffers: a pinned allocation and free per render cost milliseconds,
     // now and then far more
     if (!w.h_counts)
-        KS_CUDA_TRY(ctx, cudaMallocHost((void **)&w.h_counts, sizeof(uint32_t) * 8));
+        KS_CUDA_TRY(ctx, cudaMallocHost((void **)&w.h_counts, sizeof(uint32_t) * 2 * (kCounters + 1)));
     // guided renders: the guide's filter and inference run on a second stream, overlapping the
     // sampling and the miss shading, and join before the hit shading
     cudaStream_t aux = nullptr;
@@ -1051,7 +1060,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     struct Flight
     {
         cudaEvent_t ev[6] = {}, g0 = nullptr, g1 = nullptr, done = nullptr;
-        uint32_t *counters = nullptr, *h_counts = nullptr; // device and pinned: next paths, shadow rays, guide rows
+        uint32_t *counters = nullptr, *h_counts = nullptr; // device, and pinned with the guide's rows behind them
         uint32_t bound = 0;                                // its paths, or more
         int cur = 0;                                       // its path buffer
     } flights[2];
@@ -1064,7 +1073,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             cudaEventCreate(&flights[k].g1);
         }
         flights[k].counters = w.counters.ptr + k * kCounters;
-        flights[k].h_counts = w.h_counts + 4 * k;
+        flights[k].h_counts = w.h_counts + (kCounters + 1) * k;
     }
     cudaEvent_t t_begin, t_end;
     cudaEventCreate(&t_begin);
@@ -1074,13 +1083,15 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     const unsigned max_grid = (unsigned)ctx->sm_count * 16;
     // opacity maps: the traversal kernels with the candidate-hit filter (flat scenes)
     const bool alpha = scene->any_opacity;
-    // and the variants of trees too deep for the 4-wide view
-    const auto ext_kernel = scene->deep ? (alpha ? k_extend_pt<false, true, true> : k_extend_pt<false, false, true>)
-                                        : (alpha ? k_extend_pt<false, true> : k_extend_pt<false>);
+    // and the variants of trees too deep for the 4-wide view, and of scenes whose closest hits take the exact steps
+    const auto exact_kernel = alpha ? k_extend_pt<false, true, true> : k_extend_pt<false, false, true>;
+    const auto view_kernel = alpha ? k_extend_pt<false, true> : k_extend_pt<false>;
+    bool exact = scene->deep || scene->coincident;
     const auto shadow_kernel = scene->deep ? (alpha ? k_shadow_pt<false, true, true> : k_shadow_pt<false, false, true>)
                                            : (alpha ? k_shadow_pt<false, true> : k_shadow_pt<false>);
     const unsigned ext_grid = scene->n_instances ? resident_grid(k_extend_inst_pt, 128, ctx->sm_count)
-                                                 : resident_grid(ext_kernel, 128, ctx->sm_count);
+                                                 : std::min(resident_grid(exact_kernel, 128, ctx->sm_count),
+                                                            resident_grid(view_kernel, 128, ctx->sm_count));
     const unsigned shadow_grid = scene->n_instances ? resident_grid(k_shadow_inst_pt, 128, ctx->sm_count)
                                                     : resident_grid(shadow_kernel, 128, ctx->sm_count);
     const auto ext_group = alpha ? k_extend_group<false, true> : k_extend_group<>;
@@ -1122,7 +1133,8 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             // are launched and choose
             const bool can_group = !scene->n_instances && !scene->deep;
             const bool short_queue = can_group && count <= KS_GROUP_RAYS;
-            const bool ext_choose = can_group && !short_queue && count_ptr && count <= 16 * KS_GROUP_RAYS;
+            const bool ext_group_only = short_queue && !exact;
+            const bool ext_choose = can_group && !exact && !short_queue && count_ptr && count <= 16 * KS_GROUP_RAYS;
             const bool shadow_choose = can_group && !short_queue && count <= 16 * KS_GROUP_RAYS;
             const unsigned group_grid = std::min<unsigned>((count + 3) / 4, ext_group_grid);
             cudaEventRecord(f.ev[1], st);
@@ -1130,17 +1142,16 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                 k_extend_inst_pt<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[f.cur], count, count_ptr, w.hits.ptr,
                                                                            w.hit_inst.ptr, cnt + 4, w.overflow.ptr,
                                                                            work.ptr);
-            else if (!short_queue)
-                ext_kernel<<<std::min(grid, ext_grid), 128, 0, st>>>(sv, pb[f.cur], count, count_ptr, ext_choose,
-                                                                     w.hits.ptr, cnt + 4, w.overflow.ptr, work.ptr,
-                                                                     BatchView{});
-            if (short_queue || ext_choose)
+            else if (!ext_group_only)
+                (exact ? exact_kernel : view_kernel)<<<std::min(grid, ext_grid), 128, 0, st>>>(
+                    sv, pb[f.cur], count, count_ptr, ext_choose, w.hits.ptr, cnt + 4, w.overflow.ptr, work.ptr, BatchView{});
+            if (ext_group_only || ext_choose)
                 ext_group<<<group_grid, kTravBlock, 0, st>>>(sv, pb[f.cur], count, count_ptr, ext_choose, w.hits.ptr,
                                                              work.ptr, BatchView{});
             (split ? k_build_queues<false, true> : k_build_queues<false>)<<<std::min((count + 255) / 256, max_grid), 256, 0,
                                                                              st>>>(
                 sv, pb[f.cur], w.hits.ptr, count, count_ptr, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, alpha,
-                w.split.ptr, w.capacity, cnt + 8, BatchView{});
+                w.split.ptr, w.capacity, cnt + 8, cnt + 12, BatchView{});
             stats.kernel_launches++;
             cudaEventRecord(f.ev[2], st);
             if (guiding) {
@@ -1202,9 +1213,9 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                                                                 d_weights, work.ptr + 2, gv, BatchView{});
             stats.kernel_launches += 5u + ext_choose + shadow_choose;
             cudaEventRecord(f.ev[4], st);
-            cudaMemcpyAsync(f.h_counts, cnt, sizeof(uint32_t) * 2, cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(f.h_counts, cnt, sizeof(uint32_t) * kCounters, cudaMemcpyDeviceToHost, st);
             if (guiding)
-                cudaMemcpyAsync(f.h_counts + 2, gw.gcount.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+                cudaMemcpyAsync(f.h_counts + kCounters, gw.gcount.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
             cudaEventRecord(f.done, st);
             err = cudaGetLastError();
         };
@@ -1221,7 +1232,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             if (guiding) {
                 cudaEventElapsedTime(&ms, f.g0, f.g1);
                 stats.ms_guide_infer += ms;
-                stats.guide_rows += f.h_counts[2];
+                stats.guide_rows += f.h_counts[kCounters];
             }
             cudaEventElapsedTime(&ms, f.ev[5], f.ev[3]);
             stats.ms_shade += ms;
@@ -1229,6 +1240,11 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             stats.ms_shadow += ms;
             stats.shadow_rays += f.h_counts[1];
             stats.iterations++;
+            const uint32_t again = f.h_counts[12];
+            if (!exact && again >= kAgainMin && again > f.bound / kAgainShare && make_wide_steps(scene) == cudaSuccess) {
+                exact = scene->coincident = true;
+                sv.wide_steps = scene->wide_steps.ptr;
+            }
         };
         Flight *pending = nullptr;
         while (err == cudaSuccess) {
@@ -1487,7 +1503,7 @@ static void batch_iteration(ks_context *ctx, BatchWork &w, const BatchView &bv, 
     const bool split = w.split.ptr != nullptr;
     (split ? k_build_queues<true, true> : k_build_queues<true>)<<<grid, 256, 0, st>>>(
         SceneView{}, pb[cur], w.hits.ptr, 0u, nullptr, w.queue[0].ptr, w.queue[1].ptr, cnt + 2, w.overflow.ptr, 0, w.split.ptr,
-        capacity, cnt + 8, bv);
+        capacity, cnt + 8, cnt + 12, bv);
     launch_sample(true, grid, st, SceneView{}, RenderParams{}, pb[cur], w.hits.ptr, nullptr, w.queue[0].ptr, cnt + 2,
                   w.samples.ptr, bv);
     auto shade = [&](bool miss, int kernel_variant, const uint32_t *queue, const uint32_t *n) {

@@ -1277,11 +1277,56 @@ static ks_status build_wide4(ks_context *ctx, BuildScratch &bs, const TravNode *
     return KS_OK;
 }
 
+// The exact traversal's 4-wide steps: wide node i holds the children of interior node i, each interior child
+// replaced by its own two children (2 to 4 slots, in order).
 __global__ void k_widen(const TravNode *nodes, uint32_t n, WideNode *wide)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        wide[i] = widen(reinterpret_cast<const LazyWide *>(nodes), i);
+    if (i >= n)
+        return;
+    WideNode w;
+    for (int a = 0; a < 3; ++a) {
+        w.lo[a] = make_float4(kInf, kInf, kInf, kInf); // unused slots: an empty box, never hit
+        w.hi[a] = make_float4(-kInf, -kInf, -kInf, -kInf);
+    }
+    w.ref = make_uint4(kLeafBit, kLeafBit, kLeafBit, kLeafBit);
+    w.pad = make_uint4(0, 0, 0, 0);
+    float *lo = reinterpret_cast<float *>(w.lo), *hi = reinterpret_cast<float *>(w.hi);
+    uint32_t *ref = reinterpret_cast<uint32_t *>(&w.ref);
+    int m = 0;
+    auto put = [&](const TravNode &nd, int side) {
+        const float4 A = nd.a, B = nd.b, C = nd.c;
+        const float l0[3] = {A.x, A.y, A.z}, h0[3] = {A.w, B.x, B.y};
+        const float l1[3] = {B.z, B.w, C.x}, h1[3] = {C.y, C.z, C.w};
+        for (int a = 0; a < 3; ++a) {
+            lo[4 * a + m] = side ? l1[a] : l0[a];
+            hi[4 * a + m] = side ? h1[a] : h0[a];
+        }
+        ref[m] = side ? nd.d.y : nd.d.x;
+        ++m;
+    };
+    const TravNode nd = nodes[i];
+    for (int side = 0; side < 2; ++side) {
+        const uint32_t r = side ? nd.d.y : nd.d.x;
+        if (r & kLeafBit) {
+            put(nd, side);
+        } else {
+            const TravNode c = nodes[r];
+            put(c, 0);
+            put(c, 1);
+        }
+    }
+    wide[i] = w;
+}
+
+cudaError_t make_wide_steps(ks_scene *scene)
+{
+    const cudaError_t e = scene->wide_steps.alloc(scene->n_trav > 0 ? scene->n_trav : 1);
+    if (e != cudaSuccess || scene->n_trav == 0)
+        return e;
+    k_widen<<<grid_for(scene->n_trav, 256), 256, 0, scene->ctx->stream>>>(scene->trav_nodes.ptr, scene->n_trav,
+                                                                          scene->wide_steps.ptr);
+    return cudaGetLastError();
 }
 
 // BLAS concatenation: interior refs move by the node base, leaf refs by the slot base.
@@ -1549,16 +1594,15 @@ ks_status build_sbvh(ks_scene *scene, const ks_sbvh_options &o, float *build_ms)
             scene->root_ref = r.n_trav > 0 ? 0u : kLeafBit;
             // the renderer's 4-wide view of the tree, or the exact traversal's steps (timed with the build)
             scene->deep = r.n_levels > kMaxBinaryLevels;
+            scene->coincident = false;
             scene->wide_nodes.release();
             scene->wide_steps.release();
             cudaEventRecord(ev2, st);
             if (!scene->deep) {
                 s = build_wide4(ctx, build_scratch(ctx), scene->trav_nodes.ptr, r.n_trav, scene->root_ref, r.bound,
                                 r.n_levels, scene->wide_nodes);
-            } else if (scene->wide_steps.alloc(r.n_trav) != cudaSuccess) {
+            } else if (make_wide_steps(scene) != cudaSuccess) {
                 s = fail(ctx, KS_ERR_OUT_OF_MEMORY, "ks_scene_build_bvh: wide nodes");
-            } else {
-                k_widen<<<grid_for(r.n_trav, 256), 256, 0, st>>>(scene->trav_nodes.ptr, r.n_trav, scene->wide_steps.ptr);
             }
             cudaEventRecord(ev3, st);
             widened = s == KS_OK;

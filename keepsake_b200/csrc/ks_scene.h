@@ -128,8 +128,9 @@ struct ks_scene
     // traversal layout
     ksb::DevBuf<ksb::TravNode> trav_nodes;
     ksb::DevBuf<ksb::Wide4Node> wide_nodes; // flat scenes: the renderer's 4-wide view of trav_nodes
-    ksb::DevBuf<ksb::WideNode> wide_steps;  // instanced and deep scenes: 4-wide steps over trav_nodes
+    ksb::DevBuf<ksb::WideNode> wide_steps;  // instanced, deep and coincident scenes: 4-wide steps over trav_nodes
     ksb::DevBuf<float4> leaf_box; // per leaf, at its first primitive slot: its box (2 float4: lower, upper corner)
+    bool coincident = false; // closest hits by the exact steps too: many rays meet two surfaces at one distance
     bool deep = false; // the tree is too deep for the view's stack: the exact traversal over wide_steps
     ksb::DevBuf<float4> prim_tris; // 3 float4 per primitive slot: v0 (+tri index bits in w), v1, v2
     uint32_t n_trav = 0;
@@ -201,6 +202,8 @@ struct ks_scene
 namespace ksb
 {
 bool material_to_gpu(const ks_material_desc &m, MaterialGPU &g);
+// Makes scene->wide_steps from its binary nodes, on the context's stream.
+cudaError_t make_wide_steps(ks_scene *scene);
 ks_status build_sbvh(ks_scene *scene, const ks_sbvh_options &opts, float *build_ms);
 ks_status build_lights(ks_scene *scene);
 }

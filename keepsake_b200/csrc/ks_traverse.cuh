@@ -444,60 +444,11 @@ static __device__ __noinline__ WideHits wide_slabs_guarded(const WideNode *n, f3
     return h;
 }
 
-// Interior step of the 4-wide view (WideNode): the slots' boxes are tested with the same slab test,
-// the ray descends into the nearest hit slot (smallest entry time, then lowest slot) and the other
-// hit slots are pushed farthest first, each with its entry time (re-checked against tmax when
-// popped, as in trav_interior); any-hit queries take them in slot order.  Returns 1 / 0 / -1 like
-// trav_interior.  The set of leaves a closest-hit ray can reach is that of the binary tree (a
-// slot's slab interval lies inside its parent's: same operations, monotone rounding), so the
-// closest hit is the binary traversal's up to the order of exact ties.
-// The step is bound by the instructions it issues, so the arithmetic of slab() is laid out for few:
-// entry and exit planes are picked by address instead of by selects, the running maximum and
-// minimum of slab() are one max and one min over the axes (equal for boxes with lo <= hi), and the
-// 0 * inf guard, which changes nothing while every 1 / d is finite, is a path of its own.  With ranks
-// instead of a sorting network over four values per slot and 8-byte stack entries the mesh frame
-// (1.3 M triangles, 1024 x 1024 x 64) went from 101.9 to 93.5 ms, the instanced one (1080p x 4) from
-// 41.3 to 38.0 ms, every image bit for bit the same.
-// kGlobal: the node lies in global memory (else it was just made, LazyWide).
-template <bool kAnyHit, bool kGlobal, class Stack>
-KS_D int trav_wide(const WideNode *wide, TravState &s, Stack &stack, int &overflow, TravCount *count)
+// The second half of a 4-wide step: into the first slot hit, the others onto the stack.
+template <bool kAnyHit, class Stack>
+KS_D int trav_descend(const float (&t0)[4], const bool (&ok)[4], const uint32_t (&refs)[4], TravState &s, Stack &stack,
+                      int &overflow)
 {
-    const char *n = reinterpret_cast<const char *>(wide);
-    if (count)
-        count->nodes += kGlobal ? 2 : 3; // 64-byte node units (made: of the node and two children)
-    auto load = [](const auto *p) {
-        if constexpr (kGlobal)
-            return __ldg(p);
-        else
-            return *p;
-    };
-    const uint4 ref4 = load(reinterpret_cast<const uint4 *>(n + 96));
-    const uint32_t refs[4] = {ref4.x, ref4.y, ref4.z, ref4.w};
-    float t0[4];
-    bool ok[4];
-    if (!s.guard) {
-        auto plane = [&](int off) { return load(reinterpret_cast<const float4 *>(n + off)); };
-        const float4 ax = plane(s.px), ay = plane(s.py), az = plane(s.pz);
-        const float4 bx = plane(48 - s.px), by = plane(80 - s.py), bz = plane(112 - s.pz);
-        const float ex[4] = {ax.x, ax.y, ax.z, ax.w}, ey[4] = {ay.x, ay.y, ay.z, ay.w}, ez[4] = {az.x, az.y, az.z, az.w};
-        const float lx[4] = {bx.x, bx.y, bx.z, bx.w}, ly[4] = {by.x, by.y, by.z, by.w}, lz[4] = {bz.x, bz.y, bz.z, bz.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float t_in = fmaxf(fmaxf((ex[k] - s.ray.o.x) * s.inv.x, (ey[k] - s.ray.o.y) * s.inv.y),
-                                     (ez[k] - s.ray.o.z) * s.inv.z);
-            const float t_out = fminf(fminf((lx[k] - s.ray.o.x) * s.inv.x, (ly[k] - s.ray.o.y) * s.inv.y),
-                                      (lz[k] - s.ray.o.z) * s.inv.z);
-            ok[k] = t_in <= t_out && t_out > s.ray.tmin && t_in < s.ray.tmax;
-            t0[k] = t_in;
-        }
-    } else {
-        const WideHits h = wide_slabs_guarded(wide, s.ray.o, s.inv, s.ray.tmin, s.ray.tmax);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            ok[k] = (h.ok >> k) & 1u;
-            t0[k] = h.t[k];
-        }
-    }
     const int n_hit = (int)ok[0] + (int)ok[1] + (int)ok[2] + (int)ok[3];
     if (n_hit == 0)
         return 0;
@@ -541,6 +492,56 @@ KS_D int trav_wide(const WideNode *wide, TravState &s, Stack &stack, int &overfl
     return 1;
 }
 
+// Interior step of the 4-wide view (WideNode): the slots' boxes are tested with the same slab test,
+// the ray descends into the nearest hit slot (smallest entry time, then lowest slot) and the other
+// hit slots are pushed farthest first, each with its entry time (re-checked against tmax when
+// popped, as in trav_interior); any-hit queries take them in slot order.  Returns 1 / 0 / -1 like
+// trav_interior.  The set of leaves a closest-hit ray can reach is that of the binary tree (a
+// slot's slab interval lies inside its parent's: same operations, monotone rounding), so the
+// closest hit is the binary traversal's up to the order of exact ties.
+// The step is bound by the instructions it issues, so the arithmetic of slab() is laid out for few:
+// entry and exit planes are picked by address instead of by selects, the running maximum and
+// minimum of slab() are one max and one min over the axes (equal for boxes with lo <= hi), and the
+// 0 * inf guard, which changes nothing while every 1 / d is finite, is a path of its own.  With ranks
+// instead of a sorting network over four values per slot and 8-byte stack entries the mesh frame
+// (1.3 M triangles, 1024 x 1024 x 64) went from 101.9 to 93.5 ms, the instanced one (1080p x 4) from
+// 41.3 to 38.0 ms, every image bit for bit the same.
+template <bool kAnyHit, class Stack>
+KS_D int trav_wide(const WideNode *wide, TravState &s, Stack &stack, int &overflow, TravCount *count)
+{
+    const char *n = reinterpret_cast<const char *>(wide);
+    if (count)
+        count->nodes += 2; // 64-byte node units
+    const uint4 ref4 = __ldg(reinterpret_cast<const uint4 *>(n + 96));
+    const uint32_t refs[4] = {ref4.x, ref4.y, ref4.z, ref4.w};
+    float t0[4];
+    bool ok[4];
+    if (!s.guard) {
+        auto plane = [&](int off) { return __ldg(reinterpret_cast<const float4 *>(n + off)); };
+        const float4 ax = plane(s.px), ay = plane(s.py), az = plane(s.pz);
+        const float4 bx = plane(48 - s.px), by = plane(80 - s.py), bz = plane(112 - s.pz);
+        const float ex[4] = {ax.x, ax.y, ax.z, ax.w}, ey[4] = {ay.x, ay.y, ay.z, ay.w}, ez[4] = {az.x, az.y, az.z, az.w};
+        const float lx[4] = {bx.x, bx.y, bx.z, bx.w}, ly[4] = {by.x, by.y, by.z, by.w}, lz[4] = {bz.x, bz.y, bz.z, bz.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float t_in = fmaxf(fmaxf((ex[k] - s.ray.o.x) * s.inv.x, (ey[k] - s.ray.o.y) * s.inv.y),
+                                     (ez[k] - s.ray.o.z) * s.inv.z);
+            const float t_out = fminf(fminf((lx[k] - s.ray.o.x) * s.inv.x, (ly[k] - s.ray.o.y) * s.inv.y),
+                                      (lz[k] - s.ray.o.z) * s.inv.z);
+            ok[k] = t_in <= t_out && t_out > s.ray.tmin && t_in < s.ray.tmax;
+            t0[k] = t_in;
+        }
+    } else {
+        const WideHits h = wide_slabs_guarded(wide, s.ray.o, s.inv, s.ray.tmin, s.ray.tmax);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ok[k] = (h.ok >> k) & 1u;
+            t0[k] = h.t[k];
+        }
+    }
+    return trav_descend<kAnyHit>(t0, ok, refs, s, stack, overflow);
+}
+
 // Interior step for either tree layout.
 template <bool kAnyHit, class Stack>
 KS_D int trav_node(const TravNode *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
@@ -548,59 +549,58 @@ KS_D int trav_node(const TravNode *__restrict__ nodes, TravState &s, Stack &stac
 {
     return trav_interior(nodes, s, stack, overflow, count);
 }
-// The 4-wide view of binary nodes, made when a node is visited: wide node i holds the children of
-// interior node i, each interior child replaced by its own two children (2 to 4 slots, in order).
+// The same steps over the binary nodes themselves, each interior child's node read beside its parent's: slower, for
+// the few rays that are traced again.
 struct LazyWide
 {
     TravNode node;
 };
-KS_D WideNode widen(const LazyWide *__restrict__ nodes, uint32_t i)
-{
-    WideNode w;
-    for (int a = 0; a < 3; ++a) {
-        w.lo[a] = make_float4(kInf, kInf, kInf, kInf); // unused slots: an empty box, never hit
-        w.hi[a] = make_float4(-kInf, -kInf, -kInf, -kInf);
-    }
-    w.ref = make_uint4(kLeafBit, kLeafBit, kLeafBit, kLeafBit);
-    float *lo = reinterpret_cast<float *>(w.lo), *hi = reinterpret_cast<float *>(w.hi);
-    uint32_t *ref = reinterpret_cast<uint32_t *>(&w.ref);
-    int m = 0;
-    auto put = [&](const TravNode &nd, int side) {
-        const float4 A = nd.a, B = nd.b, C = nd.c;
-        const float l0[3] = {A.x, A.y, A.z}, h0[3] = {A.w, B.x, B.y};
-        const float l1[3] = {B.z, B.w, C.x}, h1[3] = {C.y, C.z, C.w};
-        for (int a = 0; a < 3; ++a) {
-            lo[4 * a + m] = side ? l1[a] : l0[a];
-            hi[4 * a + m] = side ? h1[a] : h0[a];
-        }
-        ref[m] = side ? nd.d.y : nd.d.x;
-        ++m;
-    };
-    const TravNode nd = nodes[i].node;
-    for (int side = 0; side < 2; ++side) {
-        const uint32_t r = side ? nd.d.y : nd.d.x;
-        if (r & kLeafBit) {
-            put(nd, side);
-        } else {
-            const TravNode c = nodes[r].node;
-            put(c, 0);
-            put(c, 1);
-        }
-    }
-    return w;
-}
 template <bool kAnyHit, class Stack>
 KS_D int trav_node(const LazyWide *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
                    TravCount *count)
 {
-    const WideNode w = widen(nodes, s.ref);
-    return trav_wide<kAnyHit, false>(&w, s, stack, overflow, count);
+    if (count)
+        count->nodes += 3; // 64-byte node units: the node and two children
+    const BoxHelper bh = box_helper_of(s.inv);
+    float t0[4];
+    bool ok[4];
+    uint32_t refs[4];
+    auto test = [&](int k, const float4 &A, const float4 &B, const float4 &C, int side) {
+        const float bmin[3] = {side ? B.z : A.x, side ? B.w : A.y, side ? C.x : A.z};
+        const float bmax[3] = {side ? C.y : A.w, side ? C.z : B.x, side ? C.w : B.y};
+        float t1;
+        ok[k] = slab(s.ray, bh, bmin, bmax, t0[k], t1) && t1 > s.ray.tmin && t0[k] < s.ray.tmax;
+    };
+    const TravNode *n = &nodes[s.ref].node;
+    const float4 A = __ldg(&n->a), B = __ldg(&n->b), C = __ldg(&n->c);
+    const uint4 D = __ldg(&n->d);
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const uint32_t r = side ? D.y : D.x;
+        const int k = 2 * side;
+        if (r & kLeafBit) {
+            test(k, A, B, C, side);
+            refs[k] = r;
+            ok[k + 1] = false;
+            t0[k + 1] = kInf;
+            refs[k + 1] = kLeafBit;
+        } else {
+            const TravNode *c = &nodes[r].node;
+            const float4 X = __ldg(&c->a), Y = __ldg(&c->b), Z = __ldg(&c->c);
+            const uint4 W = __ldg(&c->d);
+            test(k, X, Y, Z, 0);
+            test(k + 1, X, Y, Z, 1);
+            refs[k] = W.x;
+            refs[k + 1] = W.y;
+        }
+    }
+    return trav_descend<kAnyHit>(t0, ok, refs, s, stack, overflow);
 }
 template <bool kAnyHit, class Stack>
 KS_D int trav_node(const WideNode *__restrict__ nodes, TravState &s, Stack &stack, int &overflow,
                    TravCount *count)
 {
-    return trav_wide<kAnyHit, true>(nodes + s.ref, s, stack, overflow, count);
+    return trav_wide<kAnyHit>(nodes + s.ref, s, stack, overflow, count);
 }
 
 // Pops the next node whose entry time is below the current tmax; false when the stack is empty.

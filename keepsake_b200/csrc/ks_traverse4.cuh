@@ -12,8 +12,10 @@
 //     traversal tests the triangle at all (a leaf's box passes only if every box above it does);
 //   * which of several hits is the closest does not depend on the visiting order unless two of them
 //     are nearly equally far: within rounding of each other, or one nearer than the other's box is
-//     entered.  Trav4 keeps what is needed to see that, and such a ray (about one in a million) is
-//     traced again in the exact traversal's order (retrace).
+//     entered.  Within a leaf the order is the exact traversal's; where two leaves are concerned Trav4 keeps
+//     what is needed to see it, and such a ray is traced again in the exact traversal's order (retrace).
+//     That is about one ray in a million of the mesh frame (no two surfaces in one plane); a scene with
+//     many goes over to the exact steps (kAgainShare).
 // Trees too deep for the stack keep the exact traversal, whose stack overflow is an error status, and so do
 // instanced scenes: beside the state of their upper level this one's does not fit the registers (closest hit
 // over 400 instances at 1080p x 4: 22.0 ms by the exact traversal, 23.8 by this one at its best).
@@ -239,13 +241,30 @@ KS_D bool leaf_reached(const float4 *__restrict__ leaf_box, const Trav4 &s, uint
     return slab(s.ray, exact_helper(s), bmin, bmax, entry, t1) && t1 > s.ray.tmin && entry < s.ray.tmax;
 }
 
-// Takes note of a closest-hit ray's hit on a triangle of a leaf that the ray enters at `entry`.
-KS_D void trav4_take(Trav4 &s, const Hit &h, float entry)
+// Whether the hit at hand is one of the leaf that starts at `first`, of which `slot` is tested.
+KS_D bool in_leaf(const Trav4 &s, uint32_t first, uint32_t slot)
+{
+    return s.hit.tri != ~0u && s.hit.slot >= first && s.hit.slot < slot;
+}
+
+// The range in which primitive `slot` of a leaf is tested.  After a hit in the same leaf it ends there, as in
+// the exact traversal: the order within a leaf is the same, so which of a leaf's nearly equal hits stays
+// (a mesh given twice has its copies in one leaf) is no question of the order of leaves.
+KS_D RayQuery leaf_range(const Trav4 &s, uint32_t first, uint32_t slot)
+{
+    RayQuery q = s.ray;
+    q.tmax = in_leaf(s, first, slot) ? s.hit.t : fminf(q.tmax, s.limit);
+    return q;
+}
+
+// Takes note of a closest-hit ray's hit on a triangle of a leaf that starts at `first` and that the ray enters
+// at `entry`.
+KS_D void trav4_take(Trav4 &s, const Hit &h, float entry, uint32_t first)
 {
     if (h.tri == s.hit.tri) {
         s.entry = fminf(s.entry, entry); // the same triangle through another of its leaves
     } else if (s.hit.tri == ~0u || h.t < s.hit.t) {
-        if (s.hit.tri != ~0u)
+        if (s.hit.tri != ~0u && !in_leaf(s, first, h.slot))
             s.second = fminf(s.second, s.hit.t);
         s.entry = entry;
         s.limit = fminf(s.limit, h.t + fabsf(h.t) * kPruneSlack);
@@ -271,8 +290,7 @@ KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restri
         last = __float_as_uint(b.w) != 0u;
         const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
         const uint32_t tri = __float_as_uint(a.w);
-        RayQuery q = s.ray;
-        q.tmax = fminf(q.tmax, s.limit);
+        const RayQuery q = kAnyHit ? s.ray : leaf_range(s, first, slot);
         float t, b0, b1, b2;
         if (!cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, t, b0, b1, b2)) {
             float entry;
@@ -282,7 +300,7 @@ KS_D bool trav4_leaf(const float4 *__restrict__ leaf_box, const float4 *__restri
                     return true;
                 }
             } else if (t < q.tmax && leaf_reached(leaf_box, s, first, entry) && alpha(tri, b1, b2, s.ray)) {
-                trav4_take(s, Hit{tri, slot, t, b0, b1, b2}, entry);
+                trav4_take(s, Hit{tri, slot, t, b0, b1, b2}, entry, first);
             }
         }
         ++slot;
@@ -376,18 +394,19 @@ KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 
                 last = ends != 0u;
                 const bool mine = !last || (int)k < __ffs(ends);
                 const f3 v0 = mk(a.x, a.y, a.z), v1 = mk(b.x, b.y, b.z), v2 = mk(c.x, c.y, c.z);
-                RayQuery q = s.ray;
-                q.tmax = fminf(q.tmax, s.limit);
                 Hit h;
                 h.tri = __float_as_uint(a.w);
                 h.slot = slot;
                 float entry = 0.0f;
                 bool take = false;
+                auto test = [&]() {
+                    const RayQuery q = kAnyHit ? s.ray : leaf_range(s, first, slot);
+                    return !cull_tri(q, v0, v1, v2, culling) &&
+                           isect_tri(q, s.th, v0, v1, v2, h.t, h.b0, h.b1, h.b2) && (kAnyHit || h.t < q.tmax);
+                };
                 if (mine) {
                     count->tris++;
-                    take = !cull_tri(q, v0, v1, v2, culling) && isect_tri(q, s.th, v0, v1, v2, h.t, h.b0, h.b1, h.b2) &&
-                           (kAnyHit || h.t < q.tmax) && leaf_reached(tree.leaf_box, s, first, entry) &&
-                           alpha(h.tri, h.b1, h.b2, s.ray);
+                    take = test() && leaf_reached(tree.leaf_box, s, first, entry) && alpha(h.tri, h.b1, h.b2, s.ray);
                 }
                 uint32_t found = (__ballot_sync(mask, take) >> shift) & ((1u << kGroup) - 1u);
                 if constexpr (kAnyHit) {
@@ -396,7 +415,7 @@ KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 
                         return;
                     }
                 } else {
-                    for (; found; found &= found - 1u) { // in the leaf's order, as one lane would
+                    while (found) { // in the leaf's order, as one lane would
                         const int src = (int)(shift + __ffs(found) - 1u);
                         Hit g;
                         g.tri = __shfl_sync(mask, h.tri, src);
@@ -405,9 +424,12 @@ KS_D void group_trace(const Tree4 &tree, const float4 *__restrict__ tris, Trav4 
                         g.b0 = __shfl_sync(mask, h.b0, src);
                         g.b1 = __shfl_sync(mask, h.b1, src);
                         g.b2 = __shfl_sync(mask, h.b2, src);
-                        const float at = __shfl_sync(mask, entry, src);
-                        if (g.t < s.limit)
-                            trav4_take(s, g, at);
+                        trav4_take(s, g, __shfl_sync(mask, entry, src), first);
+                        found &= found - 1u;
+                        if (found) {
+                            const bool later = (found >> k) & 1u;
+                            found = (__ballot_sync(mask, later && test()) >> shift) & ((1u << kGroup) - 1u);
+                        }
                     }
                 }
                 base += kGroup;

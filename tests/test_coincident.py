@@ -1,0 +1,120 @@
+"""Scenes in which many rays meet two surfaces at one distance: meshes given twice, whose copies share a leaf,
+and walls with a second layer in their plane, of other triangles and so of other leaves.  Which surface is
+hit depends on the visiting order there; a ray of the 4-wide view that meets that case is traced again in
+the exact traversal's order, and a scene with many is traced by the exact steps from then on.
+
+All ways give the same hits, so images differ by the order of FP64 additions only.  And the closest hits
+cost what the surfaces cost: within twice the ratio that the exact traversal alone had to the scene without
+the second layer (1.2 for the copies, 2.4 for the layers; traced again ray by ray, 4 and 10)."""
+import numpy as np
+import pytest
+
+W, H = 256, 160
+
+
+def base(ks, kind):
+    if kind == "copies":
+        g = ks.Generated("icosphere", 0, level=7, sky=(64, 32), resolution=(W, H))
+    else:
+        g = ks.Generated("box_room", 0)
+    meshes = [[m["vertices"].copy(), m["indices"], m["material"], dict(twosided=m["twosided"])] for m in g.meshes]
+    return g, meshes, list(g.materials)
+
+
+def layer(v, n):
+    """A wall's plane as n x n squares of two triangles."""
+    x, y = np.meshgrid(np.linspace(0, 1, n + 1), np.linspace(0, 1, n + 1))
+    p = (v[0] + x[..., None] * (v[1] - v[0]) + y[..., None] * (v[3] - v[0])).reshape(-1, 3).astype(np.float32)
+    i = (np.arange(n)[:, None] * (n + 1) + np.arange(n)).reshape(-1)
+    idx = np.concatenate([np.stack([i, i + 1, i + n + 1], -1), np.stack([i + 1, i + n + 2, i + n + 1], -1)])
+    return p, idx.astype(np.uint32)
+
+
+def scene(ctx, ks, kind, twice, opacity=False):
+    g, meshes, mats = base(ks, kind)
+    once = list(meshes)
+    if twice and kind == "copies":
+        meshes = once + once
+    elif twice:
+        for k in range(5):
+            p, idx = layer(once[k][0], 60)
+            uv = np.stack(np.meshgrid(np.linspace(0, 1, 61), np.linspace(0, 1, 61)), -1).reshape(-1, 2).astype(np.float32)
+            mats.append(ks.MaterialDesc(tuple(mats[once[k][2]].basecolor), 0.7, 0.0, 1.5, 0.5, 0.0, 0.0, 0.5, (0, 0, 0), 0, 0,
+                                        (0, 0, 0)))
+            meshes.append([p, idx, len(mats) - 1, dict(twosided=1, texcoords=uv)])
+    desc, keep = ks.scene_desc(meshes, mats, g.desc.contents.sky)
+    if opacity:
+        ys, xs = np.mgrid[0:16, 0:16]
+        mask = (((xs // 4 + ys // 4) % 3) * 0.5).astype(np.float32)[..., None]
+        keep += ks.attach_textures(desc, [(mask, False)], [ks.TextureBinding.make(m, "opacity_map", 0, filter=0)
+                                                           for m in range(len(mats) - 5, len(mats))])
+    s = ks.Scene(ctx, desc, keepalive=(g, keep))
+    s.build_bvh()
+    return s, ks.camera_perspective(g.camera_to_world, g.vfov, W / H)
+
+
+def params(ks, **kw):
+    size = dict(render_width=W, render_height=H, spp=2, bounces=5, clamp_indirect=0.0)
+    size.update(kw)
+    return ks.SmallPTParams.make(**size)
+
+
+def same(a, b):
+    # sums of at most some 30 terms in another order
+    assert np.array_equal(a[1], b[1]) and np.allclose(a[0], b[0], rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.gpu
+def test_a_mesh_given_twice(ctx):
+    import keepsake_b200 as ks
+    images = []
+    for twice in (False, True):
+        s, cam = scene(ctx, ks, "copies", twice)
+        images.append(s.render(cam, params(ks)))
+        s.close()
+    assert images[0][0].sum() > 0
+    same(*images)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("opacity", [False, True])
+def test_layers_in_one_plane(ctx, opacity):
+    """The first render of a scene traces rays again, the second takes the exact steps; crops have short queues,
+    traced by groups of lanes in a scene that has rendered nothing else."""
+    import keepsake_b200 as ks
+    s, cam = scene(ctx, ks, "layers", True, opacity)
+    first = s.render(cam, params(ks))
+    second = s.render(cam, params(ks))
+    s.close()
+    assert first[0].sum() > 0
+    same(first, second)
+    s, cam = scene(ctx, ks, "layers", True, opacity)
+    a, w = np.zeros_like(first[0]), np.zeros_like(first[1])
+    for y in range(0, H, 40):
+        x, v = s.render(cam, params(ks, crop_start_x=0, crop_start_y=y, crop_width=W, crop_height=40))
+        a += x if x.shape == a.shape else np.pad(x, ((y, H - y - 40), (0, 0), (0, 0)))
+        w += v if v.shape == w.shape else np.pad(v, ((y, H - y - 40), (0, 0), (0, 0)))
+    s.close()
+    same(first, (a, w))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,limit", [("copies", 2.4), ("layers", 4.8)])
+def test_the_second_surface_costs_what_it_is(ctx, kind, limit):
+    import torch
+
+    import keepsake_b200 as ks
+    times = []
+    for twice in (False, True):
+        s, cam = scene(ctx, ks, kind, twice)
+        p = params(ks, render_width=512, render_height=512, spp=4)
+        acc = torch.zeros((512, 512, 3), dtype=torch.float64, device="cuda")
+        wts = torch.zeros((512, 512, 2), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        runs = []
+        for _ in range(6):
+            s.render_device(cam, p, acc.data_ptr(), wts.data_ptr())
+            runs.append(s.stats().ms_extend)
+        times.append(min(runs))
+        s.close()
+    assert times[1] < limit * times[0], times
