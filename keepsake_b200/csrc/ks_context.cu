@@ -65,10 +65,11 @@ cudaError_t staged_copy(ks_context *ctx, void *dst, const void *src, size_t byte
 {
     const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
     cudaStream_t st = ctx->stream;
-    if (bytes < kStageMin || ctx->stage.reserve(std::min(bytes, kStageBytes)) != cudaSuccess) {
+    if (bytes < (to_device ? kStageMinUp : kStageMinDown) ||
+        ctx->stage.reserve(std::min(bytes, kStageBytes)) != cudaSuccess) {
         cudaGetLastError();
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
-        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+        return e == cudaSuccess && !to_device ? cudaStreamSynchronize(st) : e;
     }
     cudaEvent_t done[kStageChunks] = {};
     cudaError_t err = cudaSuccess;

@@ -919,6 +919,7 @@ ks_status ks_guide_set_weights(ks_guide *g, const float *mlp_weights, const floa
     if (grid)
         KS_CUDA_TRY(g->ctx, staged_copy(g->ctx, g->grid.ptr, grid, g->grid.bytes(), true));
     g->packed = false;
+    KS_CUDA_TRY(g->ctx, cudaStreamSynchronize(g->ctx->stream));
     return KS_OK;
 }
 

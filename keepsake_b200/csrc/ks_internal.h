@@ -97,11 +97,15 @@ void host_parallel(size_t n, size_t grain, F &&f)
 }
 
 // Copies between the caller's (pageable) host memory and the device on the context's stream, through pinned
-// memory the context keeps, in kStageChunks pieces so that the link and the host threads' copies overlap;
-// the call returns when host memory is done with (a download: filled; an upload: read).  Small copies go
-// straight.  Pageable copies of 64 MB into new memory took the driver some 11 ms: one thread copying from its
-// own staging while it meets a page fault every 4 KB.
-constexpr size_t kStageBytes = (size_t)64 << 20, kStageChunks = 8, kStageMin = (size_t)1 << 20;
+// memory the context keeps, in kStageChunks pieces so that the link and the host threads' copies overlap.  A
+// download returns when it is there.  Host memory of an upload must stay until the stream is synchronised, which
+// every entry point does before it returns.  Small copies go straight.  Pageable downloads of 64 MB into new
+// memory took the driver some 11 ms: one thread copying from its own staging while it meets a page fault
+// every 4 KB.  An upload has no such faults, and through the stage it has to wait for its copy, which cost a
+// training step of 131072 rows (six arrays of up to 1.5 MB) 0.2 ms of 1.3.  Steps of 1 M rows (12 MB) 6.8 ms
+// straight and 7.5 through it, of 3 M rows (36 MB) 24.4 and 22.0.
+constexpr size_t kStageBytes = (size_t)64 << 20, kStageChunks = 8, kStageMinDown = (size_t)1 << 20,
+                 kStageMinUp = (size_t)32 << 20;
 cudaError_t staged_copy(ks_context *ctx, void *dst, const void *src, size_t bytes, bool to_device);
 
 // Records a failure on the context and returns its status.

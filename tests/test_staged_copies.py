@@ -1,5 +1,5 @@
-"""Host arrays of the guide's entry points go through pinned memory in pieces above 1 MB: what comes back
-is what was sent, whole and at sizes around the pieces' edges, and rows do not depend on how many are
+"""Host arrays of the guide's entry points go through pinned memory in pieces, downloads above 1 MB and uploads
+above 32 MB: what comes back is what was sent, whole and at sizes around the pieces' edges, and rows do not depend on how many are
 sent together (each row of the network is computed by itself)."""
 import numpy as np
 import pytest
@@ -34,4 +34,17 @@ def test_rows_are_independent_of_their_number(ctx, n):
     for k in at:
         part = guide.infer(pos[k:k + 128], wo[k:k + 128], normal[k:k + 128])
         assert np.array_equal(whole[k:k + 128], part)
+    guide.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2796202, 2796203])  # rows of 12 bytes up: below and above 32 MB
+def test_large_uploads(ctx, n):
+    import keepsake_b200 as ks
+    rng = np.random.default_rng(n)
+    pos, wo, normal = (rng.standard_normal((n, 3), dtype=np.float32) for _ in range(3))
+    guide = ks.Guide(ctx, BOUND)
+    whole = guide.infer(pos, wo, normal)
+    for k in (0, n // 2, n - 128):
+        assert np.array_equal(whole[k:k + 128], guide.infer(pos[k:k + 128], wo[k:k + 128], normal[k:k + 128]))
     guide.close()
