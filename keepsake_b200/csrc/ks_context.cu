@@ -65,7 +65,11 @@ cudaError_t staged_copy(ks_context *ctx, void *dst, const void *src, size_t byte
 {
     const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
     cudaStream_t st = ctx->stream;
-    if (bytes < (to_device ? kStageMinUp : kStageMinDown) ||
+    auto pinned = [](const void *host) {
+        cudaPointerAttributes at;
+        return cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    };
+    if (bytes < (to_device ? kStageMinUp : kStageMinDown) || pinned(to_device ? src : dst) ||
         ctx->stage.reserve(std::min(bytes, kStageBytes)) != cudaSuccess) {
         cudaGetLastError();
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);

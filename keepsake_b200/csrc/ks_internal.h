@@ -96,10 +96,11 @@ void host_parallel(size_t n, size_t grain, F &&f)
         t.join();
 }
 
-// Copies between the caller's (pageable) host memory and the device on the context's stream, through pinned
+// Copies between the caller's host memory and the device on the context's stream: pageable memory through pinned
 // memory the context keeps, in kStageChunks pieces so that the link and the host threads' copies overlap.  A
 // download returns when it is there.  Host memory of an upload must stay until the stream is synchronised, which
-// every entry point does before it returns.  Small copies go straight.  Pageable downloads of 64 MB into new
+// every entry point does before it returns.  Small copies go straight, and memory that the caller pinned (64 MB up
+// 1.24 ms, through the stage 3.1).  Pageable downloads of 64 MB into new
 // memory took the driver some 11 ms: one thread copying from its own staging while it meets a page fault
 // every 4 KB.  An upload has no such faults, and through the stage it has to wait for its copy, which cost a
 // training step of 131072 rows (six arrays of up to 1.5 MB) 0.2 ms of 1.3.  Steps of 1 M rows (12 MB) 6.8 ms
