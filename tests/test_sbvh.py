@@ -77,6 +77,15 @@ def test_builder_topology_options(ctx, opts):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [255, 256, 257, 512, 513])
+@pytest.mark.parametrize("buckets", [2, 12, 16])
+def test_builder_topology_spatial_splits(ctx, n, buckets):
+    """Spatial splits of nodes of one work item, exactly one, or one and a bit (256 references)."""
+    v, i = scenes.soup(n, seed=n, spread=2.0, size=1.5)
+    _check_build(ctx, v, i, buckets=buckets)
+
+
+@pytest.mark.gpu
 def test_builder_topology_box_room(ctx):
     import keepsake_b200 as ks
     g = ks.Generated("box_room", 0)

@@ -1,6 +1,7 @@
 """SBVH builder: nodes whose references are one work item, exactly one, or one and a bit (256 references per item,
-see KS_BUILD_CHUNK), and bucket counts below, at and above the lanes that evaluate a node's splits, against an object-split
-builder in NumPy fp32 (alpha = 1: no node overlaps more than the root's area, so none is split spatially).
+see KS_BUILD_CHUNK), and bucket counts up to the lanes that evaluate a node's splits (16, the most that a build
+takes: more are clamped), against an object-split builder in NumPy fp32 (alpha = 1: no node overlaps more than
+the root's area, so none is split spatially).
 Trees are equal: same nodes in depth-first order, bounds, axes, offsets and leaf contents."""
 import numpy as np
 import pytest
@@ -90,6 +91,21 @@ def check(ctx, n, buckets, seed, **kw):
 @pytest.mark.parametrize("buckets", [2, 12, 16])
 def test_object_splits(ctx, n, buckets):
     check(ctx, n, buckets, seed=n + buckets)
+
+
+@pytest.mark.gpu
+def test_more_buckets_than_lanes(ctx):
+    import keepsake_b200 as ks
+    v, i = scenes.soup(700, seed=9, spread=3.0, size=1.5)  # overlapping: spatial splits too
+    d, keep = ks.triangle_soup_desc(v, i)
+    s = ks.Scene(ctx, d, keep)
+    trees = []
+    for buckets in (16, 17, 40):
+        s.build_bvh(buckets=buckets)
+        trees.append(s.export_sbvh())
+    s.close()
+    for t in trees[1:]:
+        assert all(np.array_equal(t[k], trees[0][k]) for k in ("bounds", "axis", "right", "prim_offset"))
 
 
 @pytest.mark.gpu
