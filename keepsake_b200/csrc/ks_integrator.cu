@@ -1086,7 +1086,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
     // and the variants of trees too deep for the 4-wide view, and of scenes whose closest hits take the exact steps
     const auto exact_kernel = alpha ? k_extend_pt<false, true, true> : k_extend_pt<false, false, true>;
     const auto view_kernel = alpha ? k_extend_pt<false, true> : k_extend_pt<false>;
-    bool exact = scene->deep || scene->coincident;
+    bool exact = scene->deep || scene->coincident, may_go_exact = true;
     const auto shadow_kernel = scene->deep ? (alpha ? k_shadow_pt<false, true, true> : k_shadow_pt<false, false, true>)
                                            : (alpha ? k_shadow_pt<false, true> : k_shadow_pt<false>);
     const unsigned ext_grid = scene->n_instances ? resident_grid(k_extend_inst_pt, 128, ctx->sm_count)
@@ -1241,9 +1241,14 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             stats.shadow_rays += f.h_counts[1];
             stats.iterations++;
             const uint32_t again = f.h_counts[12];
-            if (!exact && again >= kAgainMin && again > f.bound / kAgainShare && make_wide_steps(scene) == cudaSuccess) {
-                exact = scene->coincident = true;
-                sv.wide_steps = scene->wide_steps.ptr;
+            if (!exact && may_go_exact && again >= kAgainMin && again > f.bound / kAgainShare) {
+                may_go_exact = make_wide_steps(scene) == cudaSuccess;
+                if (may_go_exact) {
+                    exact = scene->coincident = true;
+                    sv.wide_steps = scene->wide_steps.ptr;
+                } else {
+                    cudaGetLastError(); // no memory for them: as before
+                }
             }
         };
         Flight *pending = nullptr;
