@@ -685,7 +685,10 @@ def main():
     peak, peak_kind = measured_peaks()
     achieved_kernel = kernel_bytes / (ext_ms / 1e3) / 1e9
     tpq = profile_traffic()
-    roofline = {"kernel": "k_extend_pt (closest-hit SBVH traversal)", "bound": "hbm", "peak": peak,
+    roofline = {"kernel": "k_extend_pt (closest-hit SBVH traversal)", "bound": "issue + L1 data pipe",
+                "note": "achieved and frac: bytes fetched, most of them from L1 and L2, over the DRAM copy rate; "
+                        "dram_frac: DRAM traffic over it", "peak": peak,
+                "dram_frac": (tpq * ext_q / (ext_ms / 1e3) / 1e9 / peak) if tpq else None,
                 "peak_source": peak_kind, "unit": "GB/s",
                 "traffic": (tpq * ext_q / launches) if tpq else None,
                 "traffic_source": "profiles/k_extend_pt_icosphere_l8.json (ncu DRAM bytes per query x queries per "

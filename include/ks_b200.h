@@ -34,9 +34,11 @@ typedef struct ks_context ks_context;
 
 /* Context: one CUDA device + one stream.  (Replaces the reference's implicit global state:
  * EmbreeDevice in small_pt.cpp:182 and the TBB arena of parallel.h:93-113.)  The context keeps the
- * scratch of its SBVH builds and the buffers of its renders (wavefront state, about 300 bytes per
- * path slot up to 32 M slots, the accumulators and a pinned staging copy of them) from one call to
- * the next, and frees them in ks_context_destroy.  One thread at a time per context.
+ * scratch of its SBVH builds, the buffers of its renders (wavefront state, about 300 bytes per
+ * path slot up to 32 M slots, the accumulators and a pinned staging copy of them) and pinned staging
+ * for scene uploads and guide arrays (up to 64 MB for the latter) from one call to the next, and frees
+ * them in ks_context_destroy; a guide keeps its rows' device buffer (up to 256 MB) until
+ * ks_guide_destroy.  One thread at a time per context.
  * Device memory comes from a pool per GPU that keeps freed blocks for reuse (a scene destroyed
  * and a new one created reuse the same memory without the driver's allocator); ks_context_destroy
  * returns the pool's free blocks to the driver. */
@@ -309,10 +311,11 @@ ks_status ks_trace_rays(ks_scene *scene, const float *rays, uint32_t n, int any_
 
 /* The same queries through the renderer's traversal kernels.  Flat scenes: a 4-wide view of the
  * same SBVH with conservative boxes, nearest slot first; a hit counts when the exact slab test accepts
- * its leaf's box, so the result equals ks_trace_rays' except where two triangles are hit at
- * exactly the same distance (the visiting order then picks one of them).  Instanced scenes: the
- * persistent two-level traversal over the TLAS and 4-wide steps of the BLAS nodes, the same except
- * at exact ties.  Replaces the same reference calls as ks_trace_rays (cuda/sbvh.cu:512-603);
+ * its leaf's box.  Occlusion equals ks_trace_rays'; so does the closest hit, except where two
+ * triangles are hit within rounding of one another (the visiting order then picks one: distances
+ * agree within 8 ulp, or one part in 2^12 where a computed distance lies before its leaf's entry).
+ * Instanced scenes: the persistent two-level traversal over the TLAS and 4-wide steps of the BLAS
+ * nodes, the same but for such ties.  Replaces the same reference calls as ks_trace_rays (cuda/sbvh.cu:512-603);
  * exists to test the rendering traversal. */
 ks_status ks_trace_rays_wide(ks_scene *scene, const float *rays, uint32_t n, int any_hit, int culling,
                              uint32_t *tri_idx, float *t, float *bary);

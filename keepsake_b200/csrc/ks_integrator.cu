@@ -1094,6 +1094,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
                                                             resident_grid(view_kernel, 128, ctx->sm_count));
     const unsigned shadow_grid = scene->n_instances ? resident_grid(k_shadow_inst_pt, 128, ctx->sm_count)
                                                     : resident_grid(shadow_kernel, 128, ctx->sm_count);
+    const unsigned walk_grid = scene->any_subsurface ? subsurface_walk_grid((unsigned)ctx->sm_count) : 0u;
     const auto ext_group = alpha ? k_extend_group<false, true> : k_extend_group<>;
     const auto shadow_group = alpha ? k_shadow_group<false, true> : k_shadow_group<>;
     const unsigned ext_group_grid = resident_grid(ext_group, kTravBlock, ctx->sm_count);
@@ -1178,7 +1179,7 @@ static ks_status render_impl(ks_scene *scene, const ks_camera_desc *cam, const k
             }
             cudaEventRecord(f.ev[5], st);
             if (scene->any_subsurface) {
-                launch_subsurface(grid, (unsigned)ctx->sm_count, st, sv, rp, pb[f.cur], w.hits.ptr, w.queue[0].ptr, cnt + 2,
+                launch_subsurface(grid, walk_grid, st, sv, rp, pb[f.cur], w.hits.ptr, w.queue[0].ptr, cnt + 2,
                                   w.walks.ptr, cnt + 6, w.overflow.ptr);
                 stats.kernel_launches += 2;
             }

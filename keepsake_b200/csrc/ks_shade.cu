@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(128) k_subsurface_select(const __grid_constant
 // is left is latency: the longest walk's 256 steps one after the other, so neither the refill (4, 8, 16 idle
 // lanes: 11.1, 11.0, 11.0 ms) nor more CTAs per SM (5, 6, 8: 11.5, 12.6, 13.3 ms; by a register cap, 4 and 5 instead of 3:
 // 9.2 and 10.7 against 8.9) helps, but a shorter step does: rays through the 4-wide view, which halves
-// the nodes met, took the frame from 12.0 to 8.2 ms.  A ray with nearly equal hits, and every ray of a tree too
+// the nodes met, took the frame from 12.0 to 8.2 ms (on another machine than the 10.3).  A ray with nearly equal hits, and every ray of a tree too
 // deep for the view, takes the exact traversal.
 #ifndef KS_WALK_REFILL
 #define KS_WALK_REFILL 8
@@ -748,15 +748,20 @@ __global__ void __launch_bounds__(128) k_subsurface_walk(const __grid_constant__
         atomicOr(overflow, 1);
 }
 
-void launch_subsurface(unsigned grid, unsigned sm_count, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
+unsigned subsurface_walk_grid(unsigned sm_count)
+{
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subsurface_walk, 128, 0);
+    return (unsigned)std::max(per_sm, 1) * sm_count;
+}
+
+void launch_subsurface(unsigned grid, unsigned walk_grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
                        PathBuf cur, float4 *hits, const uint32_t *queue, const uint32_t *queue_count, uint32_t *walks,
                        uint32_t *walk_counts, int *overflow)
 {
     k_subsurface_select<<<grid, 128, 0, st>>>(sv, rp, cur, hits, queue, queue_count, walks, walk_counts);
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subsurface_walk, 128, 0);
-    k_subsurface_walk<<<std::min(grid, (unsigned)std::max(per_sm, 1) * sm_count), 128, 0, st>>>(
-        sv, rp, cur, hits, walks, walk_counts, walk_counts + 1, overflow);
+    k_subsurface_walk<<<std::min(grid, walk_grid), 128, 0, st>>>(sv, rp, cur, hits, walks, walk_counts, walk_counts + 1,
+                                                                 overflow);
 }
 
 void launch_sample(bool batch, unsigned grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp,

@@ -503,9 +503,9 @@ KS_D int trav_descend(const float (&t0)[4], const bool (&ok)[4], const uint32_t 
 // entry and exit planes are picked by address instead of by selects, the running maximum and
 // minimum of slab() are one max and one min over the axes (equal for boxes with lo <= hi), and the
 // 0 * inf guard, which changes nothing while every 1 / d is finite, is a path of its own.  With ranks
-// instead of a sorting network over four values per slot and 8-byte stack entries the mesh frame
-// (1.3 M triangles, 1024 x 1024 x 64) went from 101.9 to 93.5 ms, the instanced one (1080p x 4) from
-// 41.3 to 38.0 ms, every image bit for bit the same.
+// instead of a sorting network over four values per slot and 8-byte stack entries the instanced frame
+// (1080p x 4) went from 41.3 to 38.0 ms, every image bit for bit the same (and the mesh frame, 1.3 M triangles,
+// 1024 x 1024 x 64, from 101.9 to 93.5 ms, when flat scenes took these steps too).
 template <bool kAnyHit, class Stack>
 KS_D int trav_wide(const WideNode *wide, TravState &s, Stack &stack, int &overflow, TravCount *count)
 {
@@ -680,7 +680,8 @@ KS_D bool trav_step(const Node *__restrict__ nodes, const float4 *__restrict__ t
 // instead of with the two or three that reach a leaf in the same step.  Any-hit queries step without
 // waiting: holding back a leaf that may end the ray costs them more than the batching saves.  Returns
 // true when this lane's ray is over.  Leaf batches of 8, 12, 16 lanes: mesh frame (1.3 M triangles,
-// 1024 x 1024 x 64) 38.9, 37.7, 37.5 ms of closest hits, box room 1.80, 1.71, 1.65.
+// 1024 x 1024 x 64) 38.9, 37.7, 37.5 ms of closest hits, box room 1.80, 1.71, 1.65.  Between 12 and 16 whole calls
+// differ by little and both ways: 16 box room 0.7 % faster, textured materials 0.3, glossy passes 0.4 % slower.
 #ifndef KS_LEAF_BATCH
 #define KS_LEAF_BATCH 12
 #endif

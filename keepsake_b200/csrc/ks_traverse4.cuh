@@ -151,9 +151,7 @@ KS_D bool trav4_pop(const Wide4Node *__restrict__ nodes, Trav4 &s, const TravSta
 }
 
 // Visits node s.ref: descends to a child and returns true, or returns false when none is hit.
-// Any-hit queries take the children in slot order: nearest first took 2.5 % off the bench frame's
-// shadow rays once but made a pass of the occluded glossy scene 17 % slower (rays blocked by a distant
-// occluder then search the nearby geometry's subtrees first).
+// Any-hit queries take the children in slot order (why: trav_descend).
 template <bool kAnyHit>
 KS_D bool trav4_node(const Wide4Node *__restrict__ nodes, Trav4 &s, TravStack &stack, TravCount *count)
 {

@@ -445,8 +445,9 @@ KS_D bool ambiguous(const TravState &) { return false; }
 // ---- shading launchers (ks_shade.cu) ----------------------------------------------------------
 // k_sample: Sobol values and the NEE light sample of every path in the hit queue.
 // Subsurface entries of a bounce's hit queue (ks_shade.cu), before its light samples.  walks: room for the
-// queue's entries; walk_counts: two counters, zero.
-void launch_subsurface(unsigned grid, unsigned sm_count, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
+// queue's entries; walk_counts: two counters, zero; walk_grid: subsurface_walk_grid, one wave of resident CTAs.
+unsigned subsurface_walk_grid(unsigned sm_count);
+void launch_subsurface(unsigned grid, unsigned walk_grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
                        PathBuf cur, float4 *hits, const uint32_t *queue, const uint32_t *queue_count, uint32_t *walks,
                        uint32_t *walk_counts, int *overflow);
 void launch_sample(bool batch, unsigned grid, cudaStream_t st, const SceneView &sv, const RenderParams &rp,
