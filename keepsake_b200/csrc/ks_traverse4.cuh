@@ -118,7 +118,7 @@ KS_D bool ambiguous(const Trav4 &s)
 KS_D bool trav_begin(Trav4 &s, const RayQuery &ray, uint32_t root, uint32_t root_count, const float root_bmin[3],
                      const float root_bmax[3])
 {
-    s.hit.tri = ~0u;
+    s.hit.tri = s.hit.slot = ~0u;
     s.ray = ray;
     s.th = make_tri_helper(ray.d);
     s.set_ray(ray.d);
@@ -242,7 +242,7 @@ KS_D bool leaf_reached(const float4 *__restrict__ leaf_box, const Trav4 &s, uint
 // Whether the hit at hand is one of the leaf that starts at `first`, of which `slot` is tested.
 KS_D bool in_leaf(const Trav4 &s, uint32_t first, uint32_t slot)
 {
-    return s.hit.tri != ~0u && s.hit.slot >= first && s.hit.slot < slot;
+    return s.hit.slot - first < slot - first; // no hit yet: slot ~0u
 }
 
 // The range in which primitive `slot` of a leaf is tested.  After a hit in the same leaf it ends there, as in
