@@ -1229,7 +1229,7 @@ __global__ void k_wide4_fill(const TravNode *__restrict__ nodes, uint32_t n, boo
 
 // The view of the tree over `nodes` whose root is root_ref with box root_bound (6 floats), into out (node 0:
 // the root).  Launches kWide4Chunk levels between two looks at the counts (a level without nodes costs its
-// launch); max_levels: levels of the binary tree, at most kMaxBinaryLevels.
+// launch, some 2 us); max_levels: levels of the binary tree, at most kMaxBinaryLevels, and no fewer than the view's.
 static ks_status build_wide4(ks_context *ctx, BuildScratch &bs, const TravNode *nodes, uint32_t n_trav, uint32_t root_ref,
                              const float *root_bound, uint32_t max_levels, DevBuf<Wide4Node> &out)
 {
@@ -1251,7 +1251,7 @@ static ks_status build_wide4(ks_context *ctx, BuildScratch &bs, const TravNode *
         KS_CUDA_TRY(ctx, cudaMemcpyAsync(bs.wide_level.ptr, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         uint32_t done = 0;
         while (done < levels && count[done]) {
-            const uint32_t end = std::min(done + kWide4Chunk, levels - 1);
+            const uint32_t end = std::min(done + kWide4Chunk, max_levels);
             if (end == done)
                 return fail(ctx, KS_ERR_WATCHDOG, "sbvh build: 4-wide level limit reached");
             for (; done < end; ++done)
