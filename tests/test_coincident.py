@@ -49,7 +49,7 @@ def scene(ctx, ks, kind, twice, opacity=False):
         keep += ks.attach_textures(desc, [(mask, False)], [ks.TextureBinding.make(m, "opacity_map", 0, filter=0)
                                                            for m in range(len(mats) - 5, len(mats))])
     s = ks.Scene(ctx, desc, keepalive=(g, keep))
-    s.build_bvh()
+    s.build_bvh(alpha=1.0)  # whole triangles in the leaves: no reference is split in two
     return s, ks.camera_perspective(g.camera_to_world, g.vfov, W / H)
 
 
