@@ -174,6 +174,8 @@ __global__ void k_batch_prep(BatchState *st, uint32_t *counters, uint32_t capaci
         return;
     BatchState &s = *st;
     const uint32_t alive = counters[0];
+    if (counters[12] >= kAgainMin && counters[12] > s.count / kAgainShare)
+        s.exact = 1;
     const unsigned long long left = s.total - s.issued;
     const uint32_t n_new = (uint32_t)(left < (unsigned long long)(capacity - alive) ? left : capacity - alive);
     s.cur_count = alive;
@@ -261,30 +263,17 @@ KS_D float4 hit_record(const Hit &h, bool retrace = false)
 
 // Closest hit of every queued ray into hits[i] (slot ~0u: miss); k_build_queues then sorts the
 // paths into the hit and miss queues in index order, so that shading reads the path state in
-// order.  kBatch: paths of many jobs, the count read from the batch state.
-// kAlpha: the scene has opacity maps; candidate hits go through their stochastic test (SceneAlpha).
-// kDeep: the tree is too deep for the 4-wide view.  kMixed: a batch of which some job's is; its rays go to the
-// variant that their job's tree takes (the check cost a batch without such jobs 1.6 %).
-// count_ptr: where the count lies on the device when the host does not know it yet (else null); choose: the
-// group kernel was launched too, and short queues are its.
-template <bool kBatch = false, bool kAlpha = false, bool kDeep = false, bool kMixed = false>
-__global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
-                                                   const uint32_t *count_ptr, int choose, float4 *hits, uint32_t *fetch,
-                                                   int *overflow, unsigned long long *work, BatchView bv)
+// order.  View: the tree that is walked (TreeOf).  kSkip: rays of deep trees (kDeep: of all others) are another
+// kernel's.
+template <class View, bool kBatch, bool kSkip, bool kDeep, class Alpha>
+KS_D void extend_rays(const SceneView &sv_in, const PathBuf &pb, uint32_t count, float4 *hits, uint32_t *fetch,
+                      int *overflow, unsigned long long *work, const BatchView &bv, TravStack &stack,
+                      const Alpha &filter)
 {
-    count = queue_size<kBatch>(count, count_ptr, bv);
-    if (!kDeep && choose && count <= KS_GROUP_RAYS)
-        return; // k_extend_group's
     TravCount tc;
-    KS_TRAV_STACK(stack);
-    using View = TreeOf<kDeep>;
     typename View::State s;
     typename View::Tree tree = View::tree(sv_in);
     const float4 *tris = sv_in.prim_tris;
-    using Alpha = std::conditional_t<kAlpha, SceneAlpha, NoAlpha>;
-    Alpha filter;
-    if constexpr (kAlpha)
-        filter.sv = &sv_in;
     uint32_t ray = ~0u;
     bool drained = false;
     int of = 0;
@@ -295,7 +284,7 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
             const SceneView &sv = job_of<kBatch>(sv_in, bv.views, job);
             tree = View::tree(sv);
             tris = sv.prim_tris;
-            if (kMixed && (sv.deep != 0) != kDeep) {
+            if (kSkip && (sv.deep != 0) != kDeep) {
                 // the other variant's
             } else if (trav_begin(s, path_ray(pb, id), View::root(sv), sv.root_count, sv.bmin, sv.bmax))
                 ray = id;
@@ -320,6 +309,35 @@ __global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __gr
     if (of)
         atomicOr(overflow, 1);
     flush_counts(tc, work);
+}
+
+// kBatch: paths of many jobs, the count read from the batch state; once many of its rays are traced again
+// (kAgainShare) by the exact steps over the jobs' binary nodes.
+// kAlpha: the scene has opacity maps; candidate hits go through their stochastic test (SceneAlpha).
+// kDeep: the tree is too deep for the 4-wide view.  kMixed: a batch of which some job's is; its rays go to the
+// variant that their job's tree takes (the check cost a batch without such jobs 1.6 %).
+// count_ptr: where the count lies on the device when the host does not know it yet (else null); choose: the
+// group kernel was launched too, and short queues are its.
+template <bool kBatch = false, bool kAlpha = false, bool kDeep = false, bool kMixed = false>
+__global__ void __launch_bounds__(128, KS_EXT_MIN_BLOCKS) k_extend_pt(const __grid_constant__ SceneView sv_in, PathBuf pb, uint32_t count,
+                                                   const uint32_t *count_ptr, int choose, float4 *hits, uint32_t *fetch,
+                                                   int *overflow, unsigned long long *work, BatchView bv)
+{
+    count = queue_size<kBatch>(count, count_ptr, bv);
+    const bool exact = kBatch && !kDeep && bv.state->exact;
+    if (!kDeep && !exact && choose && count <= KS_GROUP_RAYS)
+        return; // k_extend_group's
+    KS_TRAV_STACK(stack);
+    std::conditional_t<kAlpha, SceneAlpha, NoAlpha> filter;
+    if constexpr (kAlpha)
+        filter.sv = &sv_in;
+    if constexpr (kBatch && !kDeep) {
+        if (exact) {
+            extend_rays<TreeOfBinary, true, kMixed, false>(sv_in, pb, count, hits, fetch, overflow, work, bv, stack, filter);
+            return;
+        }
+    }
+    extend_rays<TreeOf<kDeep>, kBatch, kMixed, kDeep>(sv_in, pb, count, hits, fetch, overflow, work, bv, stack, filter);
 }
 
 // Hit and miss queues from the per-ray results of k_extend_pt, one CTA-aggregated append per
@@ -500,7 +518,7 @@ __global__ void __launch_bounds__(kTravBlock, KS_GROUP_MIN_BLOCKS) k_extend_grou
     float4 *hits, unsigned long long *work, BatchView bv)
 {
     count = queue_size<kBatch>(count, count_ptr, bv);
-    if (choose && count > KS_GROUP_RAYS)
+    if ((choose && count > KS_GROUP_RAYS) || (kBatch && bv.state->exact))
         return;
     TravCount tc;
     KS_GROUP_STACK(stack);

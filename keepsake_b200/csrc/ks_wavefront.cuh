@@ -62,6 +62,7 @@ struct BatchState
     unsigned long long ext_rays, shadow_rays;     // work counters
     uint32_t cur_count, n_new, count, base_slot;  // paths alive, refilled, traced this iteration
     uint32_t iterations, max_iterations, error;
+    uint32_t exact; // closest hits by the exact steps: many rays met two surfaces at one distance
 };
 
 struct BatchView
@@ -438,6 +439,14 @@ struct TreeOf<true>
     using State = TravState;
     using Tree = const WideNode *;
     KS_D static Tree tree(const SceneView &sv) { return sv.wide_steps; }
+    KS_D static uint32_t root(const SceneView &sv) { return sv.root_ref; }
+};
+// The exact steps over binary nodes, where a scene has no others.
+struct TreeOfBinary
+{
+    using State = TravState;
+    using Tree = const LazyWide *;
+    KS_D static Tree tree(const SceneView &sv) { return reinterpret_cast<const LazyWide *>(sv.nodes); }
     KS_D static uint32_t root(const SceneView &sv) { return sv.root_ref; }
 };
 KS_D bool ambiguous(const TravState &) { return false; }

@@ -118,3 +118,41 @@ def test_the_second_surface_costs_what_it_is(ctx, kind, limit):
         times.append(min(runs))
         s.close()
     assert times[1] < limit * times[0], times
+
+
+def batch(ks, ctx, made, size):
+    import torch
+    jobs = []
+    for k, (s, cam) in enumerate(made):
+        acc = torch.zeros((size[1], size[0], 3), dtype=torch.float64, device="cuda")
+        wts = torch.zeros((size[1], size[0], 2), dtype=torch.float64, device="cuda")
+        jobs.append((s, cam, params(ks, render_width=size[0], render_height=size[1], rng_seed=k), acc, wts))
+    torch.cuda.synchronize()
+    return jobs, lambda: ks.batch_render(ctx, [(s, c, p, a.data_ptr(), w.data_ptr()) for s, c, p, a, w in jobs])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kinds", [("layers", "copies", "layers"), ("layers", "copies", "copies", "copies", "copies")])
+def test_batch(ctx, kinds):
+    """Many rays of the batch are traced again (all jobs take the exact steps), or few."""
+    import keepsake_b200 as ks
+    made = [scene(ctx, ks, k, True) for k in kinds]
+    jobs, run = batch(ks, ctx, made, (W, H))
+    run()
+    for s, cam, p, acc, wts in jobs:
+        same((acc.cpu().numpy(), wts.cpu().numpy()), s.render(cam, p))
+        s.close()
+
+
+@pytest.mark.gpu
+def test_the_second_surface_costs_what_it_is_in_a_batch(ctx):
+    """Whole batches of the room with and without layers: @@ times as long by the exact traversal."""
+    import keepsake_b200 as ks
+    times = []
+    for twice in (False, True):
+        made = [scene(ctx, ks, "layers", twice) for _ in range(4)]
+        jobs, run = batch(ks, ctx, made, (384, 384))
+        times.append(min(run().ms_total for _ in range(6)))
+        for s, _ in made:
+            s.close()
+    assert times[1] < 9.9 * times[0], times
