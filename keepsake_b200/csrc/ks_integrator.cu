@@ -72,7 +72,9 @@ constexpr uint32_t kCounters = 13;
 // Rays traced again in an iteration (k_build_queues), as a share of its rays, from which the closest hits of a scene
 // are traced by the exact steps from then on: a ray that is traced again costs twice a ray of the 4-wide view, the
 // exact steps 1.2 to 1.4 times.  A box room with a second layer of 80,000 triangles in each wall's plane, 512 x 512
-// x 8: closest hits 2.0 ms by the exact steps, 5.4 with each ray traced again.
+// x 8: closest hits 2.0 ms by the exact steps, 5.4 with each ray traced again.  A batch's iterations are not seen by
+// the host: k_batch_prep decides, and the exact steps are those over binary nodes (six such rooms of 7,200 triangles a
+// wall, 256 x 256 x 8: 7.7 ms, 10.2 traced again; 7.4 with whole nodes).
 constexpr uint32_t kAgainShare = 6, kAgainMin = 4096;
 
 // ---- kernels --------------------------------------------------------------------------------

@@ -5,7 +5,7 @@ the exact traversal's order, and a scene with many is traced by the exact steps 
 
 All ways give the same hits, so images differ by the order of FP64 additions only.  And the closest hits
 cost what the surfaces cost: within twice the ratio that the exact traversal alone had to the scene without
-the second layer (1.2 for the copies, 2.4 for the layers; traced again ray by ray, 4 and 10)."""
+the second layer (1.2 for the copies, 2.0 for the layers; traced again ray by ray, 3.7 and 6.9)."""
 import numpy as np
 import pytest
 
@@ -99,7 +99,7 @@ def test_layers_in_one_plane(ctx, opacity):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind,limit", [("copies", 2.4), ("layers", 4.8)])
+@pytest.mark.parametrize("kind,limit", [("copies", 2.4), ("layers", 4.0)])
 def test_the_second_surface_costs_what_it_is(ctx, kind, limit):
     import torch
 
@@ -146,7 +146,8 @@ def test_batch(ctx, kinds):
 
 @pytest.mark.gpu
 def test_the_second_surface_costs_what_it_is_in_a_batch(ctx):
-    """Whole batches of the room with and without layers: @@ times as long by the exact traversal."""
+    """Whole batches of the room with and without layers: 1.5 times as long by the exact traversal alone, 3.0 with
+    each ray traced again; the limit lies half-way."""
     import keepsake_b200 as ks
     times = []
     for twice in (False, True):
@@ -155,4 +156,4 @@ def test_the_second_surface_costs_what_it_is_in_a_batch(ctx):
         times.append(min(run().ms_total for _ in range(6)))
         for s, _ in made:
             s.close()
-    assert times[1] < 9.9 * times[0], times
+    assert times[1] < 2.2 * times[0], times
